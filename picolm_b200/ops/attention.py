@@ -15,8 +15,9 @@ def attention_rows(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
                    tok_seq: torch.Tensor, block_table: torch.Tensor, num_kv_heads: int, scale: float,
                    window: Optional[int] = None, out: Optional[torch.Tensor] = None,
                    sink: Optional[torch.Tensor] = None, keep_first: int = 0,
-                   slopes: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Causal attention of q [T, H, hd] over the paged cache; returns [T, H*hd].  `window` here and in the other kernels' faces:
+                   slopes: Optional[torch.Tensor] = None, longest: int = 1) -> torch.Tensor:
+    """Causal attention of q [T, H, hd] over the paged cache; returns [T, H*hd].  `longest`: the most neighbouring rows
+    that belong to one sequence (a step's `max_new`; it chooses a kernel, the result is the same to the bit).  `window` here and in the other kernels' faces:
     a sliding window of that many keys, or the negative of a chunk size for a mask of chunks (`key_mask`).  `sink` here
     and in the other faces: float32 [H], one more term exp(sink[h]) in the denominator of head h's softmax, with no key
     and no value and outside the scale (None: the plain softmax).  `keep_first` here and in the other faces: beside a sliding
@@ -36,7 +37,7 @@ def attention_rows(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
     _cache_bounds("attention_simt", (), k_cache, block_table)
     _check(_fn("attention_simt", "plm_attention_rows")(
         _p(q), _p(k_cache), _p(v_cache), _p(out), _dt(q, "q"), _p(tok_pos), _p(tok_seq), _p(block_table),
-        block_table.shape[1], T, H, G, hd, float(scale), int(window or 0), _p(sink), int(keep_first), _p(slopes), _stream()),
+        block_table.shape[1], T, H, G, hd, float(scale), int(window or 0), _p(sink), int(keep_first), _p(slopes), int(longest), _stream()),
         f"attention_rows T={T} H={H} hd={hd}")
     return out
 
@@ -286,4 +287,4 @@ def attention(q: torch.Tensor, kv, step, num_kv_heads: int, scale: float, chunk:
         return prefill(q, kv.k, kv.v, step.seq_start, step.seq_kv_len, kv.block_table, step.max_new,
                        num_kv_heads, scale, window=kv.window, **more)
     return attention_rows(q, kv.k, kv.v, step.tok_pos, step.tok_seq, kv.block_table, num_kv_heads, scale,
-                          window=kv.window, **more)
+                          window=kv.window, longest=step.max_new, **more)

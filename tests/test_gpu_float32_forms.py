@@ -1,0 +1,53 @@
+"""The forms of the float32 product and of the CUDA-core attention that are chosen by size: every form gives the bits of
+the general one, so a row does not depend on how many rows stand beside it."""
+import math
+
+import pytest
+import torch
+
+from test_gpu_kernels import DEV, DT, _paged
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,K", [(16, 4), (130, 20), (129, 100), (300, 64), (2064, 132)])
+@pytest.mark.parametrize("M", [1, 8, 9, 32, 33, 65, 200, 530])
+def test_float32_product_forms_agree_to_the_bit(M, N, K):
+    """Few rows, many rows, ragged edges of every tile: against the general kernel (which takes rows that do not start on
+    16-byte boundaries), against float64, and row by row."""
+    from picolm_b200 import ops
+    torch.manual_seed(M * 7 + N + K)
+    wide = torch.randn(M, K + 4, device=DEV)
+    w = torch.randn(N, K, device=DEV)
+    odd = wide[:, 1:1 + K]                                   # the general kernel's: K a multiple of 4, rows off by 4 bytes
+    out, general = ops.gemm_simt(odd.contiguous(), w, torch.float32), ops.gemm_simt(odd, w, torch.float32)
+    assert torch.equal(out, general)
+    assert torch.equal(out[M // 2:M // 2 + 1], ops.gemm_simt(odd[M // 2:M // 2 + 1].contiguous(), w, torch.float32))
+    ref = odd.double() @ w.double().T
+    # a piece of 16 terms: at most 16 roundings of partial sums, then one to the result
+    bound = 17 * 2.0 ** -24 * (odd.double().abs() @ w.double().abs().T)
+    assert ((out.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,G,hd", [(5, 5, 16), (6, 2, 48), (16, 4, 64), (8, 1, 128), (4, 2, 80), (3, 1, 256), (80, 2, 32)])
+@pytest.mark.parametrize("extra", [False, True])
+def test_attention_tile_form_agrees_to_the_bit(dtype, H, G, hd, extra):
+    """Prompts of unequal lengths in one step, some behind earlier positions, tiles that hold several sequences: the tile
+    form against the row form.  The last value of each sequence is infinite: rows before it must not see it."""
+    from picolm_b200 import ops
+    torch.manual_seed(H * 100 + hd)
+    lens, new = [100, 1, 65, 33, 7, 64], [90, 1, 65, 2, 7, 31]
+    ks = [torch.randn(n, G, hd) for n in lens]
+    vs = [torch.randn(n, G, hd) for n in lens]
+    for v in vs:
+        v[-1] = math.inf
+    kc, vc, table = _paged(ks, vs, lens, 16, DT[dtype], 5)
+    q = torch.randn(sum(new), H, hd).to(DT[dtype]).to(DEV)
+    pos = torch.tensor([p for n, m in zip(lens, new) for p in range(n - m, n)], dtype=torch.int32, device=DEV)
+    seq = torch.tensor([b for b, m in enumerate(new) for _ in range(m)], dtype=torch.int32, device=DEV)
+    more = dict(sink=torch.randn(H, device=DEV), slopes=torch.rand(H, device=DEV) * 0.1) if extra else {}
+    rows, tiles = (ops.attention_rows(q, kc.to(DEV), vc.to(DEV), pos, seq, table.to(DEV), G, hd ** -0.5, longest=n, **more)
+                   for n in (1, max(new)))
+    assert torch.isfinite(rows).any()
+    assert torch.equal(torch.nan_to_num(rows.float(), nan=7.0), torch.nan_to_num(tiles.float(), nan=7.0))
