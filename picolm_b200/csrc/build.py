@@ -45,6 +45,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "routed": ["routed.cu"],
     "decay_chunk": ["decay_chunk.cu"],
     "delta_chunk": ["delta_chunk.cu"],
+    "scan_chunk": ["scan_chunk.cu"],
 }
 HEADERS = ["common.cuh", "tc_common.cuh", "mma_common.cuh", "gemm_tc_static.h"]
 

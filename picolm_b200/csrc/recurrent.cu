@@ -1404,12 +1404,13 @@ extern "C" int plm_delta_scan(const float* qn, const float* kn, const float* qk,
 // on the state (the three scaled copies of k and q, A, M, e^{L_C}) is made for all chunks side by side by a first
 // kernel; the second walks a sequence's chunks with the state in registers: two passes of dot products without a chain
 // between tokens, a forward substitution over the chunk's tokens, and the state's update.
+// For keys of 129 to 256 values; smaller ones run in scan_chunk.cu, whose chunks of larger keys would not fit shared memory.
 #define DELTA_CHUNK 32
 
 __host__ __device__ static inline long delta_ws_floats(int NP) { return 3L * DELTA_CHUNK * NP + 2L * DELTA_CHUNK * DELTA_CHUNK + NP; }
 
 // The width of a row of keys in the workspace: eight times the NR values a thread of the second kernel holds.
-static inline int delta_chunk_np(int N) { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : 256; }
+static inline int delta_chunk_np(int) { return 256; }
 
 // grid (chunk of the sequence, sequence, head).  ws per (slot, head): Kp [C][NP] | Qp [C][NP] | Ke [C][NP] | A^T [C][C] | M^T [C][C]
 // | e^{L_C} [NP], NP = delta_chunk_np(N), the padding zero.  A sequence's chunk c lives in slot seq_start / C + sequence + c.
@@ -1674,7 +1675,7 @@ extern "C" int plm_delta_chunk_scan(const float* qn, const float* kn, const floa
                                     int heads_per_group, int head_decay, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     if (H <= 0 || N <= 0 || P <= 0 || heads_per_group <= 0 || H % heads_per_group) return PLM_ERR_SHAPE;
-    if (N > 256) return PLM_ERR_UNSUPPORTED;
+    if (N <= 128 || N > 256) return PLM_ERR_UNSUPPORTED;
     if (dtype != PLM_F32 && dtype != PLM_BF16) return PLM_ERR_DTYPE;
     const int NP = delta_chunk_np(N);
     const size_t prep_smem = (size_t)DELTA_CHUNK * (head_decay ? 2 * N + 1 : 3 * N) * sizeof(float);
@@ -1686,9 +1687,6 @@ extern "C" int plm_delta_chunk_scan(const float* qn, const float* kn, const floa
 #define DCS(NR_, ST_)                                                                                                     \
     return delta_chunk_launch<NR_, ST_>(ws, beta, v, dtype == PLM_F32 ? 1 : 0, ldv, state, state_stride, y, seq_start, seq_slot, \
                                         n_seqs, H, N, P, stream)
-    if (NP <= 32) DCS(4, 2);
-    if (NP <= 64) DCS(8, 2);
-    if (NP <= 128) DCS(16, 2);
     DCS(32, 1);
 #undef DCS
 }

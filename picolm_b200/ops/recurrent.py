@@ -1,5 +1,5 @@
-"""Faces of the kernels for mixers with a fixed-size state (csrc/recurrent.cu): the depthwise causal
-convolution, the gated linear recurrence, the gate-and-norm step, one small matrix per head, and rows
+"""Faces of the kernels for mixers with a fixed-size state (csrc/recurrent.cu, scan_chunk.cu, decay_chunk.cu,
+delta_chunk.cu): the depthwise causal convolution, the gated linear recurrence, the gate-and-norm step, one small matrix per head, and rows
 written into the pages of a cache."""
 from __future__ import annotations
 
@@ -7,7 +7,7 @@ from typing import Optional
 
 import torch
 
-from ._lib import PAGE_TOKENS, KernelError, _check, _dev, _dt, _fn, _i32, _p, _stream, set_bounds
+from ._lib import PAGE_TOKENS, KernelError, _check, _dev, _dt, _fn, _i32, _p, _stream, set_bounds, status_word
 
 DECAY_STEP, DECAY_SIGMOID, DECAY_GIVEN, DECAY_CONST = 1, 2, 3, 4
 
@@ -75,7 +75,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
       DECAY_CONST    raw None: d = p0[h] for the whole head and every token; with `activation="silu"` q, k and v pass
                      SiLU on their way in (float32, from the rows as they are)
     `state` float32 [slots, >= heads * key_dim * value_dim] with contiguous rows holds S of every sequence as
-    [heads, key_dim, value_dim] and is carried on."""
+    [heads, key_dim, value_dim] and is carried on.  Prompts with a decay per key channel run 64 tokens at a time
+    (csrc/scan_chunk.cu) where the sizes allow it."""
     if raw is None and mode == DECAY_CONST:
         raw = v                                              # (not read)
     if activation not in (None, "silu") or (activation and mode != DECAY_CONST):
@@ -109,6 +110,16 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     if state.dtype != torch.float32 or state.shape[1] < H * N * P:
         raise KernelError("linear_scan: the state must be float32 with heads * key_dim * value_dim values a row")
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
+    if (mode == DECAY_SIGMOID and skip is None and step.max_new >= SIGMOID_CHUNK_FROM and N <= SCAN_CHUNK_KEYS
+            and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
+        ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
+        _check(_fn("scan_chunk", "plm_sigmoid_chunk_scan")(
+            _p(q), _p(k), _p(v), _p(raw), _dt(v, "v"), ldq, ldk, ldv, ldr, _p(p0), float(q_scale), float(power), _p(state), lds, _p(y),
+            _p(ws), _p(step.seq_start), _p(step.seq_slot), step.n_seqs, int(step.max_new), H, N, P, heads_per_group, _stream()),
+            f"sigmoid_chunk_scan T={T} H={H} N={N} P={P}", kernels=4,
+            nbytes=T * ((2 * G * N + H * N + H * P) * v.element_size() + H * P * 4) + 2 * step.n_seqs * H * N * P * 4,
+            flops=2 * T * H * (2 * N * P + 64 // 2 * (N + P)))
+        return y
     # Long prompts are cut into segments that run side by side: a first pass leaves what each segment adds to the
     # state, a small kernel chains those into the state at every segment's start, a second pass gives y.
     seg_len, n_segs = scan_plan(step.n_seqs, H, N, P, step.max_new, T)
@@ -134,6 +145,24 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
         nbytes=T * (2 * G * N + H * P) * v.element_size() + T * H * P * 4 + 2 * step.n_seqs * H * N * P * 4,
         flops=(10 if n_segs > 1 else 6) * T * H * N * P)
     return y
+
+
+SCAN_CHUNK_KEYS = 128      # the largest key size of the kernels that take a decay per channel 64 tokens at a time
+# Tokens of a step's longest sequence from which `linear_scan` (with a decay per key channel) and `delta_scan` do so.  Below,
+# token by token is faster (measured: 8 heads of 128 x 128, one sequence of 64 and of 128 tokens, linear attention 44 against
+# 34 us and 42 against 62, delta rule 46 against 58 and 64 against 114; 32 sequences of 16: 88 against 39, 190 against 57).
+SIGMOID_CHUNK_FROM = 96
+DELTA_CHANNEL_CHUNK_FROM = 64
+SCAN_CHUNK_FLOATS = 1 << 31      # the most workspace that linear attention takes for it (some 4.8 KB a token and head of 128 x 256)
+_chunk_floats = {}
+
+
+def _scan_chunk_floats(n_tokens: int, n_seqs: int, heads: int, key_dim: int, value_dim: int) -> int:
+    """Floats of workspace of csrc/scan_chunk.cu for a step: a sequence's chunks start at slot seq_start // 64 + its number."""
+    floats = _chunk_floats.get((key_dim, value_dim))
+    if floats is None:
+        floats = _chunk_floats[key_dim, value_dim] = _fn("scan_chunk", "plm_scan_chunk_floats")(key_dim, value_dim)
+    return (n_tokens // 64 + n_seqs + 1) * heads * floats
 
 
 _plans = {}
@@ -478,10 +507,10 @@ DELTA_CHUNK_FROM = 16      # tokens of a step's longest sequence from which the 
 
 
 def delta_chunk_workspace(n_tokens: int, n_seqs: int, heads: int, key_dim: int) -> int:
-    """Floats of workspace the chunked delta rule takes (as the kernels lay it out): per chunk and head three copies
-    of the chunk's keys or queries [32, NP], two matrices [32, 32] and a row [NP], NP the key size rounded up to the
-    next of 32, 64, 128, 256; a sequence's chunks start at slot seq_start // 32 + its number."""
-    np_ = next(w for w in (32, 64, 128, 256) if key_dim <= w)
+    """Floats of workspace the chunked delta rule takes for keys of more than `SCAN_CHUNK_KEYS` values (as the kernels lay
+    it out): per chunk and head three copies of the chunk's keys or queries [32, 256], two matrices [32, 32] and a row
+    [256]; a sequence's chunks start at slot seq_start // 32 + its number."""
+    np_ = 256
     return (n_tokens // 32 + n_seqs + 1) * heads * (3 * 32 * np_ + 2 * 32 * 32 + np_)
 
 
@@ -525,9 +554,10 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
     (the read-out sees the token's own write; with `head_decay` one decay a head).  qn, kn, qk, decay (its logarithm), beta as `delta_prep` returns them; v [T, heads *
     value_dim] (a column slice will do); `state` float32 [slots, >= heads * key_dim * value_dim] with contiguous
     rows holds S as [heads, key_dim, value_dim] and is carried on.  Returns o, float32 [T, heads * value_dim].
-    A step whose longest sequence brings `DELTA_CHUNK_FROM` tokens or more runs chunk by chunk (two kernels: what does
-    not depend on the state for all chunks side by side, then a walk over each sequence's chunks; with one decay a head and
-    values in bfloat16 on the tensor cores, 64 tokens at a time); shorter portions and single tokens run token by token."""
+    A step whose longest sequence brings `DELTA_CHUNK_FROM` tokens or more runs chunk by chunk (what does not depend on the
+    state for all chunks side by side, then a walk over each sequence's chunks; with one decay a head and values in bfloat16
+    on the tensor cores, else 64 tokens at a time in float32, csrc/scan_chunk.cu); shorter portions and single tokens run
+    token by token."""
     H, N, P = heads, key_dim, value_dim
     T = v.shape[0]
     if H % heads_per_group:
@@ -549,6 +579,7 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
     set_bounds("recurrent", n_seqs=step.n_seqs, device=v.device)
     prompts = step.max_new >= DELTA_CHUNK_FROM and not (step.is_decode and step.n_tokens == step.n_seqs)
+    channel = not (head_decay and delta_head_chunk_supported(v, state, N, P)) and N <= SCAN_CHUNK_KEYS
     if prompts and head_decay and delta_head_chunk_supported(v, state, N, P):
         per = _head_chunk_bytes.get((N, P))
         if per is None:
@@ -562,7 +593,17 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
             nbytes=T * (8 * G * N + H * P * (4 + v.element_size())) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (3 * N * P + 64 // 2 * (2 * N + N + 2 * P)))
         return y
-    if prompts:
+    if channel and step.max_new >= DELTA_CHANNEL_CHUNK_FROM:
+        ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
+        _check(_fn("scan_chunk", "plm_delta_channel_scan")(
+            _p(qn), _p(kn), _p(decay), _p(beta), _p(v), _dt(v, "v"), ldv, _p(state), lds, _p(y), _p(ws), _p(step.seq_start),
+            _p(step.seq_slot), step.n_seqs, int(step.max_new), H, N, P, heads_per_group, 1 if head_decay else 0,
+            _p(status_word(v.device)), _stream()),
+            f"delta_channel_scan T={T} H={H} N={N} P={P}", kernels=3,
+            nbytes=T * ((2 * G * N + H * ND) * 4 + H * P * (4 + v.element_size())) + 2 * step.n_seqs * H * N * P * 4,
+            flops=2 * T * H * (3 * N * P + 64 // 2 * (3 * N + 2 * P)))
+        return y
+    if prompts and not channel:
         floats = delta_chunk_workspace(T, step.n_seqs, H, N)
         ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
         _check(_fn("recurrent", "plm_delta_chunk_scan")(

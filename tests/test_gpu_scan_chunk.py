@@ -1,0 +1,92 @@
+"""Recurrences with a decay per key channel, 64 tokens at a time (csrc/scan_chunk.cu): against the recurrence in float64,
+at the edges of chunks, blocks and tiles."""
+import types
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _step(lens):
+    start = [0]
+    for n in lens:
+        start.append(start[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    return types.SimpleNamespace(n_seqs=len(lens), n_tokens=start[-1], max_new=max(lens), is_decode=max(lens) == 1, seq_start=i32(start),
+                                 seq_slot=i32(list(range(len(lens)))[::-1]))
+
+
+def _recurrence(q, k, v, decay, beta, state, lens):
+    """float64; `state` [sequences, H, N, P] in the order of the slots."""
+    outs, states, at = [], [None] * len(lens), 0
+    for b, n in enumerate(lens):
+        S = state[len(lens) - 1 - b].double()
+        for t in range(at, at + n):
+            S = S * decay[t][:, :, None]
+            u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.bmm(k[t][:, None], S)[:, 0])
+            S = S + k[t][:, :, None] * u[:, None]
+            outs.append(torch.bmm(q[t][:, None], S)[:, 0])
+        states[len(lens) - 1 - b] = S
+        at += n
+    return torch.stack(outs), torch.stack(states)
+
+
+def _off(a, b):
+    return ((a.double() - b).norm() / b.norm()).item()
+
+
+LENS = [[64], [65, 1, 63], [16, 130, 3], [200]]
+SIZES = [(2, 1, 128, 128), (3, 3, 64, 72), (2, 2, 48, 6), (1, 1, 20, 33), (2, 1, 100, 260)]
+# The state and the outputs are sums of at most a few hundred terms in float32 whose factors (exponentials of sums of at most
+# 64 logarithms, products of three of them) are each off by a few units of 2^-24: 1e-6 over vectors whose errors do not align.
+BOUND = 1e-6
+
+
+@pytest.mark.parametrize("lens", LENS)
+@pytest.mark.parametrize("H,G,N,P", SIZES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("head_decay", [False, True])
+def test_delta_rule_in_chunks(lens, H, G, N, P, dtype, head_decay):
+    from picolm_b200 import ops
+    if head_decay and dtype == torch.bfloat16:
+        pytest.skip("one decay a head in bfloat16 has kernels of its own")
+    torch.manual_seed(sum(lens) + N + P)
+    T, step = sum(lens), _step(lens)
+    unit = lambda: torch.nn.functional.normalize(torch.randn(T, G, N, device=DEV) + 0.3, dim=-1).reshape(T, G * N).contiguous()
+    q, k, v = unit(), unit(), torch.randn(T, H * P, device=DEV).to(dtype)
+    # decays from almost one to almost nothing, neighbours of very different strength
+    decay = -torch.exp(3 * torch.randn(T, H if head_decay else H * N, device=DEV) - 3)
+    beta = torch.rand(T, H, device=DEV)
+    state0 = torch.randn(len(lens) + 1, H, N, P, device=DEV)
+    state = state0.clone().view(len(lens) + 1, -1)
+    y = ops.delta_scan(q, k, (q.view(T, G, N) * k.view(T, G, N)).sum(-1).contiguous(), decay, beta, v, state, step, H, N, P,
+                       heads_per_group=H // G, head_decay=head_decay)
+    wide = lambda x: x.double().view(T, G, N).repeat_interleave(H // G, 1)
+    d = torch.exp(decay.double()).view(T, H, -1).expand(T, H, N)
+    o, S = _recurrence(wide(q), wide(k), v.double().view(T, H, P), d, beta.double(), state0, lens)
+    assert _off(y.view(T, H, P), o) < BOUND and _off(state.view(-1, H, N, P)[:len(lens)], S) < BOUND
+    assert torch.equal(state[len(lens)], state0[len(lens)].view(-1))
+
+
+@pytest.mark.parametrize("lens", [[128], [129], [191], [400]] + [[65, 130, 3], [192, 64, 1]])
+@pytest.mark.parametrize("H,G,N,P", SIZES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_linear_attention_in_chunks(lens, H, G, N, P, dtype):
+    """Column slices of a wider projection, and a group of heads that shares keys and queries."""
+    from picolm_b200 import ops
+    torch.manual_seed(sum(lens) + N + P)
+    T, step = sum(lens), _step(lens)
+    rows = torch.randn(T, 2 * G * N + H * P + H * N + 3, device=DEV).to(dtype)
+    q, k, v, raw = (t[:, :w] for t, w in ((rows, G * N), (rows[:, G * N:], G * N), (rows[:, 2 * G * N:], H * P),
+                                          (rows[:, 2 * G * N + H * P:], H * N)))
+    bias, power = torch.rand(H * N, device=DEV) * 8 - 4, 1.0 / 16.0
+    state0 = torch.randn(len(lens) + 1, H, N, P, device=DEV)
+    state = state0.clone().view(len(lens) + 1, -1)
+    y = ops.linear_scan(q, k, v, raw, ops.DECAY_SIGMOID, bias, None, None, N ** -0.5, power, state, step, H, N, P, heads_per_group=H // G)
+    wide = lambda x: x.double().reshape(T, G, N).repeat_interleave(H // G, 1)
+    d = (torch.sigmoid(raw.double() + bias.double()) ** power).view(T, H, N)
+    o, S = _recurrence(wide(q) * N ** -0.5, wide(k), v.double().reshape(T, H, P), d, None, state0, lens)
+    assert _off(y.view(T, H, P), o) < BOUND and _off(state.view(-1, H, N, P)[:len(lens)], S) < BOUND
+    assert torch.equal(state[len(lens)], state0[len(lens)].view(-1))
