@@ -43,6 +43,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "sampling": ["sampling.cu"],
     "recurrent": ["recurrent.cu"],
     "routed": ["routed.cu"],
+    "routed_stream": ["routed_stream.cu"],
     "decay_chunk": ["decay_chunk.cu"],
     "delta_chunk": ["delta_chunk.cu"],
     "scan_chunk": ["scan_chunk.cu"],

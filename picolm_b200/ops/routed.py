@@ -97,6 +97,24 @@ def moe_align(ids: torch.Tensor, n_experts: int, bm: int, n_skip: int = 0) -> So
     return SortedPairs(sorted_, tile_expert, where, bm, max_tiles, top, T)
 
 
+STREAM_TILES = 2048        # the most tiles of the streaming products
+
+
+def _few_rows(a: torch.Tensor, lda: int, w: torch.Tensor, out: torch.Tensor, mode: int, pairs: SortedPairs, N: int, K: int,
+              interleaved: bool) -> int:
+    """The experts' products over sorted pairs on mma.sync or the CUDA cores: bfloat16 tiles of 16 rows stream their weights
+    through one CTA an SM (csrc/routed_stream.cu: N a multiple of 32, K of 64); the rest by plm_moe_gemm.  Both give the
+    same bits."""
+    if (a.dtype == torch.bfloat16 and pairs.bm == 16 and N % 32 == 0 and K % 64 == 0 and pairs.max_tiles <= STREAM_TILES
+            and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+        return _fn("routed_stream", "plm_moe_stream")(
+            _p(a), lda, pairs.top, _p(w), w.shape[0], _p(out), out.shape[1], mode, _p(pairs.tile_expert), _p(pairs.sorted),
+            pairs.max_tiles, N, K, 1 if interleaved else 0, _p(status_word(a.device)), _stream())
+    return _fn("routed", "plm_moe_gemm")(
+        _p(a), lda, pairs.top, _p(w), _p(out), out.shape[1], _dt(a, "a"), mode, _p(pairs.tile_expert), _p(pairs.sorted),
+        pairs.max_tiles, pairs.bm, N, K, 1 if interleaved else 0, _stream())
+
+
 def moe_gate_up(h: torch.Tensor, w_gate_up: torch.Tensor, pairs: SortedPairs, interleaved: bool = False) -> torch.Tensor:
     """silu(W_gate[e] h) * (W_up[e] h) for every sorted pair: `h` [T, d], `w_gate_up` [E, 2F, d] (an expert's F gate
     rows, then its F up rows; `interleaved`: 64 gate rows, their 64 up rows, and so on, as `interleave_gate_up` lays
@@ -108,9 +126,7 @@ def moe_gate_up(h: torch.Tensor, w_gate_up: torch.Tensor, pairs: SortedPairs, in
         raise KernelError("moe_gate_up: h [T, d] and w_gate_up [E, 2F, d] of one type are expected")
     F = F2 // 2
     out = torch.empty((pairs.rows, F), dtype=h.dtype, device=h.device)
-    _check(_fn("routed", "plm_moe_gemm")(
-        _p(h), d, pairs.top, _p(w_gate_up), _p(out), F, _dt(h, "h"), 0, _p(pairs.tile_expert), _p(pairs.sorted),
-        pairs.max_tiles, pairs.bm, F, d, 1 if interleaved else 0, _stream()),
+    _check(_few_rows(h, d, w_gate_up, out, 0, pairs, F, d, interleaved),
         f"moe_gate_up tiles<={pairs.max_tiles}x{pairs.bm} F={F} d={d}",
         flops=2 * pairs.n_tokens * pairs.top * F2 * d, nbytes=w_gate_up.numel() * w_gate_up.element_size())
     return out
@@ -124,9 +140,7 @@ def moe_up(h: torch.Tensor, w_up: torch.Tensor, pairs: SortedPairs) -> torch.Ten
     if h.dtype != w_up.dtype or h.shape != (pairs.n_tokens, d):
         raise KernelError("moe_up: h [T, d] and w_up [E, F, d] of one type are expected")
     out = torch.empty((pairs.rows, F), dtype=h.dtype, device=h.device)
-    _check(_fn("routed", "plm_moe_gemm")(
-        _p(h), d, pairs.top, _p(w_up), _p(out), F, _dt(h, "h"), 2, _p(pairs.tile_expert), _p(pairs.sorted),
-        pairs.max_tiles, pairs.bm, F, d, 0, _stream()), f"moe_up tiles<={pairs.max_tiles}x{pairs.bm} F={F} d={d}",
+    _check(_few_rows(h, d, w_up, out, 2, pairs, F, d, False), f"moe_up tiles<={pairs.max_tiles}x{pairs.bm} F={F} d={d}",
         flops=2 * pairs.n_tokens * pairs.top * F * d, nbytes=w_up.numel() * w_up.element_size())
     return out
 
@@ -138,9 +152,7 @@ def moe_down(act: torch.Tensor, w_down: torch.Tensor, pairs: SortedPairs) -> tor
     if act.dtype != w_down.dtype or act.shape != (pairs.rows, F):
         raise KernelError("moe_down: act [rows, F] and w_down [E, d, F] of one type are expected")
     out = torch.empty((pairs.rows, d), dtype=torch.float32, device=act.device)
-    _check(_fn("routed", "plm_moe_gemm")(
-        _p(act), F, pairs.top, _p(w_down), _p(out), d, _dt(act, "act"), 1, _p(pairs.tile_expert), _p(pairs.sorted),
-        pairs.max_tiles, pairs.bm, d, F, 0, _stream()), f"moe_down tiles<={pairs.max_tiles}x{pairs.bm} d={d} F={F}",
+    _check(_few_rows(act, F, w_down, out, 1, pairs, d, F, False), f"moe_down tiles<={pairs.max_tiles}x{pairs.bm} d={d} F={F}",
         flops=2 * pairs.n_tokens * pairs.top * F * d, nbytes=w_down.numel() * w_down.element_size())
     return out
 
