@@ -44,6 +44,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "recurrent": ["recurrent.cu"],
     "routed": ["routed.cu"],
     "routed_stream": ["routed_stream.cu"],
+    "routed_tc": ["routed_tc.cu"],
     "decay_chunk": ["decay_chunk.cu"],
     "delta_chunk": ["delta_chunk.cu"],
     "scan_chunk": ["scan_chunk.cu"],

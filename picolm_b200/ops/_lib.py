@@ -49,8 +49,8 @@ _SIGNATURES = {
     "plm_router_logits": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _vp],
     "plm_moe_align": [_vp, _i, _i, _i, _vp, _vp, _vp, _i, _i, _vp],
     "plm_moe_gemm": [_vp, _l, _i, _vp, _vp, _l, _i, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp],
+    "plm_moe_tc": [_vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _i, _i, _i, _l, _vp, _vp],
     "plm_moe_stream": [_vp, _l, _i, _vp, _i, _vp, _l, _i, _vp, _vp, _i, _i, _i, _i, _vp, _vp],
-    "plm_gemm_tc_wide_grouped": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _l, _l, _i, _vp, _vp, _vp],
     "plm_moe_gather": [_vp, _vp, _vp, _i, _i, _l, _vp],
     "plm_moe_combine": [_vp, _l, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _vp, _i, _vp, _f, _i, _vp],
     "plm_rope_store": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -68,6 +68,7 @@ _SIGNATURES = {
     "plm_gemm_tc_wide_pieces": [_i, _i, _i, _i, _vp, _i],
     "plm_gemm_tc_wide_how": [_i, _i, _i, _i, _i, _vp],
     "plm_gemm_tc_wide_splits": [_i, _i, _i],
+    "plm_gemm_tc_wide_grouped": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _l, _l, _i, _vp, _vp, _vp],
     "plm_gemm_tc_pair": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _l, _l, _vp, _vp],
     "plm_gemm_simt": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _l, _l, _l, _vp],
     "plm_attention_rows": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _i, _vp, _i, _vp],

@@ -215,29 +215,36 @@ def moe_tc_supported(h: torch.Tensor, w_in: torch.Tensor, w_down: torch.Tensor) 
             and wide and d % 8 == 0 and d >= 64 and w_in.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
 
-def _grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, pairs: SortedPairs, what: str,
-             store_act: Optional[str] = None) -> torch.Tensor:
+def _grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, pairs: SortedPairs, what: str) -> torch.Tensor:
+    """The experts' products on tcgen05 (`epilogue` 0 store, 1 gated, 2 squared ReLU).  Tiles of 128 sorted rows: with the
+    tokens on the MMA's 128 rows (gemm_tc_wide.cu); smaller ones, a multiple of 16: with the weights there (routed_tc.cu)."""
     E, N, K = w.shape
-    if pairs.bm != 128 or x.shape != (pairs.rows, K) or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
-        raise KernelError(f"{what}: tiles of 128 sorted rows [rows, {K}] in bfloat16 are expected")
-    lib, flags = _gated_library("gemm_tc_wide", (), store_act or "silu")
-    _check(_fn(lib, "plm_gemm_tc_wide_grouped", flags)(
-        _p(x), _p(w), _p(out), _dt(out, "out"), epilogue, pairs.rows, N, K, K, K, out.shape[1], E, _p(pairs.tile_expert),
-        _p(status_word(x.device)), _stream()), f"{what} tiles<={pairs.max_tiles}x128 N={N} K={K}",
-        flops=2 * pairs.n_tokens * pairs.top * N * K, nbytes=w.numel() * 2)
+    if pairs.bm % 16 or x.shape != (pairs.rows, K) or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        raise KernelError(f"{what}: tiles of sorted rows [rows, {K}] in bfloat16 are expected, a multiple of 16 rows each")
+    if pairs.bm == 128:
+        lib, flags = _gated_library("gemm_tc_wide", (), "relu2" if epilogue == 2 else "silu")
+        rc = _fn(lib, "plm_gemm_tc_wide_grouped", flags)(
+            _p(x), _p(w), _p(out), _dt(out, "out"), epilogue % 2, pairs.rows, N, K, K, K, out.shape[1], E, _p(pairs.tile_expert),
+            _p(status_word(x.device)), _stream())
+    else:
+        rc = _fn("routed_tc", "plm_moe_tc")(
+            _p(x), _p(w), _p(out), _dt(out, "out"), epilogue, pairs.n_tokens * pairs.top, _p(pairs.tile_expert), pairs.max_tiles,
+            pairs.bm, E, N, K, out.shape[1], _p(status_word(x.device)), _stream())
+    _check(rc, f"{what} tiles<={pairs.max_tiles}x{pairs.bm} N={N} K={K}",
+           flops=2 * pairs.n_tokens * pairs.top * N * K, nbytes=w.numel() * 2)
     return out
 
 
 def moe_up_tc(x_sorted: torch.Tensor, w_up: torch.Tensor, pairs: SortedPairs) -> torch.Tensor:
-    """`moe_up` on tcgen05 for tiles of 128 rows: `x_sorted` [rows, d] from `moe_gather`, `w_up` [E, F, d]; the squared
+    """`moe_up` on tcgen05: `x_sorted` [rows, d] from `moe_gather`, `w_up` [E, F, d]; the squared
     ReLU in the product's epilogue; [rows, F] bfloat16."""
     _dev(x_sorted, "x_sorted"), _dev(w_up, "w_up")
     out = torch.empty((pairs.rows, w_up.shape[1]), dtype=torch.bfloat16, device=x_sorted.device)
-    return _grouped(x_sorted, w_up, out, 0, pairs, "moe_up_tc", store_act="relu2")
+    return _grouped(x_sorted, w_up, out, 2, pairs, "moe_up_tc")
 
 
 def moe_gate_up_tc(x_sorted: torch.Tensor, w_gate_up: torch.Tensor, pairs: SortedPairs) -> torch.Tensor:
-    """`moe_gate_up` on tcgen05 for tiles of 128 rows: `x_sorted` [rows, d] from `moe_gather`, `w_gate_up` [E, 2F, d]
+    """`moe_gate_up` on tcgen05: `x_sorted` [rows, d] from `moe_gather`, `w_gate_up` [E, 2F, d]
     interleaved in turns of 64 rows; the activation in the product's epilogue; [rows, F] bfloat16."""
     _dev(x_sorted, "x_sorted"), _dev(w_gate_up, "w_gate_up")
     out = torch.empty((pairs.rows, w_gate_up.shape[1] // 2), dtype=torch.bfloat16, device=x_sorted.device)
@@ -245,7 +252,7 @@ def moe_gate_up_tc(x_sorted: torch.Tensor, w_gate_up: torch.Tensor, pairs: Sorte
 
 
 def moe_down_tc(act: torch.Tensor, w_down: torch.Tensor, pairs: SortedPairs) -> torch.Tensor:
-    """`moe_down` on tcgen05 for tiles of 128 rows; float32 [rows, d]."""
+    """`moe_down` on tcgen05; float32 [rows, d]."""
     _dev(act, "act"), _dev(w_down, "w_down")
     out = torch.empty((pairs.rows, w_down.shape[1]), dtype=torch.float32, device=act.device)
     return _grouped(act, w_down, out, 0, pairs, "moe_down_tc")

@@ -97,6 +97,16 @@ class PlainMLP(Part):
         return ops.linear(act, self.w_down, torch.float32, defer=True)
 
 
+# Pairs an expert on average from which the experts' products run on tcgen05.  Measured, both ways through sort, products and
+# sum: 32 experts of 2,048 x 2,048 with 9, 19 and 42 pairs each 167, 167 and 175 us against 150, 205 and 345 in tiles of 16
+# rows; 16 of 4,096 x 3,584 with 9, 19 and 56 pairs 293, 294 and 302 against 240, 384 and 865.
+TC_PAIRS = 16
+# And from which the tokens take the MMA's 128 rows instead of the weights: their tiles are nearly full by then, and a tile of
+# 128 x 256 loads less for its work than 128 weight rows with half of 300 tokens.  192, 256 and 281 pairs an expert: 222, 481
+# and 352 us with the weights on the rows, 246, 459 and 340 with the tokens there (32 experts of 2,048 x 2,048; 16 of 4,096 x 5,376).
+WIDE_PAIRS = 224
+
+
 @register_part("feed_forward", "routed_mlp")
 class RoutedMLP(Part):
     """A mixture of experts: every token uses `top` of `experts` small gated MLPs (`W_down(silu(W_gate h) * W_up h)`,
@@ -225,9 +235,9 @@ class RoutedMLP(Part):
                                             float(self.params["route_scale"]), self.gate_col, scores=self.scores,
                                             group_score=self.group_score, normalize=self.normalize)
         skip = self.identity
-        if (self.interleaved or not self.gated) and T * self.top >= 64 * self.E and ops.moe_tc_supported(h, self.w_in, self.w_down):
-            # many pairs an expert (prompts): tiles of 128 rows on tcgen05, the tokens' rows laid out in sorted order first
-            pairs = ops.moe_align(ids, self.E, 128, skip)
+        if (self.interleaved or not self.gated) and T * self.top >= TC_PAIRS * self.E and ops.moe_tc_supported(h, self.w_in, self.w_down):
+            # many pairs an expert (prompts): an expert's rows at once on tcgen05, laid out in sorted order first
+            pairs = ops.moe_align(ids, self.E, 16 if T * self.top < WIDE_PAIRS * self.E else 128, skip)
             rows = ops.moe_gather(h, pairs)
             act = ops.moe_gate_up_tc(rows, self.w_in, pairs) if self.gated else ops.moe_up_tc(rows, self.w_in, pairs)
             y = ops.moe_down_tc(act, self.w_down, pairs)
