@@ -104,7 +104,10 @@ TC_PAIRS = 16
 # And from which the tokens take the MMA's 128 rows instead of the weights: their tiles are nearly full by then, and a tile of
 # 128 x 256 loads less for its work than 128 weight rows with half of 300 tokens.  192, 256 and 281 pairs an expert: 222, 481
 # and 352 us with the weights on the rows, 246, 459 and 340 with the tokens there (32 experts of 2,048 x 2,048; 16 of 4,096 x 5,376).
+# So too where an expert's pairs fill one of those tiles (more than 104 to 128 on average): 16 experts of 4,096 x 5,376 with 121
+# pairs each take 364 us for the layer that way and 373 with the weights on the rows.
 WIDE_PAIRS = 224
+FULL_TILE_PAIRS = (104, 128)
 
 
 @register_part("feed_forward", "routed_mlp")
@@ -237,7 +240,9 @@ class RoutedMLP(Part):
         skip = self.identity
         if (self.interleaved or not self.gated) and T * self.top >= TC_PAIRS * self.E and ops.moe_tc_supported(h, self.w_in, self.w_down):
             # many pairs an expert (prompts): an expert's rows at once on tcgen05, laid out in sorted order first
-            pairs = ops.moe_align(ids, self.E, 16 if T * self.top < WIDE_PAIRS * self.E else 128, skip)
+            n, (lo, hi) = T * self.top, FULL_TILE_PAIRS
+            wide = n >= WIDE_PAIRS * self.E or lo * self.E < n <= hi * self.E
+            pairs = ops.moe_align(ids, self.E, 128 if wide else 16, skip)
             rows = ops.moe_gather(h, pairs)
             act = ops.moe_gate_up_tc(rows, self.w_in, pairs) if self.gated else ops.moe_up_tc(rows, self.w_in, pairs)
             y = ops.moe_down_tc(act, self.w_down, pairs)
