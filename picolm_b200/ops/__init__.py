@@ -19,6 +19,6 @@ from .gemm import (PLAIN_ACTIVATIONS, PendingLinear, ScaledRows, gemm_simt, gemm
 from .recurrent import (DECAY_CONST, DECAY_SIGMOID, DECAY_STEP, GATE_AFTER_NORM, GATE_BEFORE_NORM, GATE_NONE, causal_conv,  # noqa: F401
                         decay_chunk_supported, decay_powers, decay_scan, delta_prep, delta_scan, diag_scan, gated_norm, head_linear, linear_scan, rglru_gates,
                         store_rows_paged, latent_store)
-from .routed import (SortedPairs, moe_align, moe_combine, moe_down, moe_down_tc, moe_gate_up, moe_gate_up_tc,  # noqa: F401
+from .routed import (TC_EXPERTS, SortedPairs, moe_align, moe_combine, moe_down, moe_down_tc, moe_gate_up, moe_gate_up_tc,  # noqa: F401
                      moe_gather, moe_max_tiles, moe_tc_supported, moe_up, moe_up_tc, route_topk, router_logits)
 from .sampling import argmax, sample  # noqa: F401

@@ -111,7 +111,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
         raise KernelError("linear_scan: the state must be float32 with heads * key_dim * value_dim values a row")
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
     if (mode == DECAY_SIGMOID and skip is None and step.max_new >= SIGMOID_CHUNK_FROM and N <= SCAN_CHUNK_KEYS
-            and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
+            and step.n_seqs <= SCAN_CHUNK_SEQS and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
         ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
         _check(_fn("scan_chunk", "plm_sigmoid_chunk_scan")(
             _p(q), _p(k), _p(v), _p(raw), _dt(v, "v"), ldq, ldk, ldv, ldr, _p(p0), float(q_scale), float(power), _p(state), lds, _p(y),
@@ -147,6 +147,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     return y
 
 
+SCAN_CHUNK_SEQS = 65535    # the most sequences of their grids (the general scan takes more)
 SCAN_CHUNK_KEYS = 128      # the largest key size of the kernels that take a decay per channel 64 tokens at a time
 # Tokens of a step's longest sequence from which `linear_scan` (with a decay per key channel) and `delta_scan` do so.  Below,
 # token by token is faster (measured: 8 heads of 128 x 128, one sequence of 64 and of 128 tokens, linear attention 44 against

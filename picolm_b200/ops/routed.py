@@ -215,6 +215,9 @@ def moe_tc_supported(h: torch.Tensor, w_in: torch.Tensor, w_down: torch.Tensor) 
             and wide and d % 8 == 0 and d >= 64 and w_in.data_ptr() % 16 == 0 and w_down.data_ptr() % 16 == 0)
 
 
+TC_EXPERTS = 1024          # the most experts of the tcgen05 products with the weights on the rows (tiles of 128 take any number)
+
+
 def _grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: int, pairs: SortedPairs, what: str) -> torch.Tensor:
     """The experts' products on tcgen05 (`epilogue` 0 store, 1 gated, 2 squared ReLU).  Tiles of 128 sorted rows: with the
     tokens on the MMA's 128 rows (gemm_tc_wide.cu); smaller ones, a multiple of 16: with the weights there (routed_tc.cu)."""

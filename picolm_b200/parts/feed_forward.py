@@ -108,6 +108,20 @@ TC_PAIRS = 16
 # pairs each take 364 us for the layer that way and 373 with the weights on the rows.
 WIDE_PAIRS = 224
 FULL_TILE_PAIRS = (104, 128)
+# More experts than the kernel with the weights on the rows takes (ops.TC_EXPERTS): tiles of 128 of the tokens' rows, half full or
+# better, since a tile of 128 costs the same with one row as with 128.
+MANY_EXPERTS_PAIRS = 64
+
+
+def tc_tile_rows(n_pairs: int, experts: int) -> int:
+    """Rows of the tiles that `n_pairs` (token, expert) pairs are sorted into for tcgen05: 128 (the tokens on the MMA's rows),
+    16 (the weights there) or 0 (too few pairs an expert for either)."""
+    if experts > ops.TC_EXPERTS:
+        return 128 if n_pairs >= MANY_EXPERTS_PAIRS * experts else 0
+    if n_pairs < TC_PAIRS * experts:
+        return 0
+    lo, hi = FULL_TILE_PAIRS
+    return 128 if n_pairs >= WIDE_PAIRS * experts or lo * experts < n_pairs <= hi * experts else 16
 
 
 @register_part("feed_forward", "routed_mlp")
@@ -238,11 +252,10 @@ class RoutedMLP(Part):
                                             float(self.params["route_scale"]), self.gate_col, scores=self.scores,
                                             group_score=self.group_score, normalize=self.normalize)
         skip = self.identity
-        if (self.interleaved or not self.gated) and T * self.top >= TC_PAIRS * self.E and ops.moe_tc_supported(h, self.w_in, self.w_down):
+        tc_rows = tc_tile_rows(T * self.top, self.E)
+        if (self.interleaved or not self.gated) and tc_rows and ops.moe_tc_supported(h, self.w_in, self.w_down):
             # many pairs an expert (prompts): an expert's rows at once on tcgen05, laid out in sorted order first
-            n, (lo, hi) = T * self.top, FULL_TILE_PAIRS
-            wide = n >= WIDE_PAIRS * self.E or lo * self.E < n <= hi * self.E
-            pairs = ops.moe_align(ids, self.E, 128 if wide else 16, skip)
+            pairs = ops.moe_align(ids, self.E, tc_rows, skip)
             rows = ops.moe_gather(h, pairs)
             act = ops.moe_gate_up_tc(rows, self.w_in, pairs) if self.gated else ops.moe_up_tc(rows, self.w_in, pairs)
             y = ops.moe_down_tc(act, self.w_down, pairs)
