@@ -147,7 +147,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     return y
 
 
-SCAN_CHUNK_SEQS = 65535    # the most sequences of their grids (the general scan takes more)
+SCAN_CHUNK_SEQS = 65535    # the most sequences of csrc/scan_chunk.cu's grids (the general scan takes more)
 SCAN_CHUNK_KEYS = 128      # the largest key size of the kernels that take a decay per channel 64 tokens at a time
 # Tokens of a step's longest sequence from which `linear_scan` (with a decay per key channel) and `delta_scan` do so.  Below,
 # token by token is faster (measured: 8 heads of 128 x 128, one sequence of 64 and of 128 tokens, linear attention 44 against
