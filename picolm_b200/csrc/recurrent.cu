@@ -593,7 +593,7 @@ __global__ void sigmoid_decay_kernel(const T* raw, long ld, const float* bias, f
 
 extern "C" int plm_sigmoid_decay(const void* raw, int dtype, long ld, const float* bias, float power, float* out, int n_rows,
                                  int C, cudaStream_t stream) {
-    if (n_rows <= 0 || C <= 0) return PLM_ERR_SHAPE;
+    if (n_rows <= 0 || C <= 0 || !bias) return PLM_ERR_SHAPE;
     const unsigned grid = (unsigned)(((long)n_rows * C + 255) / 256);
     if (dtype == PLM_F32)
         return plm_status_of(launch_pdl(sigmoid_decay_kernel<float>, dim3(grid), dim3(256), 0, stream, (const float*)raw, ld, bias,

@@ -805,6 +805,7 @@ extern "C" int plm_sigmoid_chunk_scan(const void* q, const void* k, const void* 
                                       long ldr, const float* bias, float q_scale, float power, float* state, long state_stride, float* y,
                                       float* ws, const int* seq_start, const int* seq_slot, int n_seqs, int max_new, int H, int N, int P,
                                       int heads_per_group, cudaStream_t stream) {
+    if (!bias) return PLM_ERR_SHAPE;
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     const Args a = {q, k, v, raw, ldq, ldk, ldv, ldr, nullptr, bias, power, q_scale, ws, state, state_stride, y, seq_start, seq_slot,
                     H, N, P, heads_per_group, 0,
