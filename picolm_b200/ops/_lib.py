@@ -352,6 +352,14 @@ def set_bounds(library: str, extra_flags=(), *, n_pages: int = 0, n_seqs: int = 
         raise KernelError(f"plm_check_bounds: CUDA error {code}")
 
 
+# What the status word says: what the checked build met (csrc/common.cuh), or whose wait ran out.
+_OUT_OF_BOUNDS = {16: "page number", 17: "sequence index", 18: "position", 19: "row index"}
+_WAITS = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting", 5: "a decode step's pages", 40: "the walk over chunks",
+          41: "the experts' streamed weights", 42: "the experts' streamed products", 43: "the experts' streamed rows",
+          51: "the experts' TMA producer", 52: "the experts' MMA issuer, results unread", 53: "the experts' MMA issuer",
+          54: "the experts' epilogue"}
+
+
 def check_status(device="cuda:0") -> None:
     """Raise if a kernel gave up a bounded wait since the last check (this
     synchronises with the device)."""
@@ -361,10 +369,8 @@ def check_status(device="cuda:0") -> None:
     code = int(t.item())
     if code:
         t.zero_()
-        if code >= 16:
-            what = {16: "page number", 17: "sequence index", 18: "position", 19: "row index"}.get(code, str(code))
-            raise KernelError(f"a kernel of the checked build met a {what} outside its bounds and did not follow it; "
+        if code in _OUT_OF_BOUNDS:
+            raise KernelError(f"a kernel of the checked build met a {_OUT_OF_BOUNDS[code]} outside its bounds and did not follow it; "
                               f"its output is not valid")
-        where = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting"}.get(code, str(code))
-        raise KernelError(f"a tensor-core kernel gave up waiting on an mbarrier ({where}); its output is not valid")
+        raise KernelError(f"a kernel gave up waiting on an mbarrier ({_WAITS.get(code, code)}); its output is not valid")
 
