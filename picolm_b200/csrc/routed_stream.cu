@@ -153,7 +153,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_1, const __grid_consta
 #pragma unroll
             for (int m = 0; m < NACC; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0.f;
             for (int s = 0; s < n_stages; ++s, ++i) {
-                if (!mbar_wait(full0 + 8 * (i % STAGES), (i / STAGES) & 1, status, 42)) { ok = false; s_abort = 1; break; }
+                if (!mbar_wait_warp(full0 + 8 * (i % STAGES), (i / STAGES) & 1, status, 42)) { ok = false; s_abort = 1; break; }
                 if (mine) {
                     const uint8_t* stage = smem_raw + (base - raw) + (i % STAGES) * Ring<MODE>::STAGE;
                     const uint8_t* at = stage + (half * GN + row) * 128;             // [64 of K][columns of the unit][128 bytes]

@@ -17,12 +17,37 @@ using namespace plm_tc;
 
 namespace {
 
+// A test build only (-DPLM_TEST_GIVE_UP, never the library that serves): while the switch is 1, the loader announces 64 bytes
+// more for every stage than it loads, so that every wait runs out; while it is 2, one warp of the eight that read results
+// acts as if its wait for its CTA's second unit had run out.  The kernel must record it, let what it has in flight land, free
+// its tensor memory and return.
+#ifdef PLM_TEST_GIVE_UP
+__device__ int plm_give_up_switch = 0;
+#define PLM_STALL_BYTES (plm_give_up_switch == 1 ? 64u : 0u)
+#define PLM_GIVES_UP(warp, unit) (plm_give_up_switch == 2 && (warp) == 3 && (unit) == 1)
+#else
+#define PLM_STALL_BYTES 0u
+#define PLM_GIVES_UP(warp, unit) false
+#endif
+
 constexpr int FT = 128, EPI_WARPS = 8, THREADS = (2 + EPI_WARPS) * 32;
 constexpr uint32_t W_SLAB = FT * 128, RING_BYTES = 196608;              // 64 of K of the weight rows; all stages
 constexpr int MAX_GROUPS = 1024;
 constexpr uint32_t TURN = 2 * 16 * 64 * 4;             // what the gate's and the up branch's threads hand each other, an accumulator
 constexpr size_t SMEM = (size_t)RING_BYTES + 2 * TURN + 1024 + 256;
 enum { STORE = 0, GATED = 1, RELU2 = 2 };
+
+// Whether all 128 threads of a named barrier say yes.
+__device__ __forceinline__ bool set_agrees(int barrier, bool yes) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, %2, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(all) : "r"(yes ? 1u : 0u), "r"(barrier) : "memory");
+    return all != 0;
+}
 
 struct Unit { int row, n, f0, group; };                // first sorted row, its tokens (a multiple of 16), first weight row, expert
 
@@ -106,7 +131,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                 for (int k = 0; k < n_k; ++k, ++i) {
                     const uint32_t bar = full0 + 8 * (i % RING), dst = base + (i % RING) * STAGE;
                     if (*(volatile int*)&s_abort || !mbar_wait(empty0 + 8 * (i % RING), ((i / RING) & 1) ^ 1, status, 51)) { s_abort = 1; break; }
-                    mbar_expect_tx(bar, W_BYTES + SLABS * box * 64 * 128);
+                    mbar_expect_tx(bar, W_BYTES + SLABS * box * 64 * 128 + PLM_STALL_BYTES);
                     if (SLABS > 1) {
                         tma_load_3d(dst, &map_w, bar, x.group * F + x.f0, k * SLABS);
                         tma_load_3d(dst + W_BYTES, map_x, bar, x.row, k * SLABS);
@@ -123,7 +148,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMAs
         if (lane == 0) {
-            int i = 0, done = 0;
+            int i = 0, done = 0, handed = 0;           // stages consumed, units begun, units handed to the warps that read them
             bool ok = true;
             for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++done) {
                 const Unit x = unit_at(u);
@@ -143,11 +168,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
                                         smem_desc_sw128(t + s * x_slab) + (uint64_t)(j * 2), idesc, (k > 0 || s > 0 || j > 0) ? 1u : 0u);
                     tc_commit(empty0 + 8 * (i % RING));
                 }
-                if (ok) tc_commit(acc_full0 + 8 * acc);
+                if (ok) { tc_commit(acc_full0 + 8 * acc); ++handed; }
             }
             if (!ok) s_abort = 1;
-            // the last commits have to arrive before the barriers go
-            for (int s = max(0, i - RING); s < i && ok; ++s) mbar_wait(empty0 + 8 * (s % RING), (s / RING) & 1, nullptr, 0);
+            // what was issued has to be done, and its commits to have arrived, before the tensor memory and the barriers go
+            for (int s = max(0, i - RING); s < i; ++s) mbar_wait(empty0 + 8 * (s % RING), (s / RING) & 1, nullptr, 0);
+            for (int x = max(0, handed - 2); x < handed; ++x) mbar_wait(acc_full0 + 8 * (x & 1), (x >> 1) & 1, nullptr, 0);
         }
     } else {
         // ------------------------------------------------------------ results: two sets of four warps, 32 tokens in turn
@@ -162,7 +188,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
             const int acc = done & 1, f = EPI == GATED ? x.f0 / 2 + (r & 63) : x.f0 + r;
             const bool in_f = f < (EPI == GATED ? F / 2 : F);
             const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + acc * NMAX;
-            if (!mbar_wait(acc_full0 + 8 * acc, (done >> 1) & 1, status, 54)) { s_abort = 1; break; }
+            // One verdict for all that meet below: the lanes of a warp (tcgen05.ld), and with a gate the four warps of a set (the
+            // barriers around what they hand each other have no limit of their own).
+            bool there = mbar_wait_warp(acc_full0 + 8 * acc, (done >> 1) & 1, status, 54);
+            if (PLM_GIVES_UP(warp, done)) { atomicCAS(status, 0, 54); there = false; }
+            if (EPI == GATED) there = set_agrees(1 + set, there);
+            if (!there) { s_abort = 1; break; }
             tc_fence_after();
             for (int c = set * 32; c < x.n; c += 64) {
                 uint32_t v[32];
@@ -259,3 +290,9 @@ extern "C" int plm_moe_tc(const void* x, const void* w, void* out, int out_dtype
     if (out_dtype != PLM_F32) return PLM_ERR_DTYPE;
     return launch<STORE, float>(x, w, out, ldo, n_pairs, tile_expert, max_tiles, bm, E, F, K, status, stream);
 }
+
+#ifdef PLM_TEST_GIVE_UP
+extern "C" int plm_test_give_up(int how, cudaStream_t stream) {
+    return plm_status_of(cudaMemcpyToSymbolAsync(plm_give_up_switch, &how, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
+}
+#endif

@@ -41,6 +41,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
     if (status) atomicCAS(status, 0, where);
     return false;
 }
+// The same for a whole warp, whose lanes leave with one verdict: what follows may be an instruction that all of them take.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int where) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, where));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -49,6 +49,53 @@ def test_a_wait_that_runs_out_is_reported_not_hung():
     assert torch.allclose(out.double().cpu(), ref, atol=2e-3, rtol=1e-4)
 
 
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+@pytest.mark.parametrize("how", [1, 2])
+def test_the_experts_product_gives_up_as_one(epilogue, how):
+    """The same for the experts' product with the weights on the MMA's rows, whose gated epilogue has barriers inside sets of
+    four warps: with no stage ever filling (1), and with a single warp that gives up on its CTA's second unit while the others
+    go on (2), the kernel says so and returns; switched off again the same library gives the right product."""
+    from picolm_b200 import ops
+    from picolm_b200.csrc.build import load_library
+    from picolm_b200.ops import _lib
+    lib = load_library("routed_tc@give_up", ["-DPLM_WAIT_LIMIT=20000", "-DPLM_TEST_GIVE_UP"])
+    lib.plm_moe_tc.argtypes = _lib._SIGNATURES["plm_moe_tc"]
+    lib.plm_test_give_up.argtypes = [ctypes.c_int, ctypes.c_void_p]
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    E, F, K, T = 8, 8192, 128, 100                              # 512 units or more: every CTA has at least three
+    torch.manual_seed(5)
+    ids = torch.randint(0, E, (T, 1), device=DEV, dtype=torch.int32)
+    pairs = ops.moe_align(ids, E, 16)
+    x = ops.moe_gather((torch.randn(T, K, device=DEV) / K ** 0.25).to(torch.bfloat16), pairs)
+    w = (torch.randn(E, F, K, device=DEV) / K ** 0.25).to(torch.bfloat16)
+    out = torch.zeros((pairs.rows, F // 2 if epilogue == 1 else F), dtype=torch.bfloat16 if epilogue else torch.float32, device=DEV)
+    status = ops.status_word(DEV)
+    ops.check_status(DEV)
+
+    def product():
+        return lib.plm_moe_tc(x.data_ptr(), w.data_ptr(), out.data_ptr(), 1 if epilogue else 0, epilogue, T, pairs.tile_expert.data_ptr(),
+                              pairs.max_tiles, pairs.bm, E, F, K, out.shape[1], status.data_ptr(), stream)
+
+    assert lib.plm_test_give_up(how, stream) == 0
+    assert product() == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) in ((51, 52, 53, 54) if how == 1 else (54,))
+    with pytest.raises(ops.KernelError, match="gave up waiting"):
+        ops.check_status(DEV)
+    assert lib.plm_test_give_up(0, stream) == 0
+    assert product() == 0
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    used = pairs.sorted >= 0
+    z = torch.einsum("rk,rnk->rn", x[used].double(), w.double()[pairs.tile_expert.long().repeat_interleave(16)[used]])
+    if epilogue == 1:
+        z = z.view(len(z), F // 128, 2, 64)
+        z = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(len(z), F // 2)
+    elif epilogue == 2:
+        z = torch.relu(z) ** 2
+    assert torch.allclose(out[used].double(), z, atol=2e-3 if epilogue == 0 else 2e-2, rtol=1e-4 if epilogue == 0 else 1.2e-2)
+
+
 CHECKED_SCRIPT = r'''
 import os, sys, json
 sys.path.insert(0, sys.argv[1]); sys.path.insert(0, os.path.join(sys.argv[1], "tests"))
