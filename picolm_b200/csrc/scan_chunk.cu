@@ -534,7 +534,7 @@ chunk_walk_kernel(const Args a) {
             }
         }
         __syncthreads();
-        if (owns) {
+        if (owns && n < N) {                             // (padding stays zero, whatever U holds)
             float4 sum = part[tid];
 #pragma unroll
             for (int i = 1; i < SPLITS; ++i) sum = add4(sum, part[i * 8 * NG + tid]);
@@ -652,7 +652,8 @@ chunk_outer_kernel(const Args a) {
 #pragma unroll
         for (int x = 0; x < PT / 64; ++x) {
             const int n = n0 + r / 4 * 32 + ty * 4 + r % 4, p = p0 + x * 64 + tx * 4;
-            if (n < NP && p < PP) *reinterpret_cast<float4*>(w + Lay::s(PP) + (long)n * PP + p) = four(acc, r, x);
+            if (n < NP && p < PP)                        // (padding stays zero, whatever U holds)
+                *reinterpret_cast<float4*>(w + Lay::s(PP) + (long)n * PP + p) = n < a.N ? four(acc, r, x) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 }
 
@@ -701,7 +702,23 @@ chunk_chain_kernel(const Args a) {
     }
 }
 
-// O = Q S + M U of one chunk; grid (chunk x columns by PT, sequence, head)
+// One result of the kernel below from the rows that its token sees: the same sum in the same order.
+template <int NP>
+__device__ __noinline__ float one_output(const float* w, int PP, int t, int p) {
+    using Lay = Layout<NP>;
+    float sum = 0.f;
+    for (int n = 0; n < NP; ++n) sum = fmaf(w[Lay::QT + n * C + t], w[Lay::s(PP) + (long)n * PP + p], sum);
+    for (int s = 0; s <= t; ++s) sum = fmaf(w[Lay::MT + s * C + t], w[Lay::U + (long)s * PP + p], sum);
+    return sum;
+}
+template <int NP> __device__ __forceinline__ float seen_only(float sum, const float* w, int PP, int t, int p) {
+    return fabsf(sum) < INFINITY ? sum : one_output<NP>(w, PP, t, p);
+}
+
+// O = Q S + M U of one chunk; grid (chunk x columns by PT, sequence, head).  M is multiplied whole, zeros above its diagonal
+// included; where a later token's row of U holds an infinity or no number, those products are no zeros, and a sum that comes
+// out so is taken once more without them.  (Leaving them out of the tiles' steps, by steps and a select in the step on the
+// diagonal, took 2 to 3 % of a mixer's time.)
 template <int NP, int PT>
 __global__ void __launch_bounds__(128)
 chunk_out_kernel(const Args a) {
@@ -730,7 +747,10 @@ chunk_out_kernel(const Args a) {
 #pragma unroll
         for (int x = 0; x < PT / 64; ++x) {
             const int p = p0 + x * 64 + tx * 4;
-            const float4 v = four(acc, r, x);
+            float4 v = four(acc, r, x);
+            if (p < P && !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY))
+                v = make_float4(seen_only<NP>(v.x, w, PP, t, p), seen_only<NP>(v.y, w, PP, t, p + 1), seen_only<NP>(v.z, w, PP, t, p + 2),
+                                seen_only<NP>(v.w, w, PP, t, p + 3));
             if (P % 4 == 0) {
                 if (p < P) *reinterpret_cast<float4*>(y + p) = v;
             } else {

@@ -90,3 +90,59 @@ def test_linear_attention_in_chunks(lens, H, G, N, P, dtype):
     o, S = _recurrence(wide(q) * N ** -0.5, wide(k), v.double().reshape(T, H, P), d, None, state0, lens)
     assert _off(y.view(T, H, P), o) < BOUND and _off(state.view(-1, H, N, P)[:len(lens)], S) < BOUND
     assert torch.equal(state[len(lens)], state0[len(lens)].view(-1))
+
+
+def _rows_before(lens, poisoned):
+    """Per token: whether what it sees (its own sequence up to itself) is clean of the poisoned tokens."""
+    out, at = [], 0
+    for n in lens:
+        bad = False
+        for t in range(at, at + n):
+            bad = bad or t in poisoned
+            out.append(not bad)
+        at += n
+    return torch.tensor(out, device=DEV)
+
+
+@pytest.mark.parametrize("H,G,N,P", [(2, 1, 128, 128), (3, 3, 48, 72), (2, 2, 100, 33)])
+@pytest.mark.parametrize("where", ["v", "k", "q", "decay"])
+@pytest.mark.parametrize("what", [float("inf"), float("nan")])
+@pytest.mark.parametrize("rule", ["channel", "head", "linear"])
+def test_what_is_not_finite_reaches_no_earlier_token(H, G, N, P, where, what, rule):
+    """Poisoned tokens at the places of a block of four, of sixteen and of a chunk: the tokens before them and the other
+    sequences have the bits that they have without, and one value column of v touches that column alone."""
+    from picolm_b200 import ops
+    lens = [200, 96, 130]
+    T, step, poisoned = sum(lens), _step(lens), {2, 61, 200 + 79, 200 + 96 + 128}
+    torch.manual_seed(N + P)
+    x = {n: torch.randn(T, c, device=DEV) for n, c in (("q", G * N), ("k", G * N), ("v", H * P), ("decay", H if rule == "head" else H * N))}
+    x["k"] = torch.nn.functional.normalize(x["k"].view(T, G, N), dim=-1).reshape(T, G * N).contiguous()
+    if rule != "linear":
+        x["decay"] = -x["decay"].abs()
+    beta, bias = torch.rand(T, H, device=DEV), torch.rand(H * N, device=DEV)
+    state0 = torch.randn(len(lens), H * N * P, device=DEV)
+
+    def run(x):
+        state = state0.clone()
+        if rule == "linear":
+            y = ops.linear_scan(x["q"], x["k"], x["v"], x["decay"], ops.DECAY_SIGMOID, bias, None, None, 1.0, 1 / 16, state, step, H, N, P,
+                                heads_per_group=H // G)
+        else:
+            y = ops.delta_scan(x["q"], x["k"], torch.ones(T, G, device=DEV), x["decay"], beta, x["v"], state, step, H, N, P,
+                               heads_per_group=H // G, head_decay=rule == "head")
+        return y
+    clean = run(x)
+    assert torch.isfinite(clean).all()
+    column = 5                                                           # of the first head
+    for t in poisoned:
+        if where == "v":
+            x["v"][t, column] = what
+        else:
+            x[where][t] = what if where != "decay" or rule == "linear" else -abs(what)
+    y = run(x)
+    before = _rows_before(lens, poisoned)
+    assert before.sum() > 100 and torch.equal(y[before], clean[before])
+    if where == "v":
+        others = torch.arange(H * P, device=DEV) != column
+        assert torch.equal(y[:, others], clean[:, others])
+        assert not torch.isfinite(y[sorted(poisoned), column]).any()
