@@ -95,7 +95,7 @@ template <typename T, int NP, bool DELTA>
 __global__ void __launch_bounds__(PREP_THREADS)
 chunk_prep_kernel(const Args a) {
     constexpr int LD = NP + 4, SEG = C * NP / PREP_THREADS;
-    static_assert(SEG % B4 == 0 && NB * 32 == PREP_THREADS && PAIRS * 4 <= PREP_THREADS, "threads");
+    static_assert(SEG % B4 == 0 && NB * 32 == PREP_THREADS && PAIRS * 4 <= PREP_THREADS && PAIRS * 4 % 32 == 0, "threads");
     using Lay = Layout<NP>;
     using Tk = typename std::conditional<DELTA, float, T>::type;         // the delta rule's q and k come in float32
     extern __shared__ __align__(16) float sm[];
@@ -314,8 +314,7 @@ chunk_prep_kernel(const Args a) {
                 }
             }
         }
-        // the four lanes' sums: the first two end with A, the others with M, each with two of the four s
-        const unsigned lanes = __activemask();
+        // the four lanes' sums: the first two end with A, the others with M, each with two of the four s (whole warps are here)
         float r[4][2];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -323,12 +322,12 @@ chunk_prep_kernel(const Args a) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const float give = part & 2 ? x[i][j] : m[i][j];
-                y[j] = (part & 2 ? m[i][j] : x[i][j]) + __shfl_xor_sync(lanes, give, 2);
+                y[j] = (part & 2 ? m[i][j] : x[i][j]) + __shfl_xor_sync(0xffffffffu, give, 2);
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const float give = part & 1 ? y[j] : y[j + 2];
-                r[i][j] = (part & 1 ? y[j + 2] : y[j]) + __shfl_xor_sync(lanes, give, 1);
+                r[i][j] = (part & 1 ? y[j + 2] : y[j]) + __shfl_xor_sync(0xffffffffu, give, 1);
             }
         }
         const int t = I * B4;
