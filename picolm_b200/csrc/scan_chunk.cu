@@ -533,7 +533,7 @@ chunk_walk_kernel(const Args a) {
             }
         }
         __syncthreads();
-        if (owns && n < N) {                             // (padding stays zero, whatever U holds)
+        if (owns) {
             float4 sum = part[tid];
 #pragma unroll
             for (int i = 1; i < SPLITS; ++i) sum = add4(sum, part[i * 8 * NG + tid]);
@@ -701,22 +701,9 @@ chunk_chain_kernel(const Args a) {
     }
 }
 
-// One result of the kernel below from the rows that its token sees: the same sum in the same order.
-template <int NP>
-__device__ __noinline__ float one_output(const float* w, int PP, int t, int p) {
-    using Lay = Layout<NP>;
-    float sum = 0.f;
-    for (int n = 0; n < NP; ++n) sum = fmaf(w[Lay::QT + n * C + t], w[Lay::s(PP) + (long)n * PP + p], sum);
-    for (int s = 0; s <= t; ++s) sum = fmaf(w[Lay::MT + s * C + t], w[Lay::U + (long)s * PP + p], sum);
-    return sum;
-}
-template <int NP> __device__ __forceinline__ float seen_only(float sum, const float* w, int PP, int t, int p) {
-    return fabsf(sum) < INFINITY ? sum : one_output<NP>(w, PP, t, p);
-}
-
 // O = Q S + M U of one chunk; grid (chunk x columns by PT, sequence, head).  M is multiplied whole, zeros above its diagonal
-// included; where a later token's row of U holds an infinity or no number, those products are no zeros, and a sum that comes
-// out so is taken once more without them.  (Leaving them out of the tiles' steps, by steps and a select in the step on the
+// included; where a later token's row of U holds an infinity or no number, those products are no zeros, and a thread with a sum
+// that comes out so takes its sums once more without them.  (Leaving them out of the tiles' steps, by steps and a select in the step on the
 // diagonal, took 2 to 3 % of a mixer's time.)
 template <int NP, int PT>
 __global__ void __launch_bounds__(128)
@@ -738,6 +725,7 @@ chunk_out_kernel(const Args a) {
         pb = w + (j < 0 ? Lay::s(PP) + (long)i * TK * PP : Lay::U + (long)j * TK * PP) + p0;
     });
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    bool finite = true;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int t = r / 4 * 32 + ty * 4 + r % 4;
@@ -746,10 +734,8 @@ chunk_out_kernel(const Args a) {
 #pragma unroll
         for (int x = 0; x < PT / 64; ++x) {
             const int p = p0 + x * 64 + tx * 4;
-            float4 v = four(acc, r, x);
-            if (p < P && !(fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY))
-                v = make_float4(seen_only<NP>(v.x, w, PP, t, p), seen_only<NP>(v.y, w, PP, t, p + 1), seen_only<NP>(v.z, w, PP, t, p + 2),
-                                seen_only<NP>(v.w, w, PP, t, p + 3));
+            const float4 v = four(acc, r, x);
+            if (p < P) finite = finite && fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY;
             if (P % 4 == 0) {
                 if (p < P) *reinterpret_cast<float4*>(y + p) = v;
             } else {
@@ -760,6 +746,18 @@ chunk_out_kernel(const Args a) {
             }
         }
     }
+    if (!finite)                         // (rare: the same sums in the same order, over the rows that a token sees)
+#pragma unroll 1
+        for (int i = 0; i < 8 * (PT / 16); ++i) {
+            const int t = i % 8 / 4 * 32 + ty * 4 + i % 4, p = p0 + i / 32 * 64 + tx * 4 + i / 8 % 4;
+            if (t >= nt || p >= P) continue;
+            float sum = 0.f;
+#pragma unroll 1
+            for (int n = 0; n < NP; ++n) sum = fmaf(w[Lay::QT + n * C + t], w[Lay::s(PP) + (long)n * PP + p], sum);
+#pragma unroll 1
+            for (int s = 0; s <= t; ++s) sum = fmaf(w[Lay::MT + s * C + t], w[Lay::U + (long)s * PP + p], sum);
+            a.y[(long)(t0 + t) * a.H * P + (long)h * P + p] = sum;
+        }
 }
 
 template <int NP, typename T, bool DELTA, int PT>
