@@ -90,7 +90,8 @@ template <int NP> constexpr size_t prep_smem() {
 // logarithms and none a difference of running sums, where a strong decay's large sum would take the low digits of its
 // neighbours' (2,048 tokens: 2.2e-6 off in the state with running sums, 2.2e-7 this way).
 // Bound by shared memory (a float4 a lane is four of its cycles a warp), so products are tiles of 4 x 4 pairs of tokens a
-// lane, with the channels dealt to four neighbouring lanes.  grid (chunk of the sequence, sequence, head)
+// lane, with the channels dealt to four neighbouring lanes.  grid (chunk of the sequence, head, sequence: a captured
+// step's sequences without tokens come last)
 template <typename T, int NP, bool DELTA>
 __global__ void __launch_bounds__(PREP_THREADS)
 chunk_prep_kernel(const Args a) {
@@ -110,7 +111,7 @@ chunk_prep_kernel(const Args a) {
     float* bt = between + PAIRS * NP;    // [C] beta, 0 behind the last token
     pdl_launch_dependents();
     pdl_wait();
-    const int c = blockIdx.x, b = blockIdx.y, h = blockIdx.z, tid = threadIdx.x;
+    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
     const int s0 = a.seq_start[b], s1 = a.seq_start[b + 1], t0 = s0 + c * C;
     if (t0 >= s1) return;
     const int nt = min(C, s1 - t0), N = a.N, P = a.P, PP = pad4(P), H = a.H, g = h / a.heads_per_group;
@@ -626,7 +627,7 @@ template <int TN> __device__ __forceinline__ float4 four(const uint64_t (&acc)[4
 }
 
 // Linear attention: what a chunk adds to the state, sum_s (k_s e^(L_C - L_s)) v_s^T, into the state's place in the workspace.
-// grid (chunk x channels by 64 x columns by PT, sequence, head)
+// grid (chunk x channels by 64 x columns by PT, head, sequence)
 template <int NP, int PT>
 __global__ void __launch_bounds__(128)
 chunk_outer_kernel(const Args a) {
@@ -636,7 +637,7 @@ chunk_outer_kernel(const Args a) {
     pdl_launch_dependents();
     pdl_wait();
     const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, n0 = blockIdx.x / ptiles % MT * 64, c = blockIdx.x / ptiles / MT, b = blockIdx.y, h = blockIdx.z;
+    const int p0 = blockIdx.x % ptiles * PT, n0 = blockIdx.x / ptiles % MT * 64, c = blockIdx.x / ptiles / MT, h = blockIdx.y, b = blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
     float* w = a.ws + ((long)(s0 / C + b + c) * a.H + h) * Lay::floats(PP);
@@ -701,7 +702,7 @@ chunk_chain_kernel(const Args a) {
     }
 }
 
-// O = Q S + M U of one chunk; grid (chunk x columns by PT, sequence, head).  M is multiplied whole, zeros above its diagonal
+// O = Q S + M U of one chunk; grid (chunk x columns by PT, head, sequence).  M is multiplied whole, zeros above its diagonal
 // included; where a later token's row of U holds an infinity or no number, those products are no zeros, and a thread with a sum
 // that comes out so takes its sums once more without them.  (Leaving them out of the tiles' steps, by steps and a select in the step on the
 // diagonal, took 2 to 3 % of a mixer's time.)
@@ -713,7 +714,7 @@ chunk_out_kernel(const Args a) {
     pdl_launch_dependents();
     pdl_wait();
     const int P = a.P, PP = pad4(P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, c = blockIdx.x / ptiles, b = blockIdx.y, h = blockIdx.z;
+    const int p0 = blockIdx.x % ptiles * PT, c = blockIdx.x / ptiles, h = blockIdx.y, b = blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
     const float* w = a.ws + ((long)(s0 / C + b + c) * a.H + h) * Lay::floats(PP);
@@ -767,7 +768,7 @@ int run(const Args& a, int n_seqs, int max_new, cudaStream_t stream) {
     if (prep_ok != cudaSuccess) return (int)prep_ok;
     const unsigned chunks = (unsigned)((max_new + C - 1) / C);
     const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
-    cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, n_seqs, a.H), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
+    cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, a.H, n_seqs), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
     if (e != cudaSuccess) return (int)e;
     if (DELTA) {
         static const cudaError_t walk_ok =
@@ -776,12 +777,12 @@ int run(const Args& a, int n_seqs, int max_new, cudaStream_t stream) {
         e = launch_pdl(chunk_walk_kernel<NP>, dim3((unsigned)((long)n_seqs * a.H * ((a.P + WC - 1) / WC))), dim3(WALK_THREADS), walk_smem<NP>(),
                        stream, a);
     } else {
-        e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP > 64 ? NP / 64 : 1), n_seqs, a.H), dim3(128), 0, stream, a);
+        e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP > 64 ? NP / 64 : 1), a.H, n_seqs), dim3(128), 0, stream, a);
         if (e != cudaSuccess) return (int)e;
         e = launch_pdl(chunk_chain_kernel<NP>, dim3((NP * (PP / 4) + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a);
     }
     if (e != cudaSuccess) return (int)e;
-    return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks * ptiles, n_seqs, a.H), dim3(128), 0, stream, a));
+    return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks * ptiles, a.H, n_seqs), dim3(128), 0, stream, a));
 }
 
 template <typename T, bool DELTA>

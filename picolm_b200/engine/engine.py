@@ -21,7 +21,7 @@ from ..config.registry import read_config, spec_of
 from ..runtime import Runtime
 from ..weights.loader import load_weights
 from .model import Model
-from .step_batch import build_step_batch
+from .step_batch import StepShape, build_step_batch
 
 
 class Engine:
@@ -57,7 +57,10 @@ class Engine:
             # table needs every launch between two events
             self.use_graphs = False
         self._graphs: Dict[Tuple[int, int], "DecodeGraph"] = {}
-        self._prompt_graphs: Dict[Tuple[int, int], "PromptGraph"] = {}
+        self._prompt_graphs: Dict[tuple, "PromptGraph"] = {}
+        # parts that choose by a step's shape, one of each kind (layers of one kind choose alike)
+        choosers = {(type(part), repr(sorted(part.params.items()))): part for part in parts if getattr(part, "chooses_by_shape", False)}
+        self._choosers = list(choosers.values())
         # steps with prompts replay a graph too where every sequence wants its last token's logits (generation);
         # float32 runs launch them kernel by kernel (their kernels take longer than the launches)
         import os
@@ -237,12 +240,14 @@ class Engine:
         key = (token_class(n_tokens), seq_class(n))
         if key[0] is None or key[1] is None:
             return None, False
+        shape = StepShape.of([len(toks) for _, toks in entries])
+        key += tuple(part.step_route(shape) for part in self._choosers)
         n_want = sum(len(w) for w in wants)
         if n_want not in (0, n) or (n_want and any(list(w) != [len(toks) - 1] for w, (_, toks) in zip(wants, entries))):
             return None, False
         g = self._prompt_graphs.get(key)
         if g is None:
-            g = PromptGraph(self, key[0], key[1])
+            g = PromptGraph(self, key[0], key[1], shape)
             g.capture()
             self._prompt_graphs[key] = g
         logits = g.run(entries)

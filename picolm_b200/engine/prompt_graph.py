@@ -9,6 +9,10 @@ points at the cache's null page and whose state row is the null slot, so that wh
 where nothing reads it; no sequence of the step covers them (`seq_start` ends before them), so attention
 skips them, and every other kernel works row by row, so whatever their rows hold stays in their rows.
 Sequences are padded with sequences of no tokens.  Logits are computed for the last token of every sequence.
+
+A graph serves the batches of its size class for which every part that goes by the sequences' lengths chooses what it
+chose when the graph was captured (`Part.step_route`): a step of many short prompts and one of a long prompt have one size
+and are not run alike.
 """
 from __future__ import annotations
 
@@ -17,7 +21,7 @@ from typing import List, Optional, Sequence, Tuple
 import numpy as np
 import torch
 
-from .step_batch import StepBatch
+from .step_batch import StepBatch, StepShape
 
 # padded token counts: steps of 64 up to 512, of 128 up to 1,024, of 256 up to 2,048
 TOKEN_CLASSES = tuple(range(64, 513, 64)) + tuple(range(640, 1025, 128)) + tuple(range(1280, 2049, 256))
@@ -39,7 +43,7 @@ def seq_class(n: int) -> Optional[int]:
 
 
 class PromptGraph:
-    def __init__(self, engine, tokens: int, seqs: int):
+    def __init__(self, engine, tokens: int, seqs: int, shape: Optional[StepShape] = None):
         self.engine = engine
         self.T, self.n_real = tokens, seqs
         self.B = B = seqs + 1                               # the last sequence takes the padding tokens' writes
@@ -64,7 +68,7 @@ class PromptGraph:
             max_position=cache.max_seq_tokens - 1, max_new=T, is_decode=False,
             tok_ids=self.d[0], tok_seq=self.d[1], tok_pos=self.d[2], seq_slot=self.d[3], seq_start=self.d[4],
             seq_kv_len=self.d[5], want_rows=self.d[6],
-            block_tables=[self.d[7 + g].view(B, P) for g in range(n_groups)], h2d_bytes=int(self.host_np.nbytes))
+            block_tables=[self.d[7 + g].view(B, P) for g in range(n_groups)], shape=shape, h2d_bytes=int(self.host_np.nbytes))
         self.copied = torch.cuda.Event()
         self.replayed: Optional[torch.cuda.Event] = None
         self.graph: Optional[torch.cuda.CUDAGraph] = None

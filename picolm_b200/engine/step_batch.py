@@ -10,6 +10,8 @@ from typing import List, Optional, Sequence
 import numpy as np
 import torch
 
+from ..ops.recurrent import StepShape
+
 
 @dataclass
 class StepBatch:
@@ -33,6 +35,9 @@ class StepBatch:
     seq_kv_len: torch.Tensor              # int32 [B]  length after this step
     want_rows: torch.Tensor               # int32 [n_want] flat token indices
     block_tables: List[torch.Tensor]      # per kv group: int32 [B, pages per sequence]
+    # host: what the sequences bring; in a captured step, what those of the batch it was captured for bring: it serves the
+    # batches of its size for which every part chooses alike (`Part.step_route`)
+    shape: Optional[StepShape] = None
     h2d_bytes: int = 0                    # size of the one host-to-device copy that brought all of the above
     _seq_slot_long: Optional[torch.Tensor] = None
 
@@ -103,5 +108,5 @@ def build_step_batch(entries: Sequence[tuple], wants: Sequence[Sequence[int]], c
         tok_ids=dviews[0], tok_seq=dviews[1], tok_pos=dviews[2], seq_slot=dviews[3], seq_start=dviews[4],
         seq_kv_len=dviews[5], want_rows=dviews[6],
         block_tables=[dviews[7 + gi].view(B, P) for gi in range(n_groups)],
-        h2d_bytes=int(host.nbytes),
+        shape=StepShape.of(new_lens), h2d_bytes=int(host.nbytes),
     )

@@ -3,13 +3,35 @@ delta_chunk.cu): the depthwise causal convolution, the gated linear recurrence, 
 written into the pages of a cache."""
 from __future__ import annotations
 
-from typing import Optional
+from typing import NamedTuple, Optional, Sequence
 
 import torch
 
 from ._lib import PAGE_TOKENS, KernelError, _check, _dev, _dt, _fn, _i32, _p, _stream, set_bounds, status_word
 
 DECAY_STEP, DECAY_SIGMOID, DECAY_GIVEN, DECAY_CONST = 1, 2, 3, 4
+
+
+class StepShape(NamedTuple):
+    """What a step's sequences bring, for what is chosen by it: a captured step's `max_new`, `n_seqs` and `n_tokens` are
+    the bounds of all batches it serves and say little about the one at hand."""
+    longest: int        # the most tokens of a sequence
+    tokens: int
+    seqs: int
+    chunks: int         # chunks of 64 tokens, each sequence's counted by itself
+
+    @staticmethod
+    def of(lens: Sequence[int]) -> "StepShape":
+        return StepShape(max(lens), sum(lens), len(lens), sum((n + 63) // 64 for n in lens))
+
+
+def step_shape(step) -> StepShape:
+    """The shape that the step was made with, else what its bounds allow."""
+    shape = getattr(step, "shape", None)
+    if shape is None:
+        longest, seqs = int(step.max_new), int(step.n_seqs)
+        shape = StepShape(longest, int(step.n_tokens), seqs, min(step.n_tokens // 64 + seqs, seqs * ((longest + 63) // 64)))
+    return shape
 
 
 def _cols(t: torch.Tensor, name: str) -> int:
@@ -75,8 +97,9 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
       DECAY_CONST    raw None: d = p0[h] for the whole head and every token; with `activation="silu"` q, k and v pass
                      SiLU on their way in (float32, from the rows as they are)
     `state` float32 [slots, >= heads * key_dim * value_dim] with contiguous rows holds S of every sequence as
-    [heads, key_dim, value_dim] and is carried on.  Prompts with a decay per key channel run 64 tokens at a time
-    (csrc/scan_chunk.cu) where the sizes allow it."""
+    [heads, key_dim, value_dim] and is carried on.  Prompts with a decay per key channel and no skip run 64 tokens at a time
+    (csrc/scan_chunk.cu) where that is faster (`linear_scan_route`: it depends on all sequences of the step, and with it the
+    order of the sums)."""
     if raw is None and mode == DECAY_CONST:
         raw = v                                              # (not read)
     if activation not in (None, "silu") or (activation and mode != DECAY_CONST):
@@ -110,8 +133,10 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     if state.dtype != torch.float32 or state.shape[1] < H * N * P:
         raise KernelError("linear_scan: the state must be float32 with heads * key_dim * value_dim values a row")
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
-    if (mode == DECAY_SIGMOID and skip is None and step.max_new >= SIGMOID_CHUNK_FROM and N <= SCAN_CHUNK_KEYS
-            and step.n_seqs <= SCAN_CHUNK_SEQS and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
+    route = None
+    if mode == DECAY_SIGMOID and skip is None and N <= SCAN_CHUNK_KEYS:
+        route = linear_scan_route(step_shape(step), H, N, P)
+    if (route == IN_CHUNKS and step.n_seqs <= SCAN_CHUNK_SEQS and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
         ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
         _check(_fn("scan_chunk", "plm_sigmoid_chunk_scan")(
             _p(q), _p(k), _p(v), _p(raw), _dt(v, "v"), ldq, ldk, ldv, ldr, _p(p0), float(q_scale), float(power), _p(state), lds, _p(y),
@@ -122,7 +147,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
         return y
     # Long prompts are cut into segments that run side by side: a first pass leaves what each segment adds to the
     # state, a small kernel chains those into the state at every segment's start, a second pass gives y.
-    seg_len, n_segs = scan_plan(step.n_seqs, H, N, P, step.max_new, T)
+    seg_len, n_segs = (step.max_new, 1) if route == ONE_PASS else scan_plan(step.n_seqs, H, N, P, step.max_new, T)
     seg_state = seg_decay = None
     kernels, run_mode = 1, mode
     if n_segs > 1:
@@ -149,11 +174,50 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
 
 SCAN_CHUNK_SEQS = 65535    # the most sequences of csrc/scan_chunk.cu's grids (the general scan takes more)
 SCAN_CHUNK_KEYS = 128      # the largest key size of the kernels that take a decay per channel 64 tokens at a time
-# Tokens of a step's longest sequence from which `linear_scan` (with a decay per key channel) and `delta_scan` do so.  Below,
-# token by token is faster (measured: 8 heads of 128 x 128, one sequence of 64 and of 128 tokens, linear attention 44 against
-# 34 us and 42 against 62, delta rule 46 against 58 and 64 against 114; 32 sequences of 16: 88 against 39, 190 against 57).
+ONE_PASS, IN_CHUNKS = 1, 2
+
+# When 64 tokens at a time are faster than token by token, as a cost of both in microseconds, fitted to what was measured: one to 32
+# sequences of 16 to 400 tokens, and steps that mix a long one with many short, 8 and 16 heads.  Token by token a sequence's tokens are
+# a chain and all heads' states pass the same memory; in chunks a sequence of one token costs a whole chunk, so what counts
+# is the chunks and not the tokens.
+# Linear attention, 8 heads of 128 x 256, token by token against chunks: one sequence of 96 tokens 49 against 44, of 128 63 against
+# 42; 2 and 4 of 96 49 against 56 and 63 against 65; 16 of 128 183 against 131; 100 tokens beside 31 sequences of 16 84 against 142.
+# From 192 tokens on the general scan runs in segments, twice, where sequences leave SMs idle: 200 tokens 87 against 49.
 SIGMOID_CHUNK_FROM = 96
-DELTA_CHANNEL_CHUNK_FROM = 64
+
+
+def linear_scan_route(shape: StepShape, heads: int, key_dim: int, value_dim: int) -> int:
+    """How `linear_scan` with a decay per key channel (at most `SCAN_CHUNK_KEYS` of them) runs a step of this shape."""
+    longest, tokens, seqs, chunks = shape
+    if longest < SIGMOID_CHUNK_FROM:
+        return ONE_PASS
+    if seqs == 1 or scan_plan(seqs, heads, key_dim, value_dim, longest, tokens)[1] > 1:
+        return IN_CHUNKS
+    size = (key_dim / 128) ** 0.5
+    work, prepared = heads * size * value_dim / 256, heads * size * (0.5 + value_dim / 512)
+    token_by_token = 0.42 * longest + 0.0078 * work * tokens
+    return IN_CHUNKS if token_by_token >= 48 + 0.36 * prepared * chunks else ONE_PASS
+
+
+# The delta rule, 8 heads of 128 x 128: one sequence of 48, 64 and 128 tokens 45 against 41, 59 against 44 and 114 against 65;
+# 32 of 16 tokens 57 against 190, of 128 564 against 305; 64 tokens beside 63 single ones 69 against 355, 1,000 beside 8 of 20 892
+# against 137.  (In chunks of 32, the kernel of larger keys, 61, 61, 79, 171, 545, 269 and 300.)
+# By the padded key size: a step's chunks: microseconds at all, a chunk and head, a sequence and head; token by token: a token of the
+# longest sequence, a token and head.
+DELTA_CHUNK_FROM_SHORTEST, DELTA_CHANNEL_CHUNK_FROM = 48, 64      # with one or two sequences, with more
+_DELTA_COSTS = {64: (30.0, 0.276, 0.064, 0.56, 0.0034), 128: (40.0, 0.38, 0.27, 0.88, 0.0107)}
+
+
+def delta_scan_in_chunks(shape: StepShape, heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether `delta_scan` runs a step of this shape 64 tokens at a time in float32 (keys of at most `SCAN_CHUNK_KEYS`)."""
+    longest, tokens, seqs, chunks = shape
+    if longest < (DELTA_CHUNK_FROM_SHORTEST if seqs <= 2 else DELTA_CHANNEL_CHUNK_FROM):
+        return False
+    fixed, chunk, seq, chain, token = _DELTA_COSTS[64 if key_dim <= 64 else 128]
+    work = heads * value_dim / 128
+    return chain * longest + token * work * tokens > fixed + work * (chunk * chunks + seq * seqs)
+
+
 SCAN_CHUNK_FLOATS = 1 << 31      # the most workspace that linear attention takes for it (some 4.8 KB a token and head of 128 x 256)
 _chunk_floats = {}
 
@@ -497,11 +561,14 @@ def diag_scan(a: torch.Tensor, x: torch.Tensor, y_raw: torch.Tensor, y_bias: Opt
 _head_chunk_bytes = {}
 
 
+def delta_head_chunk_sizes(key_dim: int, value_dim: int) -> bool:
+    return key_dim % 16 == 0 and key_dim <= 128 and value_dim % 8 == 0
+
+
 def delta_head_chunk_supported(v: torch.Tensor, state: torch.Tensor, key_dim: int, value_dim: int) -> bool:
     """Whether the delta rule with one decay a head can run prompts on the tensor cores: values in bfloat16, a key size
     that is a multiple of 16 up to 128, a value size that is a multiple of 8."""
-    return (v.dtype == torch.bfloat16 and key_dim % 16 == 0 and key_dim <= 128 and value_dim % 8 == 0
-            and state.stride(0) % 2 == 0 and state.data_ptr() % 16 == 0)
+    return (v.dtype == torch.bfloat16 and delta_head_chunk_sizes(key_dim, value_dim) and state.stride(0) % 2 == 0 and state.data_ptr() % 16 == 0)
 
 
 DELTA_CHUNK_FROM = 16      # tokens of a step's longest sequence from which the delta rule runs chunk by chunk
@@ -555,10 +622,10 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
     (the read-out sees the token's own write; with `head_decay` one decay a head).  qn, kn, qk, decay (its logarithm), beta as `delta_prep` returns them; v [T, heads *
     value_dim] (a column slice will do); `state` float32 [slots, >= heads * key_dim * value_dim] with contiguous
     rows holds S as [heads, key_dim, value_dim] and is carried on.  Returns o, float32 [T, heads * value_dim].
-    A step whose longest sequence brings `DELTA_CHUNK_FROM` tokens or more runs chunk by chunk (what does not depend on the
-    state for all chunks side by side, then a walk over each sequence's chunks; with one decay a head and values in bfloat16
-    on the tensor cores, else 64 tokens at a time in float32, csrc/scan_chunk.cu); shorter portions and single tokens run
-    token by token."""
+    Prompts run chunk by chunk (what does not depend on the state for all chunks side by side, then a walk over each
+    sequence's chunks): with one decay a head and values in bfloat16 on the tensor cores, with keys of more than
+    `SCAN_CHUNK_KEYS` values 32 tokens at a time, both from `DELTA_CHUNK_FROM` tokens of the longest sequence on; all others 64 at a
+    time in float32 (csrc/scan_chunk.cu) where that is faster (`delta_scan_in_chunks`).  The rest runs token by token."""
     H, N, P = heads, key_dim, value_dim
     T = v.shape[0]
     if H % heads_per_group:
@@ -594,7 +661,7 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
             nbytes=T * (8 * G * N + H * P * (4 + v.element_size())) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (3 * N * P + 64 // 2 * (2 * N + N + 2 * P)))
         return y
-    if channel and step.max_new >= DELTA_CHANNEL_CHUNK_FROM:
+    if channel and delta_scan_in_chunks(step_shape(step), H, N, P):
         ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
         _check(_fn("scan_chunk", "plm_delta_channel_scan")(
             _p(qn), _p(kn), _p(decay), _p(beta), _p(v), _dt(v, "v"), ldv, _p(state), lds, _p(y), _p(ws), _p(step.seq_start),

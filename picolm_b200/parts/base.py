@@ -71,6 +71,12 @@ class Part:
     # host, not even `step.slots` or `step.new_lens` (they are None in a captured step), and rows that belong to no
     # sequence (padding) may hold anything.  Steps with prompts replay graphs only if every part says so.
     graph_safe_prompts: bool = False
+    # Whether forward() runs a step with prompts in different ways by what its sequences bring (`step.shape`).  `step_route`
+    # then says in which, and a captured step is replayed only for shapes with the same answer.
+    chooses_by_shape: bool = False
+
+    def step_route(self, shape):
+        return None
 
     def __init__(self, params: Mapping[str, Any], runtime: Optional[Runtime]):
         self.params = dict(params)

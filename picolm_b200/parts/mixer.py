@@ -329,6 +329,13 @@ class ParallelMixers(Part):
     def graph_safe_prompts(self) -> bool:
         return all(bool(getattr(part, "graph_safe_prompts", False)) for _, part in self.halves)
 
+    @property
+    def chooses_by_shape(self) -> bool:
+        return any(getattr(part, "chooses_by_shape", False) for _, part in self.halves)
+
+    def step_route(self, shape):
+        return tuple(part.step_route(shape) for _, part in self.halves if getattr(part, "chooses_by_shape", False))
+
     def weight_specs(self):
         return {self._join(prefix, name): ws for prefix, part in self.halves + (self.norms or [])
                 for name, ws in part.weight_specs().items()}

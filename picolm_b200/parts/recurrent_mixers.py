@@ -134,6 +134,13 @@ class GatedLinearAttention(_StateMixer):
     def cache_spec(self):
         return CacheSpec.state((self.H * self.N * self.P,))
 
+    @property
+    def chooses_by_shape(self) -> bool:
+        return self.N <= ops.SCAN_CHUNK_KEYS
+
+    def step_route(self, shape):
+        return ops.linear_scan_route(shape, self.H, self.N, self.P)
+
     def forward(self, h, step, cache):
         dt = self.runtime.dtype
         HN, HP = self.H * self.N, self.H * self.P
@@ -409,6 +416,13 @@ class GatedDeltaRule(_StateMixer):
     def cache_spec(self):
         # one row per sequence: S as [heads, dim, vdim], then the convolution's last inputs
         return CacheSpec.state((self.n_state + self.n_conv,))
+
+    @property
+    def chooses_by_shape(self) -> bool:
+        return self.N <= ops.SCAN_CHUNK_KEYS and not (self.head_decay and ops.delta_head_chunk_sizes(self.N, self.P))
+
+    def step_route(self, shape):
+        return ops.delta_scan_in_chunks(shape, self.H, self.N, self.P)
 
     def _narrow_product(self, cols, w, dt):
         # a bottleneck of a few columns: the CUDA-core product reads them where they lie; a wide one is copied out
