@@ -314,6 +314,24 @@ int launch_f32_few(const void* A, const void* W, void* C, int M, int N, int K, l
     return plm_launch_status();
 }
 
+// The form whose waves of blocks take the least time: measured microseconds at K = 2,048 (all grow with K alike) of a wave with
+// one, two or three blocks an SM, three or two being what an SM holds.
+int f32_form(int M, int N) {
+    struct Form { int bm, bn, per_sm, us[3]; };
+    constexpr Form FORMS[] = {{8, 16, 3, {21, 29, 37}}, {32, 16, 3, {30, 43, 56}}, {32, 32, 2, {49, 72, 0}},
+                              {64, 64, 3, {142, 170, 219}}, {64, 128, 2, {187, 258, 0}}};
+    int best = 0;
+    long best_us = -1;
+    for (int f = 0; f < 5; ++f) {
+        const Form& form = FORMS[f];
+        const long rows = (M + form.bm - 1) / form.bm, blocks = rows * ((N + form.bn - 1) / form.bn);
+        const long wave = (long)form.per_sm * PLM_SM_COUNT, rest = (blocks % wave + PLM_SM_COUNT - 1) / PLM_SM_COUNT;
+        const long us = blocks / wave * form.us[form.per_sm - 1] + (rest ? form.us[rest - 1] : 0);
+        if (rows <= 65535 && (best_us < 0 || us < best_us)) { best = f; best_us = us; }
+    }
+    return best;
+}
+
 template <typename Ta, typename Tw, typename To>
 int launch(const void* A, const void* W, void* C, int M, int N, int K, long lda, long ldw, long ldc,
            cudaStream_t stream) {
@@ -333,20 +351,7 @@ extern "C" int plm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dt
     if ((M + BM - 1) / BM > 65535) return PLM_ERR_SHAPE;
     if (a_dtype == PLM_F32 && w_dtype == PLM_F32 && c_dtype == PLM_F32 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
         !(((uintptr_t)A | (uintptr_t)W) & 15)) {
-        // The form whose waves of blocks take the least time: measured microseconds at K = 2,048 (all grow with K alike) of a
-        // wave with one, two or three blocks an SM, three or two being what an SM holds.
-        struct Form { int bm, bn, per_sm, us[3]; };
-        constexpr Form FORMS[] = {{8, 16, 3, {21, 29, 37}}, {32, 16, 3, {30, 43, 56}}, {32, 32, 2, {49, 72, 0}},
-                                  {64, 64, 3, {142, 170, 219}}, {64, 128, 2, {187, 258, 0}}};
-        int best = 0;
-        long best_us = -1;
-        for (int f = 0; f < 5; ++f) {
-            const Form& form = FORMS[f];
-            const long rows = (M + form.bm - 1) / form.bm, blocks = rows * ((N + form.bn - 1) / form.bn);
-            const long wave = (long)form.per_sm * PLM_SM_COUNT, rest = (blocks % wave + PLM_SM_COUNT - 1) / PLM_SM_COUNT;
-            const long us = blocks / wave * form.us[form.per_sm - 1] + (rest ? form.us[rest - 1] : 0);
-            if (rows <= 65535 && (best_us < 0 || us < best_us)) { best = f; best_us = us; }
-        }
+        const int best = f32_form(M, N);
         if (best == 0) return launch_f32_few<8, 16>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         if (best == 1) return launch_f32_few<32, 16>(A, W, C, M, N, K, lda, ldw, ldc, stream);
         if (best == 2) return launch_f32_few<32, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
@@ -365,3 +370,6 @@ extern "C" int plm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dt
         return launch<bf16, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     return PLM_ERR_DTYPE;
 }
+
+// Which of the float32 forms a product of M rows and N columns takes: 8 x 16, 32 x 16, 32 x 32 (few rows), 64 x 64, 64 x 128.
+extern "C" int plm_gemm_simt_form(int M, int N) { return f32_form(M, N); }

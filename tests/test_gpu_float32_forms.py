@@ -7,11 +7,26 @@ import torch
 
 from test_gpu_kernels import DEV, DT, _paged
 
-pytestmark = pytest.mark.gpu
+SIZES = [(M, N, K) for M in (1, 8, 9, 32, 33, 65, 200, 530) for N, K in ((16, 4), (130, 20), (129, 100), (300, 64), (2064, 132))]
+# ragged edges of each of the five tiles, by rows and by columns
+SIZES += [(5, 2070, 132), (24, 4100, 132), (24, 8190, 132), (61, 4100, 36), (150, 8190, 36), (462, 2050, 132), (462, 16390, 132), (530, 32001, 36)]
 
 
-@pytest.mark.parametrize("N,K", [(16, 4), (130, 20), (129, 100), (300, 64), (2064, 132)])
-@pytest.mark.parametrize("M", [1, 8, 9, 32, 33, 65, 200, 530])
+def _form(M, N):
+    from picolm_b200.csrc.build import load_library
+    return load_library("gemm_simt").plm_gemm_simt_form(M, N)
+
+
+def test_every_form_of_the_float32_product_is_tested():
+    """(8 x 16, 32 x 16, 32 x 32, 64 x 64, 64 x 128: at least two sizes each, with rows and columns that end inside a tile)"""
+    tiles = [(8, 16), (32, 16), (32, 32), (64, 64), (64, 128)]
+    for form, (bm, bn) in enumerate(tiles):
+        of_it = [(M, N) for M, N, _ in SIZES if _form(M, N) == form]
+        assert len(of_it) >= 2 and any(M % bm and N % bn for M, N in of_it), (form, of_it)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", SIZES)
 def test_float32_product_forms_agree_to_the_bit(M, N, K):
     """Few rows, many rows, ragged edges of every tile: against the general kernel (which takes rows that do not start on
     16-byte boundaries), against float64, and row by row."""
@@ -29,6 +44,7 @@ def test_float32_product_forms_agree_to_the_bit(M, N, K):
     assert ((out.double() - ref).abs() <= bound).all()
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,G,hd", [(5, 5, 16), (6, 2, 48), (16, 4, 64), (8, 1, 128), (4, 2, 80), (3, 1, 256), (80, 2, 32)])
 @pytest.mark.parametrize("extra", [False, True])
