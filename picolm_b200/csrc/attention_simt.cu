@@ -102,10 +102,12 @@ attention_rows_kernel(const Ta* q, const Tc* kc, const Tc* vc,
     }
 }
 
-// The same for prompts: a block takes 32 (token, query head) rows of one KV head, eight a warp, and brings the keys and
-// values of 32 positions into shared memory once for all of them.  Without a mask every row's groups of 32 keys start at
-// position 0, so a row sees the operations of the kernel above in the same order, bit for bit: how tokens are cut into
-// steps does not show.  A block whose tokens belong to several sequences walks one sequence's keys after the other.
+// The same for prompts: a block takes 32 (token, query head) rows of one sequence and KV head, eight a warp, and brings the
+// keys and values of 32 positions into shared memory once for all of them.  Without a mask every row's groups of 32 keys start
+// at position 0, so a row sees the operations of the kernel above in the same order, bit for bit: how tokens are cut into
+// steps does not show.  A sequence's tiles begin at block seq_start * (heads a KV head) / 32 + its number, so that single
+// tokens beside a prompt have blocks of their own (tiles over several sequences walked their keys one after the other: 8
+// tokens beside 63 single ones of 2,048 positions, 32 heads of 64, 1.9 ms by the kernel above, 12.3 by such tiles).
 // Bound by shared memory (9 loads of 16 bytes for 32 multiply-adds); the kernel above reads every key's row from the
 // second-level cache, a lane a row: 462 tokens of two sequences, 32 heads of 64 over 8, float32: 632 -> 75 us.
 constexpr int TILE_ROWS = 32, ROWS_A_WARP = TILE_ROWS / WARPS;
@@ -123,18 +125,27 @@ static size_t tile_smem(int hd, int max_hd) { return (size_t)(32 * (hd + 4) + 32
 template <typename T, int MAX_HD>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_tile_kernel(const T* q, const T* kc, const T* vc, T* __restrict__ out, const int* tok_pos, const int* tok_seq,
-                      const int* block_table, int max_pages, int n_tokens, int H, int G, int hd, float scale, const float* sink,
-                      const float* slopes) {
+                      const int* seq_start, int n_seqs, const int* block_table, int max_pages, int H, int G, int hd, float scale,
+                      const float* sink, const float* slopes) {
     constexpr int VEC = MAX_HD / 32, R = ROWS_A_WARP;
     extern __shared__ __align__(16) float tile_sm[];
     float* ks = tile_sm;                            // [32][hd + 4]
     float* vs = ks + 32 * (hd + 4);                 // [32][MAX_HD], zero from hd on
     float* qs = vs + 32 * MAX_HD;                   // [TILE_ROWS][hd]
     float* ps = qs + TILE_ROWS * hd;                // [TILE_ROWS][32]
+    __shared__ int warps_last[WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quads = hd / 4;
     const int per = H / G, g = blockIdx.y;
-    const long pair0 = (long)blockIdx.x * TILE_ROWS, n_pairs = (long)n_tokens * per;
-    const int t_first = (int)(pair0 / per), t_last = (int)((min(pair0 + TILE_ROWS, n_pairs) - 1) / per);
+    // the sequence whose tiles this block is among: the last that begins at or before it
+    int b = -1;
+    for (int from = 0; from < n_seqs; from += WARPS * 32) {
+        const int i = from + threadIdx.x;
+        b += __syncthreads_count(i < n_seqs && (long)seq_start[i] * per / TILE_ROWS + i <= (long)blockIdx.x);
+    }
+    if (b < 0) return;
+    const long tile = (long)blockIdx.x - ((long)seq_start[b] * per / TILE_ROWS + b);
+    const long pair0 = (long)seq_start[b] * per + tile * TILE_ROWS, n_pairs = (long)seq_start[b + 1] * per;
+    if (pair0 >= n_pairs) return;
 
     for (int i = threadIdx.x; i < TILE_ROWS * quads; i += WARPS * 32) {
         const long pair = pair0 + i / quads;
@@ -145,109 +156,104 @@ attention_tile_kernel(const T* q, const T* kc, const T* vc, T* __restrict__ out,
     for (int i = threadIdx.x; i < 32 * (MAX_HD - hd); i += WARPS * 32) vs[i / (MAX_HD - hd) * MAX_HD + hd + i % (MAX_HD - hd)] = 0.f;
 
     float acc[R][VEC], m[R], l[R], slope[R];
-    int tok[R], pos[R];
+    int tok[R], seen[R];                            // a row's token and position, -1 behind the sequence's last row
+    int warp_last = -1, warp_first = 0x7fffffff;    // of the warp's rows: the largest and the smallest position
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const long pair = pair0 + warp * R + r;
         tok[r] = pair < n_pairs ? (int)(pair / per) : -1;
-        pos[r] = tok[r] >= 0 ? PLM_POSITION(tok_pos[tok[r]]) : -1;
+        seen[r] = tok[r] >= 0 ? PLM_POSITION(tok_pos[tok[r]]) : -1;
+        warp_last = max(warp_last, seen[r]);
+        warp_first = min(warp_first, seen[r]);
         slope[r] = slopes && tok[r] >= 0 ? slopes[g * per + pair % per] : 0.f;
         m[r] = -1e30f;
         l[r] = 0.f;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) acc[r][i] = 0.f;
     }
-    for (int ta = t_first, tb; ta <= t_last; ta = tb) {                  // the tile's tokens of one sequence: ta .. tb - 1
-        const int seq = tok_seq[ta];
-        int last_key = PLM_POSITION(tok_pos[ta]);
-        for (tb = ta + 1; tb <= t_last && tok_seq[tb] == seq; ++tb) last_key = max(last_key, PLM_POSITION(tok_pos[tb]));
-        const int* pages = block_table + (size_t)PLM_SEQ_NO(seq) * max_pages;
-        int warp_last = -1, warp_first = 0x7fffffff;                     // of the warp's rows: the largest and the smallest position
-        int seen[R];                                                     // a row's position, -1 where it is not this sequence's
+    if (lane == 0) warps_last[warp] = warp_last;
+    const int* pages = block_table + (size_t)PLM_SEQ_NO(tok_seq[pair0 / per]) * max_pages;
+    __syncthreads();
+    int last_key = -1;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            seen[r] = tok[r] >= ta && tok[r] < tb ? pos[r] : -1;
-            warp_last = max(warp_last, seen[r]);
-            warp_first = min(warp_first, seen[r]);
+    for (int w = 0; w < WARPS; ++w) last_key = max(last_key, warps_last[w]);
+    for (int base = 0; base <= last_key; base += 32) {
+        __syncthreads();                                             // what was there has been read (and q is there)
+        for (int i = threadIdx.x; i < 32 * quads; i += WARPS * 32) {
+            const int j = i / quads, c = i % quads * 4, key = base + j;
+            float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
+            if (key <= last_key) {
+                const size_t at = (((size_t)PLM_PAGE_NO(pages[key / PLM_PAGE]) * G + g) * PLM_PAGE + key % PLM_PAGE) * hd + c;
+                kv = load4<T>(kc + at);
+                vv = load4<T>(vc + at);
+            }
+            *reinterpret_cast<float4*>(ks + j * (hd + 4) + c) = kv;
+            *reinterpret_cast<float4*>(vs + j * MAX_HD + c) = vv;
         }
-        for (int base = 0; base <= last_key; base += 32) {
-            __syncthreads();                                             // what was there has been read (and q is there)
-            for (int i = threadIdx.x; i < 32 * quads; i += WARPS * 32) {
-                const int j = i / quads, c = i % quads * 4, key = base + j;
-                float4 kv = make_float4(0.f, 0.f, 0.f, 0.f), vv = kv;
-                if (key <= last_key) {
-                    const size_t at = (((size_t)PLM_PAGE_NO(pages[key / PLM_PAGE]) * G + g) * PLM_PAGE + key % PLM_PAGE) * hd + c;
-                    kv = load4<T>(kc + at);
-                    vv = load4<T>(vc + at);
-                }
-                *reinterpret_cast<float4*>(ks + j * (hd + 4) + c) = kv;
-                *reinterpret_cast<float4*>(vs + j * MAX_HD + c) = vv;
-            }
-            __syncthreads();
-            if (base > warp_last) continue;
-            float dot[R];
+        __syncthreads();
+        if (base > warp_last) continue;
+        float dot[R];
 #pragma unroll
-            for (int r = 0; r < R; ++r) dot[r] = 0.f;
-            const float* kr = ks + lane * (hd + 4);
-            const float* qr = qs + warp * R * hd;
+        for (int r = 0; r < R; ++r) dot[r] = 0.f;
+        const float* kr = ks + lane * (hd + 4);
+        const float* qr = qs + warp * R * hd;
 #pragma unroll 2
-            for (int i = 0; i < hd; i += 4) {
-                const float4 kv = *reinterpret_cast<const float4*>(kr + i);
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float4 qv = *reinterpret_cast<const float4*>(qr + r * hd + i);
-                    dot[r] = fmaf(qv.w, kv.w, fmaf(qv.z, kv.z, fmaf(qv.y, kv.y, fmaf(qv.x, kv.x, dot[r]))));
-                }
-            }
-            float* pr = ps + warp * R * 32;
+        for (int i = 0; i < hd; i += 4) {
+            const float4 kv = *reinterpret_cast<const float4*>(kr + i);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                const bool valid = base + lane <= seen[r];
-                float s = -1e30f;
-                if (valid) {
-                    s = __fmul_rn(dot[r], scale);
-                    if (slopes) s = fmaf(-slope[r], (float)(seen[r] - base - lane), s);
-                }
-                const float m_new = fmaxf(m[r], warp_max(s));
-                const float corr = expf(m[r] - m_new);
-                const float p = valid ? expf(s - m_new) : 0.f;
-                l[r] = fmaf(l[r], corr, warp_sum(p));
-                m[r] = m_new;
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) acc[r][i] *= corr;
-                pr[r * 32 + lane] = p;
+                const float4 qv = *reinterpret_cast<const float4*>(qr + r * hd + i);
+                dot[r] = fmaf(qv.w, kv.w, fmaf(qv.z, kv.z, fmaf(qv.y, kv.y, fmaf(qv.x, kv.x, dot[r]))));
             }
-            __syncwarp();
-            const bool whole = warp_first >= base + 31;                  // every row sees all of the group's keys
+        }
+        float* pr = ps + warp * R * 32;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool valid = base + lane <= seen[r];
+            float s = -1e30f;
+            if (valid) {
+                s = __fmul_rn(dot[r], scale);
+                if (slopes) s = fmaf(-slope[r], (float)(seen[r] - base - lane), s);
+            }
+            const float m_new = fmaxf(m[r], warp_max(s));
+            const float corr = expf(m[r] - m_new);
+            const float p = valid ? expf(s - m_new) : 0.f;
+            l[r] = fmaf(l[r], corr, warp_sum(p));
+            m[r] = m_new;
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) acc[r][i] *= corr;
+            pr[r * 32 + lane] = p;
+        }
+        __syncwarp();
+        const bool whole = warp_first >= base + 31;                  // every row sees all of the group's keys
 #pragma unroll 2
-            for (int j = 0; j < 32; j += 4) {
-                float v[4][VEC];
+        for (int j = 0; j < 32; j += 4) {
+            float v[4][VEC];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int i = 0; i < VEC; i += (VEC >= 4 ? 4 : 2)) {
+                    const float* at = vs + (j + k) * MAX_HD + lane * VEC + i;
+                    if (VEC >= 4) {
+                        const float4 x = *reinterpret_cast<const float4*>(at);
+                        v[k][i] = x.x; v[k][i + 1] = x.y; v[k][(i + 2) % VEC] = x.z; v[k][(i + 3) % VEC] = x.w;
+                    } else {
+                        const float2 x = *reinterpret_cast<const float2*>(at);
+                        v[k][i] = x.x; v[k][i + 1] = x.y;
+                    }
+                }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const float4 p4 = *reinterpret_cast<const float4*>(pr + r * 32 + j);
+                const float p[4] = {p4.x, p4.y, p4.z, p4.w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
+                    if (whole || base + j + k <= seen[r])            // (a value that a row does not see may be anything)
 #pragma unroll
-                    for (int i = 0; i < VEC; i += (VEC >= 4 ? 4 : 2)) {
-                        const float* at = vs + (j + k) * MAX_HD + lane * VEC + i;
-                        if (VEC >= 4) {
-                            const float4 x = *reinterpret_cast<const float4*>(at);
-                            v[k][i] = x.x; v[k][i + 1] = x.y; v[k][(i + 2) % VEC] = x.z; v[k][(i + 3) % VEC] = x.w;
-                        } else {
-                            const float2 x = *reinterpret_cast<const float2*>(at);
-                            v[k][i] = x.x; v[k][i + 1] = x.y;
-                        }
-                    }
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float4 p4 = *reinterpret_cast<const float4*>(pr + r * 32 + j);
-                    const float p[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (whole || base + j + k <= seen[r])            // (a value that a row does not see may be anything)
-#pragma unroll
-                            for (int i = 0; i < VEC; ++i) acc[r][i] = fmaf(p[k], v[k][i], acc[r][i]);
-                }
+                        for (int i = 0; i < VEC; ++i) acc[r][i] = fmaf(p[k], v[k][i], acc[r][i]);
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -271,16 +277,15 @@ attention_tile_kernel(const T* q, const T* kc, const T* vc, T* __restrict__ out,
 }  // namespace
 
 // q [T, H, hd] and out [T, H, hd] have the activation type, the cache its own;
-// both are PLM_F32 or both PLM_BF16.  `longest`: the most tokens a sequence brings (1: not known).
+// both are PLM_F32 or both PLM_BF16.  seq_start [n_seqs + 1] or null: where the step's sequences' rows begin.
 extern "C" int plm_attention_rows(const void* q, const void* kc, const void* vc, void* out, int dtype,
                                   const int* tok_pos, const int* tok_seq, const int* block_table, int max_pages,
                                   int n_tokens, int H, int G, int hd, float scale, int window, const float* sink,
-                                  int keep, const float* slopes, int longest, cudaStream_t stream) {
+                                  int keep, const float* slopes, const int* seq_start, int n_seqs, cudaStream_t stream) {
     if (n_tokens <= 0) return PLM_OK;
     if (H <= 0 || G <= 0 || H % G || hd <= 0 || hd > MAX_HD || keep < 0) return PLM_ERR_SHAPE;
-    // Prompts without a mask: tiles of rows that share their keys.  From eight tokens on: a tile of fewer holds several
-    // sequences, whose keys it would walk one after the other.
-    if (longest >= 8 && !window && !keep && hd % 4 == 0 && hd <= 256 && G <= 65535 &&
+    // Prompts without a mask: tiles of a sequence's rows that share their keys (the caller says where that pays).
+    if (seq_start && n_seqs > 0 && !window && !keep && hd % 4 == 0 && hd <= 256 && G <= 65535 &&
         !(((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15)) {
 #define TILE_LAUNCH(T_, MAXHD_)                                                                                             \
     do {                                                                                                                    \
@@ -289,10 +294,10 @@ extern "C" int plm_attention_rows(const void* q, const void* kc, const void* vc,
                                  (int)tile_smem(MAXHD_, MAXHD_));                                                           \
         if (configured != cudaSuccess) return (int)configured;                                                              \
         const long pairs = (long)n_tokens * (H / G);                                                                        \
-        attention_tile_kernel<T_, MAXHD_><<<dim3((unsigned)((pairs + TILE_ROWS - 1) / TILE_ROWS), G), WARPS * 32,            \
+        attention_tile_kernel<T_, MAXHD_><<<dim3((unsigned)((pairs + TILE_ROWS - 1) / TILE_ROWS + n_seqs), G), WARPS * 32,            \
                                             tile_smem(hd, MAXHD_), stream>>>(                                               \
-            (const T_*)q, (const T_*)kc, (const T_*)vc, (T_*)out, tok_pos, tok_seq, block_table, max_pages, n_tokens, H, G, \
-            hd, scale, sink, slopes);                                                                                       \
+            (const T_*)q, (const T_*)kc, (const T_*)vc, (T_*)out, tok_pos, tok_seq, seq_start, n_seqs, block_table,     \
+            max_pages, H, G, hd, scale, sink, slopes);                                                                      \
         return plm_launch_status();                                                                                         \
     } while (0)
 #define TILE_BY_SIZE(T_)                     \

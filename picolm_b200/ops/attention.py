@@ -11,13 +11,25 @@ from ._lib import (PAGE_TOKENS, SM_COUNT, KernelError, _check, _dev, _dt, _fn, _
                    status_word)
 
 
+# When `attention_rows` shares keys between rows: from eight rows of a sequence on, where some row sees 32 keys or more or the
+# rows are many.  Below, a warp a row is done before a tile has its first keys: one sequence of 8 and of 16 tokens 7 and 10 us against
+# 12 and 13, four of 10 10 against 13 (32 heads of 64 over 8); of 24 15 against 13, of 32 20 against 13, 32 sequences of 9 26 against 17.
+TILE_FROM, TILE_KEYS, TILE_ROWS = 8, 32, 8192
+
+
+def shares_keys(longest: int, max_position: int, rows: int) -> bool:
+    return longest >= TILE_FROM and (max_position + 1 >= TILE_KEYS or rows >= TILE_ROWS)
+
+
 def attention_rows(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, tok_pos: torch.Tensor,
                    tok_seq: torch.Tensor, block_table: torch.Tensor, num_kv_heads: int, scale: float,
                    window: Optional[int] = None, out: Optional[torch.Tensor] = None,
                    sink: Optional[torch.Tensor] = None, keep_first: int = 0,
-                   slopes: Optional[torch.Tensor] = None, longest: int = 1) -> torch.Tensor:
-    """Causal attention of q [T, H, hd] over the paged cache; returns [T, H*hd].  `longest`: the most neighbouring rows
-    that belong to one sequence (a step's `max_new`; it chooses a kernel, the result is the same to the bit).  `window` here and in the other kernels' faces:
+                   slopes: Optional[torch.Tensor] = None, longest: int = 1,
+                   seq_start: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Causal attention of q [T, H, hd] over the paged cache; returns [T, H*hd].  `seq_start` int32 [sequences + 1]: where
+    the rows of each of the step's sequences begin (`tok_seq` says the same), and `longest`: the most rows of one sequence.
+    With both, prompts run in tiles that share their keys; the result is the same to the bit.  `window` here and in the other kernels' faces:
     a sliding window of that many keys, or the negative of a chunk size for a mask of chunks (`key_mask`).  `sink` here
     and in the other faces: float32 [H], one more term exp(sink[h]) in the denominator of head h's softmax, with no key
     and no value and outside the scale (None: the plain softmax).  `keep_first` here and in the other faces: beside a sliding
@@ -34,10 +46,15 @@ def attention_rows(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor
         raise KernelError(f"attention: head_dim {hd} exceeds 1024, the largest this kernel takes")
     if out is None:
         out = torch.empty((T, H * hd), dtype=q.dtype, device=q.device)
+    if seq_start is not None and longest < TILE_FROM:
+        seq_start = None
+    if seq_start is not None:
+        _i32(seq_start, "seq_start")
+    n_seqs = seq_start.numel() - 1 if seq_start is not None else 0
     _cache_bounds("attention_simt", (), k_cache, block_table)
     _check(_fn("attention_simt", "plm_attention_rows")(
         _p(q), _p(k_cache), _p(v_cache), _p(out), _dt(q, "q"), _p(tok_pos), _p(tok_seq), _p(block_table),
-        block_table.shape[1], T, H, G, hd, float(scale), int(window or 0), _p(sink), int(keep_first), _p(slopes), int(longest), _stream()),
+        block_table.shape[1], T, H, G, hd, float(scale), int(window or 0), _p(sink), int(keep_first), _p(slopes), _p(seq_start), n_seqs, _stream()),
         f"attention_rows T={T} H={H} hd={hd}")
     return out
 
@@ -287,4 +304,5 @@ def attention(q: torch.Tensor, kv, step, num_kv_heads: int, scale: float, chunk:
         return prefill(q, kv.k, kv.v, step.seq_start, step.seq_kv_len, kv.block_table, step.max_new,
                        num_kv_heads, scale, window=kv.window, **more)
     return attention_rows(q, kv.k, kv.v, step.tok_pos, step.tok_seq, kv.block_table, num_kv_heads, scale,
-                          window=kv.window, longest=step.max_new, **more)
+                          window=kv.window, longest=step.max_new,
+                          seq_start=step.seq_start if shares_keys(step.max_new, step.max_position, q.shape[0] * q.shape[1]) else None, **more)

@@ -62,8 +62,34 @@ def test_attention_tile_form_agrees_to_the_bit(dtype, H, G, hd, extra):
     q = torch.randn(sum(new), H, hd).to(DT[dtype]).to(DEV)
     pos = torch.tensor([p for n, m in zip(lens, new) for p in range(n - m, n)], dtype=torch.int32, device=DEV)
     seq = torch.tensor([b for b, m in enumerate(new) for _ in range(m)], dtype=torch.int32, device=DEV)
+    start = torch.tensor([sum(new[:b]) for b in range(len(new) + 1)], dtype=torch.int32, device=DEV)
     more = dict(sink=torch.randn(H, device=DEV), slopes=torch.rand(H, device=DEV) * 0.1) if extra else {}
-    rows, tiles = (ops.attention_rows(q, kc.to(DEV), vc.to(DEV), pos, seq, table.to(DEV), G, hd ** -0.5, longest=n, **more)
-                   for n in (1, max(new)))
+    rows, tiles = (ops.attention_rows(q, kc.to(DEV), vc.to(DEV), pos, seq, table.to(DEV), G, hd ** -0.5, longest=max(new), seq_start=st, **more)
+                   for st in (None, start))
     assert torch.isfinite(rows).any()
     assert torch.equal(torch.nan_to_num(rows.float(), nan=7.0), torch.nan_to_num(tiles.float(), nan=7.0))
+
+
+@pytest.mark.parametrize("longest,max_position,rows,tiles", [(7, 5000, 1 << 20, False), (8, 30, 8191, False), (8, 31, 256, True), (8, 8, 8192, True)])
+def test_when_rows_share_keys(longest, max_position, rows, tiles):
+    from picolm_b200.ops.attention import shares_keys
+    assert shares_keys(longest, max_position, rows) == tiles
+
+
+@pytest.mark.gpu
+def test_single_tokens_beside_a_prompt_have_tiles_of_their_own():
+    """More sequences than a block has threads, heads in pairs: every sequence's rows against the row form."""
+    from picolm_b200 import ops
+    torch.manual_seed(11)
+    H, G, hd = 4, 2, 16
+    new = [1] * 70 + [33] + [1] * 80 + [9, 0, 2]
+    lens = [n + 40 + 3 * b for b, n in enumerate(new)]
+    ks, vs = [torch.randn(n, G, hd) for n in lens], [torch.randn(n, G, hd) for n in lens]
+    kc, vc, table = _paged(ks, vs, lens, sum((n + 63) // 64 for n in lens) + 8, torch.float32, 6)
+    q = torch.randn(sum(new), H, hd, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    pos = i32([p for n, m in zip(lens, new) for p in range(n - m, n)])
+    seq = i32([b for b, m in enumerate(new) for _ in range(m)])
+    start = i32([sum(new[:b]) for b in range(len(new) + 1)])
+    rows, tiles = (ops.attention_rows(q, kc.to(DEV), vc.to(DEV), pos, seq, table.to(DEV), G, hd ** -0.5, longest=33, seq_start=st) for st in (None, start))
+    assert torch.equal(rows, tiles) and torch.isfinite(rows).all()
