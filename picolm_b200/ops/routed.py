@@ -97,7 +97,11 @@ def moe_align(ids: torch.Tensor, n_experts: int, bm: int, n_skip: int = 0) -> So
     return SortedPairs(sorted_, tile_expert, where, bm, max_tiles, top, T)
 
 
-STREAM_TILES = 2048        # the most tiles of the streaming products
+STREAM_TILES = 512         # the most tiles of the streaming products (1,216 tiles of 1,024 experts of 512 x 256: 193 us either way)
+# The most pairs an expert on average for them: what they save is weights read at less than the memory's rate, and with many
+# tiles an expert the products themselves count.  Gate and up, then down, in a stream and without: 16 experts of 2,048 x 1,344
+# with 64 pairs each 178 and 205 us, with 256 689 and 626; 8 of 512 x 352 with 10 and 32 pairs 12 and 12, 15 and 15, with 512 114 and 50.
+STREAM_PAIRS = 64
 
 
 def _few_rows(a: torch.Tensor, lda: int, w: torch.Tensor, out: torch.Tensor, mode: int, pairs: SortedPairs, N: int, K: int,
@@ -105,7 +109,7 @@ def _few_rows(a: torch.Tensor, lda: int, w: torch.Tensor, out: torch.Tensor, mod
     """The experts' products over sorted pairs on mma.sync or the CUDA cores: bfloat16 tiles of 16 rows stream their weights
     through one CTA an SM (csrc/routed_stream.cu: N a multiple of 32, K of 64); the rest by plm_moe_gemm.  Both give the
     same bits."""
-    if (a.dtype == torch.bfloat16 and pairs.bm == 16 and N % 32 == 0 and K % 64 == 0 and pairs.max_tiles <= STREAM_TILES
+    if (a.dtype == torch.bfloat16 and pairs.bm == 16 and N % 32 == 0 and K % 64 == 0 and pairs.max_tiles <= STREAM_TILES and pairs.n_tokens * pairs.top <= STREAM_PAIRS * w.shape[0]
             and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
         return _fn("routed_stream", "plm_moe_stream")(
             _p(a), lda, pairs.top, _p(w), w.shape[0], _p(out), out.shape[1], mode, _p(pairs.tile_expert), _p(pairs.sorted),

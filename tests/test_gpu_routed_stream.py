@@ -44,6 +44,28 @@ def test_streamed_products_give_the_same_bits(mode, T, E, top, N, K, monkeypatch
         assert torch.allclose(streamed[used].double(), torch.relu(z) ** 2, atol=2e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("mode", ["gate_up", "up", "down"])
+@pytest.mark.parametrize("T,E,busy", [(1300, 40, 1), (700, 24, 3), (16 * 380, 100, 1)])
+def test_experts_with_many_tiles(mode, T, E, busy, monkeypatch):
+    """All tokens but a few at one expert or three: runs of hundreds of tiles between experts of one tile and of none."""
+    from picolm_b200 import ops
+    from picolm_b200.ops import routed
+    torch.manual_seed(T)
+    N, K = 96, 128
+    ids = torch.randint(0, busy, (T, 1), device=DEV, dtype=torch.int32) * 7 + 2
+    ids[::97, 0] = torch.randint(0, E, (len(ids[::97]),), device=DEV, dtype=torch.int32)
+    pairs = ops.moe_align(ids, E, 16)
+    assert pairs.max_tiles <= routed.STREAM_TILES and T <= routed.STREAM_PAIRS * E
+    a = torch.randn(pairs.rows if mode == "down" else T, K, device=DEV).to(torch.bfloat16)
+    w = (torch.randn(E, (2 if mode == "gate_up" else 1) * N, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    product = {"gate_up": ops.moe_gate_up, "up": ops.moe_up, "down": ops.moe_down}[mode]
+    streamed = product(a, w, pairs)
+    ops.check_status(DEV)
+    monkeypatch.setattr(routed, "STREAM_TILES", 0)
+    used = pairs.sorted >= 0
+    assert torch.equal(streamed[used], product(a, w, pairs)[used])
+
+
 @pytest.mark.parametrize("T", [1, 8])
 def test_more_sms_than_pieces(T):
     """Fewer pieces of columns than SMs: every CTA has one or none."""
