@@ -39,6 +39,50 @@ def test_experts_products_against_float64(bm, mode, T, E, top, N, K):
         assert torch.allclose(got[used].double(), want, atol=1e-2, rtol=1.2e-2)
 
 
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+# K in whole and in ragged pairs of 64 (3.5 and 8 of them: the ring of three or four stages comes round), and one that only the
+# form with single stages takes
+@pytest.mark.parametrize("K", [448, 1024, 456])
+def test_every_cta_takes_several_units(epilogue, K):
+    """Both forms on the same rows, from the C entry, which is told by the number of pairs which to take: over 450 units, so that every
+    CTA uses both accumulators again, and an expert with 300 rows among some with 30: two or three chunks of its tokens."""
+    import ctypes
+    from picolm_b200 import ops
+    from picolm_b200.csrc.build import load_library
+    from picolm_b200.ops import _lib
+    product = load_library("routed_tc").plm_moe_tc
+    product.argtypes = _lib._SIGNATURES["plm_moe_tc"]
+    E, F = 12, 5120 + (0 if epilogue == 1 else 40)           # (weight rows that end inside a tile of 128)
+    torch.manual_seed(K + epilogue)
+    rows_of = [300, 0, 1, 16, 17, 64, 65, 129, 33, 30, 30, 30]
+    ids = torch.tensor([e for e, n in enumerate(rows_of) for _ in range(n)], dtype=torch.int32)[torch.randperm(sum(rows_of))]
+    pairs = ops.moe_align(ids[:, None].contiguous().to(DEV), E, 16)
+    x = ops.moe_gather(torch.randn(len(ids), K, device=DEV).to(torch.bfloat16), pairs)
+    w = (torch.randn(E, F, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    used = (pairs.sorted >= 0).nonzero()[:, 0]
+    of = pairs.tile_expert.long().repeat_interleave(16)[used]
+    want = torch.empty(len(used), F // 2 if epilogue == 1 else F, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        z = x[used[of == e]].double() @ w[e].double().T
+        if epilogue == 1:
+            z = z.view(len(z), F // 128, 2, 64)
+            z = (torch.nn.functional.silu(z[:, :, 0]) * z[:, :, 1]).reshape(len(z), F // 2)
+        want[of == e] = torch.relu(z) ** 2 if epilogue == 2 else z
+    outs = []
+    for n_pairs in (1, 1 << 20):                             # 128 tokens and pairs of stages (K a multiple of 64), 256 and single ones
+        out = torch.full((pairs.rows, want.shape[1]), float("nan"), dtype=torch.bfloat16 if epilogue else torch.float32, device=DEV)
+        assert product(x.data_ptr(), w.data_ptr(), out.data_ptr(), 1 if epilogue else 0, epilogue, n_pairs, pairs.tile_expert.data_ptr(),
+                       pairs.max_tiles, 16, E, F, K, out.shape[1], ops.status_word(DEV).data_ptr(),
+                       ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        ops.check_status(DEV)
+        outs.append(out[used])
+        if epilogue == 0:                    # sums of up to K / 16 steps, each rounded at 2^-23 of a partial sum of some 4 at most
+            assert (out[used].double() - want).abs().max() <= K / 16 * 4 * 2.0 ** -23
+        else:                                # branches and results rounded to bf16: three roundings of 2^-9 at most
+            assert torch.allclose(out[used].double(), want, atol=1e-2, rtol=1.2e-2)
+    assert torch.allclose(outs[0].float(), outs[1].float(), atol=1e-4, rtol=2.0 ** -7)
+
+
 @pytest.mark.parametrize("types", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("T,E,K", [(1, 5, 64), (8, 16, 4096), (3, 1, 132), (2050, 33, 260), (1185, 32, 2048)])
 def test_router_tiles_give_the_bits_of_the_general_kernel(types, T, E, K):
