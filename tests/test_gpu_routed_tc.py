@@ -83,6 +83,25 @@ def test_every_cta_takes_several_units(epilogue, K):
     assert torch.allclose(outs[0].float(), outs[1].float(), atol=1e-4, rtol=2.0 ** -7)
 
 
+@pytest.mark.parametrize("E", [31, 33, 64, 1000, 1024])
+def test_many_experts(E):
+    """The table of units by expert: a part of 32 experts, a whole one, many; experts without rows among them."""
+    from picolm_b200 import ops
+    torch.manual_seed(E)
+    T, N, K = 3 * E, 200, 64
+    ids = torch.randint(0, E, (T, 2), device=DEV, dtype=torch.int32)
+    ids[: T // 8] = E - 1
+    pairs = ops.moe_align(ids, E, 16)
+    x = ops.moe_gather(torch.randn(T, K, device=DEV).to(torch.bfloat16), pairs)
+    w = (torch.randn(E, N, K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    got = ops.moe_down_tc(x, w, pairs)
+    ops.check_status(DEV)
+    used = pairs.sorted >= 0
+    e = pairs.tile_expert.long().repeat_interleave(16)[used]
+    want = torch.cat([torch.einsum("rk,rnk->rn", a.double(), w[b].double()) for a, b in zip(x[used].split(512), e.split(512))])
+    assert torch.allclose(got[used].double(), want, atol=1e-5, rtol=1e-5)
+
+
 @pytest.mark.parametrize("types", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.bfloat16, torch.float32)])
 @pytest.mark.parametrize("T,E,K", [(1, 5, 64), (8, 16, 4096), (3, 1, 132), (2050, 33, 260), (1185, 32, 2048)])
 def test_router_tiles_give_the_bits_of_the_general_kernel(types, T, E, K):
