@@ -6,7 +6,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("group", [96, 124, 128, 132, 256, 260, 512, 516, 1020, 1024])
+@pytest.mark.parametrize("group", [96, 124, 128, 132, 256, 260, 388, 512, 516, 528, 532, 600, 640, 704, 768, 800, 896, 900, 916, 1020, 1024])
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("types", [(torch.float32, torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32, torch.float32)])
 @pytest.mark.parametrize("norm", [True, False])
