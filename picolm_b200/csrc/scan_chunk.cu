@@ -42,9 +42,13 @@ struct Args {
     int H, N, P, heads_per_group, head_decay;
     int v_quads;                         // v's rows can be read four values at a time
     int* status;                         // device int that stays 0 unless a bounded wait ran out
+    int b0, c0, stretch;                 // the launch's first sequence and chunk, and how many chunks of each sequence it takes (0: all)
+    // the place in the workspace of a sequence's chunk: a whole step's chunks lie one behind the other, a stretch's by sequence
+    __device__ long slot(int s0, int b, int c) const { return stretch ? (long)(b - b0) * stretch + (c - c0) : (long)(s0 / C + b + c); }
+    __device__ int chunks_end(int n_chunks) const { return stretch ? min(n_chunks, c0 + stretch) : n_chunks; }
 };
 
-// The workspace of one (chunk, head), in floats.  A sequence's chunk c lies in slot seq_start / C + sequence + c.
+// The workspace of one (chunk, head), in floats.
 // NP: the key size rounded up to 32, 64 or 128, PP: the value size rounded up to a multiple of 4; padding is zero.
 template <int NP> struct Layout {
     static constexpr long KE = 0, WT = KE + (long)C * NP, QT = WT + (long)C * NP, MT = QT + (long)C * NP, GE = MT + C * C, U = GE + NP;
@@ -111,11 +115,11 @@ chunk_prep_kernel(const Args a) {
     float* bt = between + PAIRS * NP;    // [C] beta, 0 behind the last token
     pdl_launch_dependents();
     pdl_wait();
-    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x;
+    const int c = a.c0 + blockIdx.x, h = blockIdx.y, b = a.b0 + blockIdx.z, tid = threadIdx.x;
     const int s0 = a.seq_start[b], s1 = a.seq_start[b + 1], t0 = s0 + c * C;
     if (t0 >= s1) return;
     const int nt = min(C, s1 - t0), N = a.N, P = a.P, PP = pad4(P), H = a.H, g = h / a.heads_per_group;
-    float* out = a.ws + ((long)(s0 / C + b + c) * H + h) * Lay::floats(PP);
+    float* out = a.ws + (a.slot(s0, b, c) * H + h) * Lay::floats(PP);
 
     if (!DELTA) {                        // U is v
         const T* v = static_cast<const T*>(a.v) + (long)t0 * a.ldv + (long)h * P;
@@ -420,7 +424,7 @@ __device__ __forceinline__ void outer_step(uint64_t (&acc)[2][WC], const float* 
 }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
-template <int NP>
+template <int NP, bool STRETCH>
 __global__ void __launch_bounds__(WALK_THREADS)
 chunk_walk_kernel(const Args a) {
     constexpr int NG = NP / 4, SPLITS = WALK_THREADS / NG, SS = C / SPLITS, NS = NP / 16, UNITS = 2 * NP;
@@ -431,14 +435,18 @@ chunk_walk_kernel(const Args a) {
     float4* part = reinterpret_cast<float4*>(Us + walk_row(C));
     pdl_launch_dependents();
     const int P = a.P, PP = pad4(P), N = a.N, H = a.H, ptiles = (P + WC - 1) / WC;
-    const int p0 = blockIdx.x % ptiles * WC, h = blockIdx.x / ptiles % H, b = blockIdx.x / ptiles / H;
+    const int p0 = blockIdx.x % ptiles * WC, h = blockIdx.x / ptiles % H, b = (STRETCH ? a.b0 : 0) + blockIdx.x / ptiles / H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_wait();
     const int s0 = a.seq_start[b], s1 = a.seq_start[b + 1];
     if (s1 <= s0) return;
-    const int n_chunks = (s1 - s0 + C - 1) / C;
+    int n_chunks = (s1 - s0 + C - 1) / C;
+    if (STRETCH) {                                     // from c0 on
+        n_chunks = a.chunks_end(n_chunks) - a.c0;
+        if (n_chunks <= 0) return;
+    }
     const long step = (long)H * Lay::floats(PP);
-    float* ws = a.ws + ((long)(s0 / C + b) * H + h) * Lay::floats(PP);
+    float* ws = a.ws + ((STRETCH ? a.slot(s0, b, a.c0) : (long)(s0 / C + b)) * H + h) * Lay::floats(PP);
     __shared__ __align__(8) uint64_t full[2];
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(full);
     if (tid == 0) {
@@ -637,10 +645,10 @@ chunk_outer_kernel(const Args a) {
     pdl_launch_dependents();
     pdl_wait();
     const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, n0 = blockIdx.x / ptiles % MT * 64, c = blockIdx.x / ptiles / MT, h = blockIdx.y, b = blockIdx.z;
+    const int p0 = blockIdx.x % ptiles * PT, n0 = blockIdx.x / ptiles % MT * 64, c = a.c0 + blockIdx.x / ptiles / MT, h = blockIdx.y, b = a.b0 + blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
-    float* w = a.ws + ((long)(s0 / C + b + c) * a.H + h) * Lay::floats(PP);
+    float* w = a.ws + (a.slot(s0, b, c) * a.H + h) * Lay::floats(PP);
     uint64_t acc[4][PT / 16] = {};
     tile_sums<PT>(tile, acc, (nt + TK - 1) / TK, PP - p0, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
         pa = w + Lay::KE + (long)i * TK * NP + n0, lda = NP;
@@ -665,13 +673,13 @@ chunk_chain_kernel(const Args a) {
     constexpr int AHEAD = 8;
     pdl_launch_dependents();
     pdl_wait();
-    const int P = a.P, PP = pad4(P), idx = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, b = blockIdx.z;
+    const int P = a.P, PP = pad4(P), idx = blockIdx.x * 256 + threadIdx.x, h = blockIdx.y, b = a.b0 + blockIdx.z;
     const int n = idx / (PP / 4), p = idx % (PP / 4) * 4;
     const int s0 = a.seq_start[b], len = a.seq_start[b + 1] - s0;
-    if (n >= NP || len <= 0) return;
-    const int n_chunks = (len + C - 1) / C;
+    const int n_chunks = a.chunks_end((len + C - 1) / C) - a.c0;         // from c0 on
+    if (n >= NP || n_chunks <= 0) return;
     const long step = (long)a.H * Lay::floats(PP);
-    float* w = a.ws + ((long)(s0 / C + b) * a.H + h) * Lay::floats(PP);
+    float* w = a.ws + (a.slot(s0, b, a.c0) * a.H + h) * Lay::floats(PP);
     float* at = w + Lay::s(PP) + (long)n * PP + p;
     float* st = a.state + (long)a.seq_slot[b] * a.state_stride + (long)h * a.N * P + (long)n * P + p;
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -714,10 +722,10 @@ chunk_out_kernel(const Args a) {
     pdl_launch_dependents();
     pdl_wait();
     const int P = a.P, PP = pad4(P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, c = blockIdx.x / ptiles, h = blockIdx.y, b = blockIdx.z;
+    const int p0 = blockIdx.x % ptiles * PT, c = a.c0 + blockIdx.x / ptiles, h = blockIdx.y, b = a.b0 + blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
-    const float* w = a.ws + ((long)(s0 / C + b + c) * a.H + h) * Lay::floats(PP);
+    const float* w = a.ws + (a.slot(s0, b, c) * a.H + h) * Lay::floats(PP);
     uint64_t acc[4][PT / 16] = {};
     tile_sums<PT>(tile, acc, NP / TK + (nt + TK - 1) / TK, PP - p0, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
         const int j = i - NP / TK;
@@ -761,21 +769,25 @@ chunk_out_kernel(const Args a) {
         }
 }
 
+template <int NP, bool STRETCH>
+cudaError_t launch_walk(const Args& a, int n_seqs, cudaStream_t stream) {
+    static const cudaError_t ok =
+        cudaFuncSetAttribute(chunk_walk_kernel<NP, STRETCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem<NP>());
+    if (ok != cudaSuccess) return ok;
+    return launch_pdl(chunk_walk_kernel<NP, STRETCH>, dim3((unsigned)((long)n_seqs * a.H * ((a.P + WC - 1) / WC))), dim3(WALK_THREADS),
+                      walk_smem<NP>(), stream, a);
+}
+
 template <int NP, typename T, bool DELTA, int PT>
-int run(const Args& a, int n_seqs, int max_new, cudaStream_t stream) {
+int run_stretch(const Args& a, int n_seqs, unsigned chunks, cudaStream_t stream) {
     static const cudaError_t prep_ok =
         cudaFuncSetAttribute(chunk_prep_kernel<T, NP, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem<NP>());
     if (prep_ok != cudaSuccess) return (int)prep_ok;
-    const unsigned chunks = (unsigned)((max_new + C - 1) / C);
     const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
     cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, a.H, n_seqs), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
     if (e != cudaSuccess) return (int)e;
     if (DELTA) {
-        static const cudaError_t walk_ok =
-            cudaFuncSetAttribute(chunk_walk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem<NP>());
-        if (walk_ok != cudaSuccess) return (int)walk_ok;
-        e = launch_pdl(chunk_walk_kernel<NP>, dim3((unsigned)((long)n_seqs * a.H * ((a.P + WC - 1) / WC))), dim3(WALK_THREADS), walk_smem<NP>(),
-                       stream, a);
+        e = a.stretch ? launch_walk<NP, true>(a, n_seqs, stream) : launch_walk<NP, false>(a, n_seqs, stream);
     } else {
         e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP > 64 ? NP / 64 : 1), a.H, n_seqs), dim3(128), 0, stream, a);
         if (e != cudaSuccess) return (int)e;
@@ -785,10 +797,30 @@ int run(const Args& a, int n_seqs, int max_new, cudaStream_t stream) {
     return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks * ptiles, a.H, n_seqs), dim3(128), 0, stream, a));
 }
 
+// The whole step at once where the workspace holds it.  Else so many chunks of so many sequences at a time as it holds: a state
+// that a stretch leaves is what the next one starts from, as from step to step, so results are the same to the bit.
+template <int NP, typename T, bool DELTA, int PT>
+int run(Args a, int n_tokens, int n_seqs, int max_new, long ws_floats, cudaStream_t stream) {
+    const long chunks = (max_new + C - 1) / C, slots = ws_floats / (a.H * Layout<NP>::floats(pad4(a.P)));
+    if ((long)n_tokens / C + n_seqs <= slots) return run_stretch<NP, T, DELTA, PT>(a, n_seqs, (unsigned)chunks, stream);
+    if (slots < 1) return PLM_ERR_SHAPE;
+    const int group = (int)(n_seqs < slots ? n_seqs : slots);
+    a.stretch = (int)(slots / group < chunks ? slots / group : chunks);
+    for (a.b0 = 0; a.b0 < n_seqs; a.b0 += group)
+        for (a.c0 = 0; a.c0 < chunks; a.c0 += a.stretch) {
+            const int e = run_stretch<NP, T, DELTA, PT>(a, n_seqs - a.b0 < group ? n_seqs - a.b0 : group, (unsigned)a.stretch, stream);
+            if (e != PLM_OK) return e;
+        }
+    return PLM_OK;
+}
+
 template <typename T, bool DELTA>
-int by_size(const Args& a, int n_seqs, int max_new, cudaStream_t stream) {
-    if (a.N <= 64) return a.P <= 64 ? run<64, T, DELTA, 64>(a, n_seqs, max_new, stream) : run<64, T, DELTA, 128>(a, n_seqs, max_new, stream);
-    return a.P <= 64 ? run<128, T, DELTA, 64>(a, n_seqs, max_new, stream) : run<128, T, DELTA, 128>(a, n_seqs, max_new, stream);
+int by_size(const Args& a, int n_tokens, int n_seqs, int max_new, long ws_floats, cudaStream_t stream) {
+    if (a.N <= 64)
+        return a.P <= 64 ? run<64, T, DELTA, 64>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                         : run<64, T, DELTA, 128>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
+    return a.P <= 64 ? run<128, T, DELTA, 64>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                     : run<128, T, DELTA, 128>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }
 
 int check(const Args& a, int n_seqs, int max_new, int dtype) {
@@ -800,35 +832,38 @@ int check(const Args& a, int n_seqs, int max_new, int dtype) {
 
 }  // namespace
 
-// Floats of workspace a (chunk, head) takes; a step of n_tokens tokens in n_seqs sequences needs (n_tokens / 64 + n_seqs + 1) * H of them.
+// Floats of workspace a (chunk, head) takes; a step of n_tokens tokens in n_seqs sequences runs at once in
+// (n_tokens / 64 + n_seqs) * H of them, and in stretches in any number of H.
 extern "C" int plm_scan_chunk_floats(int N, int P) { return (int)(N <= 64 ? Layout<64>::floats(pad4(P)) : Layout<128>::floats(pad4(P))); }
 
 // The gated delta rule: qn, kn float32 [T, H / heads_per_group * N], dec (the decays' logarithms) float32 [T, H * N] or with
 // head_decay [T, H], beta float32 [T, H], v of `dtype`; y float32 [T, H * P].
 extern "C" int plm_delta_channel_scan(const float* qn, const float* kn, const float* dec, const float* beta, const void* v, int dtype,
-                                      long ldv, float* state, long state_stride, float* y, float* ws, const int* seq_start,
-                                      const int* seq_slot, int n_seqs, int max_new, int H, int N, int P, int heads_per_group,
-                                      int head_decay, int* status, cudaStream_t stream) {
+                                      long ldv, float* state, long state_stride, float* y, float* ws, long ws_floats,
+                                      const int* seq_start, const int* seq_slot, int n_tokens, int n_seqs, int max_new, int H, int N, int P,
+                                      int heads_per_group, int head_decay, int* status, cudaStream_t stream) {
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     const long G = heads_per_group > 0 ? H / heads_per_group : 0;
     const Args a = {qn, kn, v, dec, G * N, G * N, ldv, head_decay ? (long)H : (long)H * N, beta, nullptr, 1.f, 1.f, ws, state, state_stride, y,
-                    seq_start, seq_slot, H, N, P, heads_per_group, head_decay, 0, status};
+                    seq_start, seq_slot, H, N, P, heads_per_group, head_decay, 0, status, 0, 0, 0};
     const int e = check(a, n_seqs, max_new, dtype);
     if (e != PLM_OK) return e;
-    return dtype == PLM_F32 ? by_size<float, true>(a, n_seqs, max_new, stream) : by_size<bf16, true>(a, n_seqs, max_new, stream);
+    return dtype == PLM_F32 ? by_size<float, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                            : by_size<bf16, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }
 
 // Linear attention with the decays sigmoid(raw + bias)^power: q, k, v, raw of `dtype`.
 extern "C" int plm_sigmoid_chunk_scan(const void* q, const void* k, const void* v, const void* raw, int dtype, long ldq, long ldk, long ldv,
                                       long ldr, const float* bias, float q_scale, float power, float* state, long state_stride, float* y,
-                                      float* ws, const int* seq_start, const int* seq_slot, int n_seqs, int max_new, int H, int N, int P,
-                                      int heads_per_group, cudaStream_t stream) {
+                                      float* ws, long ws_floats, const int* seq_start, const int* seq_slot, int n_tokens, int n_seqs,
+                                      int max_new, int H, int N, int P, int heads_per_group, cudaStream_t stream) {
     if (!bias) return PLM_ERR_SHAPE;
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     const Args a = {q, k, v, raw, ldq, ldk, ldv, ldr, nullptr, bias, power, q_scale, ws, state, state_stride, y, seq_start, seq_slot,
                     H, N, P, heads_per_group, 0,
-                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, nullptr};
+                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, nullptr, 0, 0, 0};
     const int e = check(a, n_seqs, max_new, dtype);
     if (e != PLM_OK) return e;
-    return dtype == PLM_F32 ? by_size<float, false>(a, n_seqs, max_new, stream) : by_size<bf16, false>(a, n_seqs, max_new, stream);
+    return dtype == PLM_F32 ? by_size<float, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                            : by_size<bf16, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }

@@ -136,12 +136,13 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     route = None
     if mode == DECAY_SIGMOID and skip is None and N <= SCAN_CHUNK_KEYS:
         route = linear_scan_route(step_shape(step), H, N, P)
-    if (route == IN_CHUNKS and step.n_seqs <= SCAN_CHUNK_SEQS and _scan_chunk_floats(T, step.n_seqs, H, N, P) <= SCAN_CHUNK_FLOATS):
-        ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
+    if route == IN_CHUNKS and step.n_seqs <= SCAN_CHUNK_SEQS:
+        floats, stretches = scan_chunk_plan(T, step.n_seqs, int(step.max_new), H, N, P)
+        ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
         _check(_fn("scan_chunk", "plm_sigmoid_chunk_scan")(
             _p(q), _p(k), _p(v), _p(raw), _dt(v, "v"), ldq, ldk, ldv, ldr, _p(p0), float(q_scale), float(power), _p(state), lds, _p(y),
-            _p(ws), _p(step.seq_start), _p(step.seq_slot), step.n_seqs, int(step.max_new), H, N, P, heads_per_group, _stream()),
-            f"sigmoid_chunk_scan T={T} H={H} N={N} P={P}", kernels=4,
+            _p(ws), floats, _p(step.seq_start), _p(step.seq_slot), T, step.n_seqs, int(step.max_new), H, N, P, heads_per_group, _stream()),
+            f"sigmoid_chunk_scan T={T} H={H} N={N} P={P}", kernels=4 * stretches,
             nbytes=T * ((2 * G * N + H * N + H * P) * v.element_size() + H * P * 4) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (2 * N * P + 64 // 2 * (N + P)))
         return y
@@ -218,16 +219,24 @@ def delta_scan_in_chunks(shape: StepShape, heads: int, key_dim: int, value_dim: 
     return chain * longest + token * work * tokens > fixed + work * (chunk * chunks + seq * seqs)
 
 
-SCAN_CHUNK_FLOATS = 1 << 31      # the most workspace that linear attention takes for it (some 4.8 KB a token and head of 128 x 256)
+# The most workspace they take, 512 MB (3.3 KB a token and head of 128 x 128, 4.8 of 128 x 256): what does not fit goes a stretch of
+# chunks at a time.  A captured step's 2,048 tokens in 65 sequences with 16 heads of 128 x 256 still go at once (465 MB).
+SCAN_CHUNK_FLOATS = 1 << 27
 _chunk_floats = {}
 
 
-def _scan_chunk_floats(n_tokens: int, n_seqs: int, heads: int, key_dim: int, value_dim: int) -> int:
-    """Floats of workspace of csrc/scan_chunk.cu for a step: a sequence's chunks start at slot seq_start // 64 + its number."""
-    floats = _chunk_floats.get((key_dim, value_dim))
-    if floats is None:
-        floats = _chunk_floats[key_dim, value_dim] = _fn("scan_chunk", "plm_scan_chunk_floats")(key_dim, value_dim)
-    return (n_tokens // 64 + n_seqs + 1) * heads * floats
+def scan_chunk_plan(n_tokens: int, n_seqs: int, max_new: int, heads: int, key_dim: int, value_dim: int):
+    """(floats of workspace, stretches) of csrc/scan_chunk.cu for a step."""
+    each = _chunk_floats.get((key_dim, value_dim))
+    if each is None:
+        each = _chunk_floats[key_dim, value_dim] = _fn("scan_chunk", "plm_scan_chunk_floats")(key_dim, value_dim)
+    slots = n_tokens // 64 + n_seqs                          # a sequence's chunks start at slot seq_start // 64 + its number
+    if slots * heads * each <= SCAN_CHUNK_FLOATS:
+        return slots * heads * each, 1
+    slots = max(1, SCAN_CHUNK_FLOATS // (heads * each))
+    chunks, group = (max_new + 63) // 64, min(n_seqs, slots)
+    stretch = min(slots // group, chunks)
+    return slots * heads * each, -(-n_seqs // group) * -(-chunks // stretch)
 
 
 _plans = {}
@@ -661,13 +670,14 @@ def delta_scan(qn: torch.Tensor, kn: torch.Tensor, qk: torch.Tensor, decay: torc
             nbytes=T * (8 * G * N + H * P * (4 + v.element_size())) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (3 * N * P + 64 // 2 * (2 * N + N + 2 * P)))
         return y
-    if channel and delta_scan_in_chunks(step_shape(step), H, N, P):
-        ws = torch.empty((_scan_chunk_floats(T, step.n_seqs, H, N, P),), dtype=torch.float32, device=v.device)
+    if channel and step.n_seqs <= SCAN_CHUNK_SEQS and delta_scan_in_chunks(step_shape(step), H, N, P):
+        floats, stretches = scan_chunk_plan(T, step.n_seqs, int(step.max_new), H, N, P)
+        ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
         _check(_fn("scan_chunk", "plm_delta_channel_scan")(
-            _p(qn), _p(kn), _p(decay), _p(beta), _p(v), _dt(v, "v"), ldv, _p(state), lds, _p(y), _p(ws), _p(step.seq_start),
-            _p(step.seq_slot), step.n_seqs, int(step.max_new), H, N, P, heads_per_group, 1 if head_decay else 0,
+            _p(qn), _p(kn), _p(decay), _p(beta), _p(v), _dt(v, "v"), ldv, _p(state), lds, _p(y), _p(ws), floats, _p(step.seq_start),
+            _p(step.seq_slot), T, step.n_seqs, int(step.max_new), H, N, P, heads_per_group, 1 if head_decay else 0,
             _p(status_word(v.device)), _stream()),
-            f"delta_channel_scan T={T} H={H} N={N} P={P}", kernels=3,
+            f"delta_channel_scan T={T} H={H} N={N} P={P}", kernels=3 * stretches,
             nbytes=T * ((2 * G * N + H * ND) * 4 + H * P * (4 + v.element_size())) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (3 * N * P + 64 // 2 * (3 * N + 2 * P)))
         return y

@@ -146,3 +146,56 @@ def test_what_is_not_finite_reaches_no_earlier_token(H, G, N, P, where, what, ru
         others = torch.arange(H * P, device=DEV) != column
         assert torch.equal(y[:, others], clean[:, others])
         assert not torch.isfinite(y[sorted(poisoned), column]).any()
+
+
+@pytest.mark.parametrize("H,G,N,P", [(2, 1, 128, 128), (3, 3, 48, 72)])
+@pytest.mark.parametrize("rule", ["channel", "linear"])
+@pytest.mark.parametrize("slots", [1, 3, 8])
+def test_a_workspace_that_does_not_hold_the_step(H, G, N, P, rule, slots, monkeypatch):
+    """Room for one chunk, three and eight: the step goes some chunks of some sequences at a time, to the same bits."""
+    from picolm_b200 import ops
+    from picolm_b200.ops import recurrent
+    lens = [200, 1, 96, 330, 64]
+    T, step = sum(lens), _step(lens)
+    torch.manual_seed(N + P)
+    q, k, v = torch.randn(T, G * N, device=DEV), torch.randn(T, G * N, device=DEV) * N ** -0.5, torch.randn(T, H * P, device=DEV)
+    decay, beta, bias = torch.randn(T, H * N, device=DEV), torch.rand(T, H, device=DEV), torch.rand(H * N, device=DEV)
+    state0 = torch.randn(len(lens), H * N * P, device=DEV)
+
+    def run():
+        state = state0.clone()
+        if rule == "linear":
+            return ops.linear_scan(q, k, v, decay, ops.DECAY_SIGMOID, bias, None, None, 1.0, 1 / 16, state, step, H, N, P, heads_per_group=H // G), state
+        return ops.delta_scan(q, k, torch.ones(T, G, device=DEV), -decay.abs(), beta, v, state, step, H, N, P, heads_per_group=H // G), state
+    whole = run()
+    ops.check_status(DEV)
+    each = recurrent._chunk_floats[N, P] * H
+    monkeypatch.setattr(recurrent, "SCAN_CHUNK_FLOATS", slots * each)
+    floats, stretches = recurrent.scan_chunk_plan(T, len(lens), max(lens), H, N, P)
+    assert floats == slots * each and stretches == {1: 30, 3: 12, 8: 6}[slots]
+    before = ops.launch_count()
+    parts = run()
+    ops.check_status(DEV)
+    assert ops.launch_count() - before == (4 if rule == "linear" else 3) * stretches
+    assert torch.equal(parts[0], whole[0]) and torch.equal(parts[1], whole[1])
+
+
+@pytest.mark.parametrize("rule", ["channel", "linear"])
+def test_long_prompts_take_a_bounded_workspace(rule):
+    """One prompt of 40,000 tokens, 8 heads of 128 x 128: 1.1 GB for all its chunks."""
+    from picolm_b200 import ops
+    T, H, N, P = 40000, 8, 128, 128
+    step = _step([T])
+    q, k, v = [torch.randn(T, H * N, device=DEV) * N ** -0.5 for _ in range(3)]
+    decay, beta, state = -torch.rand(T, H * N, device=DEV), torch.rand(T, H, device=DEV), torch.zeros(1, H * N * P, device=DEV)
+    bias, qk = torch.rand(H * N, device=DEV), torch.ones(T, H, device=DEV)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    if rule == "linear":
+        y = ops.linear_scan(q, k, v, decay, ops.DECAY_SIGMOID, bias, None, None, 1.0, 1 / 16, state, step, H, N, P)
+    else:
+        y = ops.delta_scan(q, k, qk, decay, beta, v, state, step, H, N, P)
+    ops.check_status(DEV)
+    assert torch.isfinite(y).all()
+    assert torch.cuda.max_memory_allocated() - held <= y.numel() * 4 + (520 << 20)
