@@ -104,10 +104,13 @@ TC_PAIRS = 16
 # And from which the tokens take the MMA's 128 rows instead of the weights: their tiles are nearly full by then, and a tile of
 # 128 x 256 loads less for its work than 128 weight rows with half of 300 tokens.  192, 256 and 281 pairs an expert: 222, 481
 # and 352 us with the weights on the rows, 246, 459 and 340 with the tokens there (32 experts of 2,048 x 2,048; 16 of 4,096 x 5,376).
-# So too where an expert's pairs fill one of those tiles (more than 104 to 128 on average): 16 experts of 4,096 x 5,376 with 121
-# pairs each take 364 us for the layer that way and 373 with the weights on the rows.
+# So too where an expert's pairs fill one of those tiles and seldom spill into a second one (more than 104 to 116 on average; with the
+# weights on the rows 128 tokens at once no longer do, and 256 take longer).  106, 112, 118 and 126 pairs an expert, tokens on
+# the rows against weights there: 32 gated experts of 2,048 x 2,048 183, 184, 204, 202 against 192, 193, 195, 198; 16 ungated
+# of 4,096 x 5,376 275, 277, 296, 317 against 303, 305, 308, 312; 16 gated of 4,096 x 3,584 285, 288, 301, 318 against 313, 317, 318, 321;
+# 32 ungated of 2,048 x 3,072 184, 184, 187, 208 against 204, 206, 208, 210; 64 gated of 2,048 x 1,024 213, 213, 214, 232 against 211, 213, 216, 219.
 WIDE_PAIRS = 224
-FULL_TILE_PAIRS = (104, 128)
+FULL_TILE_PAIRS = (104, 116)
 # More experts than the kernel with the weights on the rows takes (ops.TC_EXPERTS): tiles of 128 of the tokens' rows, half full or
 # better, since a tile of 128 costs the same with one row as with 128.
 MANY_EXPERTS_PAIRS = 64

@@ -5,7 +5,7 @@ from picolm_b200 import ops
 from picolm_b200.parts.feed_forward import tc_tile_rows
 
 
-@pytest.mark.parametrize("pairs,rows", [(15, 0), (16, 16), (104, 16), (105, 128), (128, 128), (129, 16), (223, 16), (224, 128)])
+@pytest.mark.parametrize("pairs,rows", [(15, 0), (16, 16), (104, 16), (105, 128), (116, 128), (117, 16), (128, 16), (223, 16), (224, 128)])
 def test_tiles_by_pairs_an_expert(pairs, rows):
     for experts in (1, 8, ops.TC_EXPERTS):
         assert tc_tile_rows(pairs * experts, experts) == rows
