@@ -289,9 +289,8 @@ extern "C" int plm_attention_rows(const void* q, const void* kc, const void* vc,
         !(((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15)) {
 #define TILE_LAUNCH(T_, MAXHD_)                                                                                             \
     do {                                                                                                                    \
-        static const cudaError_t configured =                                                                               \
-            cudaFuncSetAttribute(attention_tile_kernel<T_, MAXHD_>, cudaFuncAttributeMaxDynamicSharedMemorySize,             \
-                                 (int)tile_smem(MAXHD_, MAXHD_));                                                           \
+        static std::atomic<unsigned long long> devices{0};                                                                  \
+        const cudaError_t configured = plm_allow_smem(attention_tile_kernel<T_, MAXHD_>, tile_smem(MAXHD_, MAXHD_), devices); \
         if (configured != cudaSuccess) return (int)configured;                                                              \
         const long pairs = (long)n_tokens * (H / G);                                                                        \
         attention_tile_kernel<T_, MAXHD_><<<dim3((unsigned)((pairs + TILE_ROWS - 1) / TILE_ROWS + n_seqs), G), WARPS * 32,            \

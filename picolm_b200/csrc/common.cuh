@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <atomic>
 
 // Tokens per cache page.  The cache, the step metadata and every kernel that
 // walks a block table agree on this one number.
@@ -206,6 +207,20 @@ extern "C" int plm_check_bounds(int n_pages, int n_seqs, int n_positions, int n_
 #endif
 
 static inline int plm_status_of(cudaError_t e) { return e == cudaSuccess ? PLM_OK : (int)e; }
+
+// Lets a kernel ask for `bytes` of dynamic shared memory on the device at hand.  `devices` is the kernel's own: the devices where
+// that is done (a bit each), since what one device allows says nothing of another.
+template <typename Kernel>
+static inline cudaError_t plm_allow_smem(Kernel kernel, size_t bytes, std::atomic<unsigned long long>& devices) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = device < 64 ? 1ull << device : 0;
+    if (bit & devices.load(std::memory_order_relaxed)) return cudaSuccess;
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) devices.fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
 
 static inline int plm_launch_status() {
     cudaError_t e = cudaGetLastError();

@@ -306,8 +306,8 @@ int launch_f32(const void* A, const void* W, void* C, int M, int N, int K, long 
 }
 template <int FM, int FN>
 int launch_f32_few(const void* A, const void* W, void* C, int M, int N, int K, long lda, long ldw, long ldc, cudaStream_t stream) {
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(gemm_f32_few_kernel<FM, FN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem<FM, FN>());
+    static std::atomic<unsigned long long> devices{0};
+    const cudaError_t configured = plm_allow_smem(gemm_f32_few_kernel<FM, FN>, few_smem<FM, FN>(), devices);
     if (configured != cudaSuccess) return (int)configured;
     gemm_f32_few_kernel<FM, FN><<<dim3((N + FN - 1) / FN, (M + FM - 1) / FM), 256, few_smem<FM, FN>(), stream>>>(
         (const float*)A, (const float*)W, (float*)C, M, N, K, lda, ldw, ldc);

@@ -225,8 +225,8 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_1, const __grid_consta
 template <int MODE>
 int launch(const CUtensorMap& map_1, const CUtensorMap& map_2, const void* a, long lda, int top, void* out, long ldo, const int* tile_expert,
            const int* sorted, int max_tiles, int N, int K, int interleaved, int* status, cudaStream_t stream) {
-    static const cudaError_t configured =
-        cudaFuncSetAttribute(moe_stream_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ring<MODE>::SMEM);
+    static std::atomic<unsigned long long> devices{0};
+    const cudaError_t configured = plm_allow_smem(moe_stream_kernel<MODE>, Ring<MODE>::SMEM, devices);
     if (configured != cudaSuccess) return (int)configured;
     const long most = (long)max_tiles * (N / GN);
     return plm_status_of(launch_pdl(moe_stream_kernel<MODE>, dim3((unsigned)(most < PLM_SM_COUNT ? most : PLM_SM_COUNT)), dim3(THREADS),

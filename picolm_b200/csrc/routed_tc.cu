@@ -252,7 +252,8 @@ template <int EPI, typename OutT, int NMAX, int SLABS>
 int launch_form(const void* x, const void* w, void* out, long ldo, const int* tile_expert, int max_tiles, int bm, int E, int F, int K, int* status,
                 cudaStream_t stream) {
     auto kernel = moe_tc_kernel<EPI, OutT, NMAX, SLABS>;
-    static const cudaError_t configured = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+    static std::atomic<unsigned long long> devices{0};
+    const cudaError_t configured = plm_allow_smem(kernel, SMEM, devices);
     if (configured != cudaSuccess) return (int)configured;
     CUtensorMap m[5];
     int rc = make_map(&m[0], w, (long)E * F, K, K, FT, SLABS);

@@ -771,8 +771,8 @@ chunk_out_kernel(const Args a) {
 
 template <int NP, bool STRETCH>
 cudaError_t launch_walk(const Args& a, int n_seqs, cudaStream_t stream) {
-    static const cudaError_t ok =
-        cudaFuncSetAttribute(chunk_walk_kernel<NP, STRETCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)walk_smem<NP>());
+    static std::atomic<unsigned long long> devices{0};
+    const cudaError_t ok = plm_allow_smem(chunk_walk_kernel<NP, STRETCH>, walk_smem<NP>(), devices);
     if (ok != cudaSuccess) return ok;
     return launch_pdl(chunk_walk_kernel<NP, STRETCH>, dim3((unsigned)((long)n_seqs * a.H * ((a.P + WC - 1) / WC))), dim3(WALK_THREADS),
                       walk_smem<NP>(), stream, a);
@@ -780,8 +780,8 @@ cudaError_t launch_walk(const Args& a, int n_seqs, cudaStream_t stream) {
 
 template <int NP, typename T, bool DELTA, int PT>
 int run_stretch(const Args& a, int n_seqs, unsigned chunks, cudaStream_t stream) {
-    static const cudaError_t prep_ok =
-        cudaFuncSetAttribute(chunk_prep_kernel<T, NP, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem<NP>());
+    static std::atomic<unsigned long long> devices{0};
+    const cudaError_t prep_ok = plm_allow_smem(chunk_prep_kernel<T, NP, DELTA>, prep_smem<NP>(), devices);
     if (prep_ok != cudaSuccess) return (int)prep_ok;
     const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
     cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, a.H, n_seqs), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
