@@ -1472,10 +1472,10 @@ extern "C" int plm_delta_scan(const float* qn, const float* kn, const float* qk,
 __host__ __device__ static inline long delta_ws_floats(int NP) { return 3L * DELTA_CHUNK * NP + 2L * DELTA_CHUNK * DELTA_CHUNK + NP; }
 
 // The width of a row of keys in the workspace: eight times the NR values a thread of the second kernel holds.
-static inline int delta_chunk_np(int) { return 256; }
+constexpr int DELTA_NR = 32, DELTA_NP = 8 * DELTA_NR;
 
 // grid (chunk of the sequence, sequence, head).  ws per (slot, head): Kp [C][NP] | Qp [C][NP] | Ke [C][NP] | A^T [C][C] | M^T [C][C]
-// | e^{L_C} [NP], NP = delta_chunk_np(N), the padding zero.  A sequence's chunk c lives in slot seq_start / C + sequence + c.
+// | e^{L_C} [NP], NP = DELTA_NP, the padding zero.  A sequence's chunk c lives in slot seq_start / C + sequence + c.
 // HEAD: one decay a head (lgd [T, H]): L is a number per token, so A and M are plain dot products times one exponential.
 template <bool HEAD>
 __global__ void __launch_bounds__(256)
@@ -1556,22 +1556,20 @@ delta_chunk_prep_kernel(const float* qn, const float* kn, const float* lgd,
 }
 
 // grid: (sequence, head, DELTA_CCOLS columns of the state).  A warp holds 4 columns; the N rows of a column are dealt to 8
-// lanes in contiguous eighths, NR values of the state a thread.  A chunk's matrices come through cp.async into one of
-// STAGES buffers, the next chunk's while this one is worked on.
+// lanes in contiguous eighths, NR values of the state a thread.  A chunk's matrices come through cp.async.
 #define DELTA_CCOLS 16
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-template <int NR, int STAGES>
 __global__ void __launch_bounds__(128)
 delta_chunk_scan_kernel(const float* ws, const float* beta, const void* v, int v_f32, long ldv,
                         float* __restrict__ state, long state_stride, float* __restrict__ y, const int* seq_start,
                         const int* seq_slot, int H, int N, int P) {
-    constexpr int C = DELTA_CHUNK, NP = NR * 8, SEG = NR + 4, RS = 8 * SEG;      // SEG: an eighth's floats in a row, padded
+    constexpr int C = DELTA_CHUNK, NR = DELTA_NR, NP = DELTA_NP, SEG = NR + 4, RS = 8 * SEG;      // SEG: an eighth's floats in a row, padded
     constexpr int STAGE = 3 * C * RS + 2 * C * C + RS;                            // Kp | Qp | Ke [C][RS], A | M [C][C], e^{L_C} [RS]
     extern __shared__ __align__(16) float smem[];
-    float* vs = smem + STAGES * STAGE;   // [C][DELTA_CCOLS]
+    float* vs = smem + STAGE;            // [C][DELTA_CCOLS]
     float* bs = vs + C * DELTA_CCOLS;    // [C]
     pdl_launch_dependents();
     const int ptiles = (P + DELTA_CCOLS - 1) / DELTA_CCOLS;
@@ -1595,9 +1593,9 @@ delta_chunk_scan_kernel(const float* ws, const float* beta, const void* v, int v
     const long wsf = 3L * C * NP + 2L * C * C + NP;
     const float* src0 = ws + (((long)(s0 / C) + b) * H + h) * wsf;
     const int n_chunks = (s1 - s0 + C - 1) / C;
-    auto fetch = [&](int chunk, int stage) {
+    auto fetch = [&](int chunk) {
         const float* src = src0 + (long)chunk * H * wsf;
-        float* dst = smem + stage * STAGE;
+        float* dst = smem;
         constexpr int ROW4 = NP / 4, MAT4 = C * ROW4;
         for (int idx = threadIdx.x; idx < 3 * MAT4; idx += 128) {
             const int m = idx / MAT4, rem = idx - m * MAT4;
@@ -1612,21 +1610,10 @@ delta_chunk_scan_kernel(const float* ws, const float* beta, const void* v, int v
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (STAGES == 2) fetch(0, 0);
     for (int chunk = 0; chunk < n_chunks; ++chunk) {
         const int base = s0 + chunk * C, nt = min(C, s1 - base);
-        const int stage = STAGES == 2 ? (chunk & 1) : 0;
-        if (STAGES == 2) {
-            if (chunk + 1 < n_chunks) {
-                fetch(chunk + 1, stage ^ 1);
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 0;" ::: "memory");
-            }
-        } else {
-            fetch(chunk, 0);
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        fetch(chunk);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         for (int idx = threadIdx.x; idx < C * DELTA_CCOLS; idx += 128) {
             const int tt = idx / DELTA_CCOLS, cc = idx - tt * DELTA_CCOLS;
             const int pp = ptile * DELTA_CCOLS + cc;
@@ -1635,7 +1622,7 @@ delta_chunk_scan_kernel(const float* ws, const float* beta, const void* v, int v
         }
         if (threadIdx.x < C) bs[threadIdx.x] = threadIdx.x < nt ? beta[(long)(base + threadIdx.x) * H + h] : 0.f;
         __syncthreads();
-        const float* Kp = smem + stage * STAGE;
+        const float* Kp = smem;
         const float* Qp = Kp + C * RS;
         const float* Ke = Qp + C * RS;
         const float* A = Ke + C * RS;
@@ -1717,20 +1704,7 @@ delta_chunk_scan_kernel(const float* ws, const float* beta, const void* v, int v
     }
 }
 
-template <int NR, int STAGES>
-static int delta_chunk_launch(const float* ws, const float* beta, const void* v, int v_f32, long ldv, float* state, long state_stride,
-                              float* y, const int* seq_start, const int* seq_slot, int n_seqs, int H, int N, int P,
-                              cudaStream_t stream) {
-    constexpr int C = DELTA_CHUNK, RS = 8 * (NR + 4);
-    const size_t smem = ((size_t)STAGES * (3 * C * RS + 2 * C * C + RS) + C * DELTA_CCOLS + C) * sizeof(float);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(delta_chunk_scan_kernel<NR, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const unsigned grid = (unsigned)((long)n_seqs * H * ((P + DELTA_CCOLS - 1) / DELTA_CCOLS));
-    return plm_status_of(launch_pdl(delta_chunk_scan_kernel<NR, STAGES>, dim3(grid), dim3(128), smem, stream, ws, beta, v, v_f32,
-                                    ldv, state, state_stride, y, seq_start, seq_slot, H, N, P));
-}
-
-// ws: ((n_tokens / DELTA_CHUNK) + n_seqs + 1) * H * delta_ws_floats(delta_chunk_np(N)) floats.
+// ws: ((n_tokens / DELTA_CHUNK) + n_seqs + 1) * H * delta_ws_floats(DELTA_NP) floats.
 extern "C" int plm_delta_chunk_scan(const float* qn, const float* kn, const float* dec, const float* beta, const void* v,
                                     int dtype, long ldv, float* state, long state_stride, float* y, float* ws,
                                     const int* seq_start, const int* seq_slot, int n_seqs, int max_new, int H, int N, int P,
@@ -1739,16 +1713,16 @@ extern "C" int plm_delta_chunk_scan(const float* qn, const float* kn, const floa
     if (H <= 0 || N <= 0 || P <= 0 || heads_per_group <= 0 || H % heads_per_group) return PLM_ERR_SHAPE;
     if (N <= 128 || N > 256) return PLM_ERR_UNSUPPORTED;
     if (dtype != PLM_F32 && dtype != PLM_BF16) return PLM_ERR_DTYPE;
-    const int NP = delta_chunk_np(N);
     const size_t prep_smem = (size_t)DELTA_CHUNK * (head_decay ? 2 * N + 1 : 3 * N) * sizeof(float);
     auto prep = head_decay ? delta_chunk_prep_kernel<true> : delta_chunk_prep_kernel<false>;
     if (prep_smem > 48 * 1024) cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem);
     const dim3 pgrid((unsigned)((max_new + DELTA_CHUNK - 1) / DELTA_CHUNK), (unsigned)n_seqs, (unsigned)H);
-    int e = plm_status_of(launch_pdl(prep, pgrid, dim3(256), prep_smem, stream, qn, kn, dec, ws, seq_start, H, N, NP, heads_per_group));
+    int e = plm_status_of(launch_pdl(prep, pgrid, dim3(256), prep_smem, stream, qn, kn, dec, ws, seq_start, H, N, DELTA_NP, heads_per_group));
     if (e != PLM_OK) return e;
-#define DCS(NR_, ST_)                                                                                                     \
-    return delta_chunk_launch<NR_, ST_>(ws, beta, v, dtype == PLM_F32 ? 1 : 0, ldv, state, state_stride, y, seq_start, seq_slot, \
-                                        n_seqs, H, N, P, stream)
-    DCS(32, 1);
-#undef DCS
+    constexpr int C = DELTA_CHUNK, RS = 8 * (DELTA_NR + 4);
+    const size_t smem = ((size_t)(3 * C * RS + 2 * C * C + RS) + C * DELTA_CCOLS + C) * sizeof(float);
+    cudaFuncSetAttribute(delta_chunk_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const unsigned grid = (unsigned)((long)n_seqs * H * ((P + DELTA_CCOLS - 1) / DELTA_CCOLS));
+    return plm_status_of(launch_pdl(delta_chunk_scan_kernel, dim3(grid), dim3(128), smem, stream, ws, beta, v, dtype == PLM_F32 ? 1 : 0, ldv,
+                                    state, state_stride, y, seq_start, seq_slot, H, N, P));
 }

@@ -49,7 +49,7 @@ struct Args {
 };
 
 // The workspace of one (chunk, head), in floats.
-// NP: the key size rounded up to 32, 64 or 128, PP: the value size rounded up to a multiple of 4; padding is zero.
+// NP: the key size rounded up to 64 or 128, PP: the value size rounded up to a multiple of 4; padding is zero.
 template <int NP> struct Layout {
     static constexpr long KE = 0, WT = KE + (long)C * NP, QT = WT + (long)C * NP, MT = QT + (long)C * NP, GE = MT + C * C, U = GE + NP;
     __host__ __device__ static long s(int PP) { return U + (long)C * PP; }           // the state that the chunk starts from
@@ -640,7 +640,7 @@ template <int NP, int PT>
 __global__ void __launch_bounds__(128)
 chunk_outer_kernel(const Args a) {
     using Lay = Layout<NP>;
-    constexpr int MT = NP / 64 > 0 ? NP / 64 : 1;
+    constexpr int MT = NP / 64;
     __shared__ __align__(16) Tile<PT> tile;
     pdl_launch_dependents();
     pdl_wait();
@@ -660,7 +660,7 @@ chunk_outer_kernel(const Args a) {
 #pragma unroll
         for (int x = 0; x < PT / 64; ++x) {
             const int n = n0 + r / 4 * 32 + ty * 4 + r % 4, p = p0 + x * 64 + tx * 4;
-            if (n < NP && p < PP)                        // (padding stays zero, whatever U holds)
+            if (p < PP)                                  // (padding stays zero, whatever U holds)
                 *reinterpret_cast<float4*>(w + Lay::s(PP) + (long)n * PP + p) = n < a.N ? four(acc, r, x) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 }
@@ -789,7 +789,7 @@ int run_stretch(const Args& a, int n_seqs, unsigned chunks, cudaStream_t stream)
     if (DELTA) {
         e = a.stretch ? launch_walk<NP, true>(a, n_seqs, stream) : launch_walk<NP, false>(a, n_seqs, stream);
     } else {
-        e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP > 64 ? NP / 64 : 1), a.H, n_seqs), dim3(128), 0, stream, a);
+        e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP / 64), a.H, n_seqs), dim3(128), 0, stream, a);
         if (e != cudaSuccess) return (int)e;
         e = launch_pdl(chunk_chain_kernel<NP>, dim3((NP * (PP / 4) + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a);
     }
