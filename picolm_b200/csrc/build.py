@@ -33,6 +33,7 @@ NVCC_FLAGS = [
 LIBRARIES: Dict[str, List[str]] = {
     "elementwise": ["elementwise.cu"],
     "gemm_simt": ["gemm_simt.cu"],
+    "gemm_f32_tc": ["gemm_f32_tc.cu"],
     "gemm_tc": ["gemm_tc.cu"],
     "gemm_tc_skinny": ["gemm_tc_skinny.cu"],
     "gemm_tc_wide": ["gemm_tc_wide.cu"],

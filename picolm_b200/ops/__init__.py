@@ -13,7 +13,7 @@ from .elementwise import (GATE_ACTIVATIONS, add_bias, add_rows, dyt_norm, embed,
                           post_pre_norm, post_pre_norm_supported, qk_norm_rope_store, rmsnorm, rope_store, scaled_sum,
                           swiglu, token_gate, rope_rows, norm_pair_shift, embed_pair, gelu_erf, joined_post_pre_norm,
                           joined_post_pre_norm_supported, embed_norm, squash, plain_act)
-from .gemm import (PLAIN_ACTIVATIONS, PendingLinear, ScaledRows, gemm_simt, gemm_tc_skinny, gemm_tc_supported,  # noqa: F401
+from .gemm import (PLAIN_ACTIVATIONS, PendingLinear, ScaledRows, gemm_f32_tc, gemm_simt, gemm_tc_skinny, gemm_tc_supported,  # noqa: F401
                    gemm_tc_wide, interleave_gate_up, linear, linear_act, linear_residual_norm, linear_swiglu, pair_pays,
                    residual_norm_supported)
 from .recurrent import (IN_CHUNKS, ONE_PASS, SCAN_CHUNK_KEYS, StepShape, delta_scan_in_chunks, linear_scan_route, step_shape,  # noqa: F401

@@ -71,6 +71,8 @@ _SIGNATURES = {
     "plm_gemm_tc_wide_grouped": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _l, _l, _i, _vp, _vp, _vp],
     "plm_gemm_tc_pair": [_vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _l, _l, _vp, _vp],
     "plm_gemm_simt": [_vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _l, _l, _l, _vp],
+    "plm_gemm_f32_tc": [_vp, _vp, _vp, _i, _i, _i, _l, _l, _l, _i, _vp, _vp],
+    "plm_gemm_f32_tc_form": [_i, _i, _i],
     "plm_attention_rows": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _i, _vp, _vp, _i, _vp],
     "plm_attn_prefill": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _i, _vp, _i, _vp, _vp],
     "plm_attn_tc_prefill": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp, _vp],
@@ -357,7 +359,8 @@ _OUT_OF_BOUNDS = {16: "page number", 17: "sequence index", 18: "position", 19: "
 _WAITS = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting", 5: "a decode step's pages", 40: "the walk over chunks",
           41: "the experts' streamed weights", 42: "the experts' streamed products", 43: "the experts' streamed rows",
           51: "the experts' TMA producer", 52: "the experts' MMA issuer, results unread", 53: "the experts' MMA issuer",
-          54: "the experts' epilogue"}
+          54: "the experts' epilogue", 60: "the float32 product's TMA producer", 61: "the float32 product's MMA issuer",
+          62: "the float32 product's split", 63: "the float32 product's sums"}
 
 
 def check_status(device="cuda:0") -> None:

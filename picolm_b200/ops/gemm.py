@@ -38,6 +38,32 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype,
     return out
 
 
+def gemm_f32_tc_supported(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> bool:
+    """Whether the float32 product runs on the tensor cores: all three float32, rows on 16-byte boundaries.  Nothing here
+    looks at the number of rows: a row's result must not depend on how many stand beside it, and the CUDA-core product's
+    sums round otherwise."""
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or out_dtype != torch.float32 or a.dim() != 2 or w.dim() != 2:
+        return False
+    K = a.shape[1]
+    return (K == w.shape[1] and K > 0 and K % 4 == 0 and a.is_cuda and a.stride(1) == 1 and a.stride(0) >= K and a.stride(0) % 4 == 0
+            and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, form: int = 0) -> torch.Tensor:
+    """out[M, N] = a[M, K] @ w[N, K]^T, all float32, on the tensor cores with every float in three bfloat16 terms and the error
+    of float32 sums (csrc/gemm_f32_tc.cu).  `form`: rows of `a` a tile + 1000 * CTAs a tile, 0 for the one that fits; every
+    form gives the same bits."""
+    _dev(w, "w")
+    if not gemm_f32_tc_supported(a, w, torch.float32):
+        raise KernelError(f"gemm_f32_tc: needs float32 rows on 16-byte boundaries, got {a.dtype} {list(a.shape)} and {w.dtype} {list(w.shape)}")
+    (M, K), N = a.shape, w.shape[0]
+    out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    _check(_fn("gemm_f32_tc", "plm_gemm_f32_tc")(
+        _p(a), _p(w), _p(out), M, N, K, a.stride(0), K, N, form, _p(status_word(a.device)), _stream()),
+        f"gemm_f32_tc {M}x{N}x{K}", **_work(a, w, out))
+    return out
+
+
 def gemm_tc_supported(a: torch.Tensor, w: torch.Tensor) -> bool:
     """Whether the tensor-core kernel takes a @ w^T: both bfloat16, K a multiple of
     8 (rows start on 16-byte boundaries, as TMA needs) and at least one K block."""
@@ -404,7 +430,7 @@ def linear(a, w: torch.Tensor, out_dtype: torch.dtype, defer: bool = False):
     """a [M, K] times w [N, K]^T -> [M, N].  The kernel is chosen by element
     types and shape, never by the model: the tensor cores for bfloat16 operands
     that TMA can address (the cluster kernel for up to 64 rows, the wide kernel
-    beyond), the CUDA cores for everything else.
+    beyond) and for float32 ones with rows on 16-byte boundaries, the CUDA cores for everything else.
 
     `a` may be `ScaledRows`.  With `defer` (a float32 delta for the residual stream) the product may
     come back as a `PendingLinear` for the next norm to run; whoever cannot use that calls `compute()`."""
@@ -427,4 +453,6 @@ def linear(a, w: torch.Tensor, out_dtype: torch.dtype, defer: bool = False):
         if a.shape[0] <= 64:
             return gemm_tc_skinny(a, w, out_dtype)
         return gemm_tc_wide(a, w, out_dtype, pair=pair_pays(a.shape[0], w.shape[0], a.shape[1], 0))
+    if gemm_f32_tc_supported(a, w, out_dtype):
+        return gemm_f32_tc(a, w)
     return gemm_simt(a, w, out_dtype)
