@@ -278,7 +278,7 @@ attn_tc_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc_s = instr_desc(BKV, false), idesc_o = instr_desc(HD, true);
             auto qk = [&](int i) {                                       // S[i % NSB] = Q K(i)^T
                 const uint32_t k_smem = k_smem0 + (i % KS) * K_BYTES;

@@ -153,7 +153,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         }
     } else if (warp == 1) {
         cluster_wait();
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = instr_desc_bf16(BN);
             for (int i = 0; i < n_kb; ++i) {
                 const int s = i % STAGES;
@@ -484,7 +484,7 @@ gemm_tc_skinny_walk_kernel(const __grid_constant__ CUtensorMap map_w, const __gr
                     mbar_wait(full0 + 8 * (g % STAGES), (g / STAGES) & 1, nullptr, 0);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t idesc = instr_desc_bf16(BN);
             bool ok = true;
             int g = 0;

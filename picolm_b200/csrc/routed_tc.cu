@@ -154,7 +154,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMAs
-        if (lane == 0) {
+        if (elect_one()) {
             int i = 0, done = 0, handed = 0;           // stages consumed, units begun, units handed to the warps that read them
             bool ok = true;
             for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++done) {
