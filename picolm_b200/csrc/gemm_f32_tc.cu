@@ -22,9 +22,10 @@
 // Bound by the MMAs (106 cycles each at 96 columns, 79 at 64, 58 at 16) and the hand-overs between the warps.  Everything done by
 // the same eight warps, with W's terms in shared memory too: 490 us for 462 x 2,048 x 8,192; splitting and adding apart 275;
 // W's terms in tensor memory 237; two issuing warps behind elect.sync 190; four splitting warps a stage in turns 171.
-#include "tc_common.cuh"
+#include "split_common.cuh"
 
 using namespace plm_tc;
+using namespace plm_split;
 
 namespace {
 
@@ -53,54 +54,6 @@ template <int NB> struct Tile {                                // NB rows of A a
 // Descriptor of a K-major bf16 tile with rows of 64 bytes and the 64-byte swizzle: eight rows are 512 bytes, layout type 4.
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
-}
-
-template <int NC> __device__ __forceinline__ void tmem_load(uint32_t addr, uint32_t (&r)[NC]) {
-    static_assert(NC == 8 || NC == 16 || NC == 32, "columns");
-    if constexpr (NC == 32) tc_ld32(addr, r);
-    if constexpr (NC == 16)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                     "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]) : "r"(addr) : "memory");
-    if constexpr (NC == 8)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 "
-                     "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr) : "memory");
-}
-// (the registers count as written by the wait, so that nothing made of them moves above it)
-template <int NC> __device__ __forceinline__ void tmem_wait(uint32_t (&r)[NC]) {
-    tc_wait_ld();
-#pragma unroll
-    for (int j = 0; j < NC; ++j) asm volatile("" : "+r"(r[j]));
-}
-__device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ bool elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r != 0;
-}
-__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t more) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(more) : "memory");
-}
-
-// two floats as pairs of bf16 terms; a and b become the remainders
-__device__ __forceinline__ uint32_t next_terms(float& a, float& b) {
-    const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(&t);
-    a -= __uint_as_float(w << 16);
-    b -= __uint_as_float(w & 0xffff0000u);
-    return w;
 }
 
 // Two floats at a time, each rounded as a sum of its own.

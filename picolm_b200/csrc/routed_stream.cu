@@ -109,7 +109,7 @@ moe_stream_kernel(const __grid_constant__ CUtensorMap map_1, const __grid_consta
 
     if (warp == CONSUMERS) {
         // ------------------------------------------------------------ tensor copies
-        if (lane == 0) {
+        if (elect_one()) {
             int i = 0;                                 // stages issued
             for (int j = begin; j < end;) {
                 const Unit u = unit_at(j, end, tiles, pieces);

@@ -18,7 +18,7 @@
 // 2,048 tokens, 8 heads of 128 x 128: the delta rule 518 us (32 tokens at a time, everything but the scaled keys and queries in
 // the chain) -> 145, linear attention 144 us (token by token in segments) -> 93; errors against 64 bits 4.9e-7 -> 2.0e-7 and
 // 2.0e-6 -> 2.7e-7 (outputs), 6.2e-7 -> 2.1e-7 and 2.4e-6 -> 1.6e-7 (state).
-#include "tc_common.cuh"
+#include "split_common.cuh"
 #include <type_traits>
 
 namespace {
@@ -769,6 +769,342 @@ chunk_out_kernel(const Args a) {
         }
 }
 
+// The two products whose sides need no order between chunks, on the tensor cores: with OUT a chunk's O = Q S + M U, without it
+// what a chunk of linear attention adds to the state, sum_s (k_s e^(L_C - L_s)) v_s^T.  A unit is one of these for 128 columns of
+// the state: they are the MMA's rows, the chunk's tokens (or the state's channels) its columns, and the sums run over 32 rows of
+// both operands at a time, every float in three bf16 terms as in gemm_f32_tc.cu.  Sums of pieces are added in fp32: the error
+// against 64 bits is below that of the FFMA tiles, whose chains are six times as long.
+// A CTA stays and walks over units; its warps' parts are those of gemm_f32_tc.cu, except that the operands come as plain bulk
+// copies (their rows lie row by row in the workspace) and both are transposed on the way: a lane of the splitting warps reads one
+// column's 32 rows for tensor memory, and the other operand stays as it lies, rows of 128 bytes with the 128-byte swizzle that
+// the MMA reads with its N contiguous.
+// Bound by the MMAs (12 a step of 64 columns, 60 to 80 cycles each) and by the hand-overs.  OUT_FIGURES
+constexpr int TC_FOLDERS = 8, TC_LOADER = 16, TC_ISSUER = 17, TC_THREADS = 640, TC_RING = 4, TC_ROWS = 128, TC_STEP = 32;
+
+template <int NB> struct TcTile {                                // NB columns of a unit: 64 or 128
+    static constexpr int RAW_P = TC_STEP * TC_ROWS * 4, RAW = RAW_P + TC_STEP * NB * 4;
+    static constexpr int BLOCK = TC_STEP * 128, TERM = NB / 64 * BLOCK, TERMS = 3 * TERM;
+    static constexpr int TERMS_P = 2 * NB, TMEM = TERMS_P + 2 * 48 <= 256 ? 256 : 512;
+    static constexpr size_t SMEM = TC_RING * RAW + 2 * TERMS + 1024;
+};
+
+// sums over the rows that a result depends on, one after the other (a result that is not finite: the split makes no numbers of
+// infinities, and later tokens' zero weights make none of theirs)
+template <int NP, bool OUT>
+__device__ __noinline__ float sum_again(const float* w, int PP, int p, int col) {
+    using Lay = Layout<NP>;
+    float sum = 0.f;
+    if (OUT) {
+#pragma unroll 1
+        for (int n = 0; n < NP; ++n) sum = fmaf(w[Lay::QT + n * C + col], w[Lay::s(PP) + (long)n * PP + p], sum);
+#pragma unroll 1
+        for (int s = 0; s <= col; ++s) sum = fmaf(w[Lay::MT + s * C + col], w[Lay::U + (long)s * PP + p], sum);
+    } else {
+#pragma unroll 1
+        for (int s = 0; s < C; ++s) sum = fmaf(w[Lay::KE + s * NP + col], w[Lay::U + (long)s * PP + p], sum);
+    }
+    return sum;
+}
+
+template <int NP, bool OUT>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_constant__ CUtensorMap map_u, const Args a, int b_first, int chunks, int n_units) {
+    using Lay = Layout<NP>;
+    constexpr int NB = OUT ? C : NP, STEPS = OUT ? (NP + C) / TC_STEP : C / TC_STEP, R = TC_RING, COLS = NB / 2;
+    using T = TcTile<NB>;
+    // D fp32, A and B bf16, B with N contiguous
+    constexpr uint32_t IDESC = plm_tc::instr_desc_bf16(NB) | (1u << 16);
+    static_assert(R % 2 == 0 && STEPS % 2 == 0, "a splitting warp must not take a phase for the one after the next");
+    extern __shared__ unsigned char tc_raw[];
+    __shared__ uint64_t bars[2 * R + 4];
+    __shared__ uint32_t tmem_at;
+    unsigned char* smem = tc_raw + ((1024 - (plm_tc::smem_u32(tc_raw) & 1023)) & 1023);
+    unsigned char* terms = smem + R * T::RAW;
+    const uint32_t bar0 = plm_tc::smem_u32(bars);
+    auto raw_full = [&](int b) { return bar0 + 8 * b; };
+    auto raw_empty = [&](int b) { return bar0 + 8 * (R + b); };
+    auto terms_full = [&](int b) { return bar0 + 8 * (2 * R + b); };
+    auto mma_done = [&](int b) { return bar0 + 8 * (2 * R + 2 + b); };
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    pdl_launch_dependents();
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(plm_tc::smem_u32(&tmem_at)), "r"(T::TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int b = 0; b < R; ++b) {
+            plm_tc::mbar_init(raw_full(b), 1);
+            plm_tc::mbar_init(raw_empty(b), 4);
+        }
+        for (int b = 0; b < 2; ++b) {
+            plm_tc::mbar_init(terms_full(b), 4 + TC_FOLDERS);    // the terms are there and the accumulator is read
+            plm_tc::mbar_init(mma_done(b), 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    plm_tc::tc_fence_before();
+    __syncthreads();
+    plm_tc::tc_fence_after();
+    pdl_wait();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_at, 0);
+    const int PP = pad4(a.P), ptiles = (PP + TC_ROWS - 1) / TC_ROWS;
+    struct Unit { const float* w; int block, p0, h, t0, nt; };     // block: the (chunk, head)'s place in the workspace
+    auto unit_at = [&](int u) {                                  // (nt <= 0: nothing there)
+        Unit x;
+        x.nt = 0;
+        if (u >= n_units) return x;
+        const unsigned v = (unsigned)u / (unsigned)ptiles, cb = v / (unsigned)chunks;
+        x.p0 = (int)((unsigned)u - v * ptiles) * TC_ROWS;
+        const int c = a.c0 + (int)(v - cb * chunks), b = b_first + (int)(cb / (unsigned)a.H), s0 = a.seq_start[b];
+        x.h = (int)(cb % (unsigned)a.H);
+        x.t0 = s0 + c * C;
+        x.nt = min(C, a.seq_start[b + 1] - x.t0);
+        x.block = (int)(a.slot(s0, b, c) * a.H + x.h);
+        x.w = a.ws + x.block * Lay::floats(PP);
+        return x;
+    };
+    // (a warp looks a unit up while it works on the one before)
+    Unit next = unit_at(blockIdx.x);
+    bool ok = true;
+    int at = 0;                                                  // steps so far, over all units
+    if (warp >= TC_LOADER) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
+            const Unit x = next;
+            next = unit_at(u + gridDim.x);
+            if (x.nt <= 0) continue;
+            if (warp == TC_LOADER) {
+                for (int s = 0; s < STEPS; ++s, ++at) {
+                    const int b = at % R;
+                    if (at >= R) ok = ok && plm_tc::mbar_wait(raw_empty(b), ((at - R) / R) & 1, a.status, 44);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    const int j = s - NP / TC_STEP;              // OUT: Q and S first, then M and U
+                    const bool first = OUT && j < 0;
+                    const float* n_rows = OUT ? (j < 0 ? x.w + Lay::QT + (long)s * TC_STEP * C : x.w + Lay::MT + (long)j * TC_STEP * C)
+                                              : x.w + Lay::KE + (long)s * TC_STEP * NP;
+                    const uint32_t to = plm_tc::smem_u32(smem + b * T::RAW);
+                    if (plm_tc::elect_one()) {
+                        plm_tc::mbar_expect_tx(raw_full(b), T::RAW);
+                        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                                     ::"r"(to), "l"((uint64_t)(first ? &map_s : &map_u)), "r"(raw_full(b)), "r"(x.p0),
+                                       "r"((OUT && !first ? j : s) * TC_STEP), "r"(x.block) : "memory");
+                        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                     ::"r"(to + T::RAW_P), "l"(n_rows), "r"(TC_STEP * NB * 4), "r"(raw_full(b)) : "memory");
+                    }
+                    __syncwarp();
+                }
+                if (!ok) {                                       // a wait ran out: no copy may be under way when the CTA ends
+                    for (int i = max(0, at - R); i < at; ++i) plm_tc::mbar_wait(raw_full(i % R), (i / R) & 1, nullptr, 0);
+                    break;
+                }
+            } else if (warp == TC_ISSUER || warp == TC_ISSUER + 1) {         // every other step each, the smallest products first
+                const int b = warp - TC_ISSUER;
+                const uint32_t p = tmem + T::TERMS_P + b * 48, d = tmem + b * NB;
+                const uint32_t n0 = plm_tc::smem_u32(terms + b * T::TERMS);
+                // N contiguous: blocks of 64 columns BLOCK bytes apart, eight rows of K 1,024
+                const uint64_t n = (uint64_t)((n0 & 0x3FFFFu) >> 4) | ((uint64_t)(T::BLOCK >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
+                                   ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+                for (int s = (at ^ b) & 1; s < STEPS && ok; s += 2) {
+                    ok = plm_tc::mbar_wait_warp(terms_full(b), ((at + s) >> 1) & 1, a.status, 45);
+                    if (!ok) break;
+                    plm_tc::tc_fence_after();
+                    constexpr int TP[6] = {1, 2, 0, 1, 0, 0}, TN[6] = {1, 0, 2, 0, 1, 0};
+                    if (plm_tc::elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < 6; ++i)
+#pragma unroll
+                            for (int k = 0; k < TC_STEP / 16; ++k)
+                                plm_split::mma_ts(d, p + TP[i] * 16 + k * 8, n + (TN[i] * T::TERM + k * 2048) / 16, IDESC, i + k > 0);
+                        plm_tc::tc_commit(mma_done(b));
+                    }
+                    __syncwarp();
+                }
+                at += STEPS;
+                if (!ok) break;
+            }
+        }
+        __syncwarp();
+    } else if (warp >= TC_FOLDERS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+        const int group = (warp - TC_FOLDERS) / 4, member = warp % 4;
+        const uint32_t p_to = tmem + ((uint32_t)(member * 32) << 16) + T::TERMS_P + group * 48;
+        unsigned char* n_to = terms + group * T::TERMS;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const bool some = next.nt > 0;
+            next = unit_at(u + gridDim.x);
+            if (!some) continue;
+            for (int s = group; s < STEPS; s += 2) {             // (a unit has an even number of steps)
+                const int now = at + s, b = now % R;
+                ok = ok && plm_tc::mbar_wait(raw_full(b), (now / R) & 1, a.status, 46);
+                const float* raw_p = reinterpret_cast<const float*>(smem + b * T::RAW) + member * 32 + lane;
+                const float* raw_n = reinterpret_cast<const float*>(smem + b * T::RAW + T::RAW_P);
+                uint32_t w[2][3][8];                             // (before the MMAs that read the buffers last are waited for)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    float v[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) v[i] = raw_p[(half * 16 + i) * TC_ROWS];
+#pragma unroll
+                    for (int t = 0; t < 3; ++t)
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) w[half][t][i] = plm_split::next_terms(v[2 * i], v[2 * i + 1]);
+                }
+                if (now >= 2) ok = ok && plm_tc::mbar_wait(mma_done(group), ((now - 2) >> 1) & 1, a.status, 46);
+                __syncwarp();
+                plm_tc::tc_fence_after();
+#pragma unroll
+                for (int half = 0; half < 2; ++half)
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) plm_split::tmem_store8(p_to + t * 16 + half * 8, w[half][t]);
+#pragma unroll
+                for (int i = 0; i < TC_STEP * (NB / 8) / 128; ++i) {         // eight columns of a row
+                    const int item = i * 128 + member * 32 + lane, k = item / (NB / 8), c8 = item % (NB / 8);
+                    float v[8];
+                    *reinterpret_cast<float4*>(v) = ld4(raw_n + k * NB + c8 * 8);
+                    *reinterpret_cast<float4*>(v + 4) = ld4(raw_n + k * NB + c8 * 8 + 4);
+                    unsigned char* to = n_to + c8 / 8 * T::BLOCK + k * 128 + ((c8 % 8) ^ (k & 7)) * 16;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        uint4 x;
+                        x.x = plm_split::next_terms(v[0], v[1]);
+                        x.y = plm_split::next_terms(v[2], v[3]);
+                        x.z = plm_split::next_terms(v[4], v[5]);
+                        x.w = plm_split::next_terms(v[6], v[7]);
+                        *reinterpret_cast<uint4*>(to + t * T::TERM) = x;
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                plm_tc::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    plm_split::mbar_arrive(terms_full(group));
+                    plm_split::mbar_arrive(raw_empty(b));
+                }
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            at += STEPS;
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
+        const uint32_t lanes = tmem + ((uint32_t)(warp % 4 * 32) << 16);
+        const int c0 = warp / 4 * COLS;
+        if (lane == 0) {                                         // both accumulators are free
+            plm_split::mbar_arrive(terms_full(0));
+            plm_split::mbar_arrive(terms_full(1));
+        }
+        __syncwarp();
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const Unit x = next;
+            next = unit_at(u + gridDim.x);
+            if (x.nt <= 0) continue;
+            float sum[COLS];
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+#pragma unroll 1
+            for (int s = 0; s < STEPS; ++s, ++at) {
+                const int b = at & 1;
+                ok = ok && plm_tc::mbar_wait(mma_done(b), (at >> 1) & 1, a.status, 47);
+                __syncwarp();
+                plm_tc::tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < COLS; c += 32) {
+                    uint32_t r[32];
+                    plm_split::tmem_load<32>(lanes + b * NB + c0 + c, r);
+                    plm_split::tmem_wait<32>(r);
+                    if (c + 32 == COLS) {
+                        plm_tc::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) plm_split::mbar_arrive(terms_full(b));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) sum[c + j] += __uint_as_float(r[j]);
+                }
+            }
+            const int p = x.p0 + warp % 4 * 32 + lane;
+            if (OUT) {
+                float* y = a.y + (long)x.t0 * a.H * a.P + (long)x.h * a.P + p;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) {
+                    const int t = c0 + j;
+                    if (p < a.P && t < x.nt) {
+                        if (!(fabsf(sum[j]) < INFINITY)) sum[j] = sum_again<NP, true>(x.w, PP, p, t);
+                        y[(long)t * a.H * a.P] = sum[j];
+                    }
+                }
+            } else {
+                float* s_to = const_cast<float*>(x.w) + Lay::s(PP) + p;
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) {
+                    const int n = c0 + j;
+                    if (p < PP) {                                // (padding stays zero, whatever U holds)
+                        if (!(fabsf(sum[j]) < INFINITY)) sum[j] = sum_again<NP, false>(x.w, PP, p, n);
+                        s_to[(long)n * PP] = n < a.N ? sum[j] : 0.f;
+                    }
+                }
+            }
+            __syncwarp();
+            ok = __all_sync(0xffffffffu, ok);
+        }
+        plm_tc::tc_fence_before();
+    }
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::TMEM) : "memory");
+}
+
+// A workspace's rows of PP values, `rows` of them in every block of `block_floats`, as boxes of 32 rows x 128 columns (a copy of a
+// row each, 33 a step, took three times the MMAs' time); kept by what they describe, as plm_tc::make_map's.
+int make_rows_map(CUtensorMap* map, const float* first, int PP, int rows, long block_floats, long blocks) {
+    struct Entry { const float* first; int PP, rows; long block_floats, blocks; bool used; CUtensorMap map; };
+    constexpr int SLOTS = 64;
+    static Entry table[SLOTS];
+    static std::mutex lock;
+    Entry& e = table[((((size_t)first >> 4) * 0x9E3779B97F4A7C15ull + (size_t)rows * 31 + (size_t)blocks * 131 + PP) >> 20) % SLOTS];
+    {
+        std::lock_guard<std::mutex> g(lock);
+        if (e.used && e.first == first && e.PP == PP && e.rows == rows && e.block_floats == block_floats && e.blocks == blocks) {
+            *map = e.map;
+            return PLM_OK;
+        }
+    }
+    plm_tc::EncodeTiledFn fn = plm_tc::encode_fn();
+    if (!fn) return PLM_ERR_UNSUPPORTED;
+    cuuint64_t dims[3] = {(cuuint64_t)PP, (cuuint64_t)rows, (cuuint64_t)blocks};
+    cuuint64_t strides[2] = {(cuuint64_t)PP * 4, (cuuint64_t)block_floats * 4};
+    cuuint32_t box[3] = {(cuuint32_t)TC_ROWS, (cuuint32_t)TC_STEP, 1}, estr[3] = {1, 1, 1};
+    if (fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(first), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return PLM_ERR_ALIGN;
+    std::lock_guard<std::mutex> g(lock);
+    e.first = first; e.PP = PP; e.rows = rows; e.block_floats = block_floats; e.blocks = blocks; e.map = *map; e.used = true;
+    return PLM_OK;
+}
+
+template <int NP, bool OUT>
+int launch_product(const Args& a, long ws_floats, int n_seqs, unsigned chunks, cudaStream_t stream) {
+    using Lay = Layout<NP>;
+    static std::atomic<unsigned long long> devices{0};
+    constexpr size_t SMEM = TcTile<OUT ? C : NP>::SMEM;
+    static_assert(SMEM <= 232448 - 256, "shared memory");
+    const cudaError_t ok = plm_allow_smem(chunk_product_kernel<NP, OUT>, SMEM, devices);
+    if (ok != cudaSuccess) return (int)ok;
+    const int PP = pad4(a.P);
+    const long blocks = ws_floats / Lay::floats(PP), of_sequence = (long)chunks * ((PP + TC_ROWS - 1) / TC_ROWS) * a.H;
+    CUtensorMap map_s, map_u;
+    int r = make_rows_map(&map_s, a.ws + Lay::s(PP), PP, NP, Lay::floats(PP), blocks);
+    if (r == PLM_OK) r = make_rows_map(&map_u, a.ws + Lay::U, PP, C, Lay::floats(PP), blocks);
+    // (a launch's units, and a unit behind them, are counted in 32 bits: more of them take several launches)
+    if (of_sequence > (1l << 30) || blocks > 0x7fffffffl) return PLM_ERR_SHAPE;
+    const int at_once = (int)((1l << 30) / of_sequence < n_seqs ? (1l << 30) / of_sequence : n_seqs);
+    for (int first = 0; r == PLM_OK && first < n_seqs; first += at_once) {
+        const int units = (int)(of_sequence * (n_seqs - first < at_once ? n_seqs - first : at_once));
+        r = plm_status_of(launch_pdl(chunk_product_kernel<NP, OUT>, dim3((unsigned)(units < PLM_SM_COUNT ? units : PLM_SM_COUNT)), dim3(TC_THREADS), SMEM,
+                                     stream, map_s, map_u, a, a.b0 + first, (int)chunks, units));
+    }
+    return r;
+}
+
 template <int NP, bool STRETCH>
 cudaError_t launch_walk(const Args& a, int n_seqs, cudaStream_t stream) {
     static std::atomic<unsigned long long> devices{0};
@@ -778,37 +1114,42 @@ cudaError_t launch_walk(const Args& a, int n_seqs, cudaStream_t stream) {
                       walk_smem<NP>(), stream, a);
 }
 
-template <int NP, typename T, bool DELTA, int PT>
-int run_stretch(const Args& a, int n_seqs, unsigned chunks, cudaStream_t stream) {
+template <int NP, typename T, bool DELTA, bool TC>
+int run_stretch(const Args& a, long ws_floats, int n_seqs, unsigned chunks, cudaStream_t stream) {
     static std::atomic<unsigned long long> devices{0};
     const cudaError_t prep_ok = plm_allow_smem(chunk_prep_kernel<T, NP, DELTA>, prep_smem<NP>(), devices);
     if (prep_ok != cudaSuccess) return (int)prep_ok;
-    const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
+    constexpr int PT = 64;               // columns of an FFMA tile: a P of at most 64 is one
     cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, a.H, n_seqs), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
     if (e != cudaSuccess) return (int)e;
     if (DELTA) {
         e = a.stretch ? launch_walk<NP, true>(a, n_seqs, stream) : launch_walk<NP, false>(a, n_seqs, stream);
     } else {
-        e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * ptiles * (NP / 64), a.H, n_seqs), dim3(128), 0, stream, a);
+        if constexpr (TC) {
+            const int r = launch_product<NP, false>(a, ws_floats, n_seqs, chunks, stream);
+            if (r != PLM_OK) return r;
+        } else
+            e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * (NP / 64), a.H, n_seqs), dim3(128), 0, stream, a);
         if (e != cudaSuccess) return (int)e;
-        e = launch_pdl(chunk_chain_kernel<NP>, dim3((NP * (PP / 4) + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a);
+        e = launch_pdl(chunk_chain_kernel<NP>, dim3((NP * (pad4(a.P) / 4) + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a);
     }
     if (e != cudaSuccess) return (int)e;
-    return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks * ptiles, a.H, n_seqs), dim3(128), 0, stream, a));
+    if constexpr (TC) return launch_product<NP, true>(a, ws_floats, n_seqs, chunks, stream);
+    else return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks, a.H, n_seqs), dim3(128), 0, stream, a));
 }
 
 // The whole step at once where the workspace holds it.  Else so many chunks of so many sequences at a time as it holds: a state
 // that a stretch leaves is what the next one starts from, as from step to step, so results are the same to the bit.
-template <int NP, typename T, bool DELTA, int PT>
+template <int NP, typename T, bool DELTA, bool TC>
 int run(Args a, int n_tokens, int n_seqs, int max_new, long ws_floats, cudaStream_t stream) {
     const long chunks = (max_new + C - 1) / C, slots = ws_floats / (a.H * Layout<NP>::floats(pad4(a.P)));
-    if ((long)n_tokens / C + n_seqs <= slots) return run_stretch<NP, T, DELTA, PT>(a, n_seqs, (unsigned)chunks, stream);
+    if ((long)n_tokens / C + n_seqs <= slots) return run_stretch<NP, T, DELTA, TC>(a, ws_floats, n_seqs, (unsigned)chunks, stream);
     if (slots < 1) return PLM_ERR_SHAPE;
     const int group = (int)(n_seqs < slots ? n_seqs : slots);
     a.stretch = (int)(slots / group < chunks ? slots / group : chunks);
     for (a.b0 = 0; a.b0 < n_seqs; a.b0 += group)
         for (a.c0 = 0; a.c0 < chunks; a.c0 += a.stretch) {
-            const int e = run_stretch<NP, T, DELTA, PT>(a, n_seqs - a.b0 < group ? n_seqs - a.b0 : group, (unsigned)a.stretch, stream);
+            const int e = run_stretch<NP, T, DELTA, TC>(a, ws_floats, n_seqs - a.b0 < group ? n_seqs - a.b0 : group, (unsigned)a.stretch, stream);
             if (e != PLM_OK) return e;
         }
     return PLM_OK;
@@ -816,11 +1157,12 @@ int run(Args a, int n_tokens, int n_seqs, int max_new, long ws_floats, cudaStrea
 
 template <typename T, bool DELTA>
 int by_size(const Args& a, int n_tokens, int n_seqs, int max_new, long ws_floats, cudaStream_t stream) {
+    // (a state of at most 64 columns would leave half of the MMA's rows idle: those run as FFMA tiles)
     if (a.N <= 64)
-        return a.P <= 64 ? run<64, T, DELTA, 64>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
-                         : run<64, T, DELTA, 128>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
-    return a.P <= 64 ? run<128, T, DELTA, 64>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
-                     : run<128, T, DELTA, 128>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
+        return a.P <= 64 ? run<64, T, DELTA, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                         : run<64, T, DELTA, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
+    return a.P <= 64 ? run<128, T, DELTA, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream)
+                     : run<128, T, DELTA, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }
 
 int check(const Args& a, int n_seqs, int max_new, int dtype) {
@@ -852,6 +1194,14 @@ extern "C" int plm_delta_channel_scan(const float* qn, const float* kn, const fl
                             : by_size<bf16, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }
 
+// The device word where this thread's launches of plm_sigmoid_chunk_scan leave a wait that ran out (a launch takes it along as an
+// argument).
+static thread_local int* g_sigmoid_status = nullptr;
+extern "C" int plm_sigmoid_chunk_status(int* status) {
+    g_sigmoid_status = status;
+    return PLM_OK;
+}
+
 // Linear attention with the decays sigmoid(raw + bias)^power: q, k, v, raw of `dtype`.
 extern "C" int plm_sigmoid_chunk_scan(const void* q, const void* k, const void* v, const void* raw, int dtype, long ldq, long ldk, long ldv,
                                       long ldr, const float* bias, float q_scale, float power, float* state, long state_stride, float* y,
@@ -861,7 +1211,7 @@ extern "C" int plm_sigmoid_chunk_scan(const void* q, const void* k, const void* 
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     const Args a = {q, k, v, raw, ldq, ldk, ldv, ldr, nullptr, bias, power, q_scale, ws, state, state_stride, y, seq_start, seq_slot,
                     H, N, P, heads_per_group, 0,
-                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, nullptr, 0, 0, 0};
+                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, g_sigmoid_status, 0, 0, 0};
     const int e = check(a, n_seqs, max_new, dtype);
     if (e != PLM_OK) return e;
     return dtype == PLM_F32 ? by_size<float, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream)

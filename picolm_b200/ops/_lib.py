@@ -92,6 +92,7 @@ _SIGNATURES = {
     "plm_delta_scan": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _l, _vp, _l, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
     "plm_scan_chunk_floats": [_i, _i],
     "plm_delta_channel_scan": [_vp, _vp, _vp, _vp, _vp, _i, _l, _vp, _l, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
+    "plm_sigmoid_chunk_status": [_vp],
     "plm_sigmoid_chunk_scan": [_vp, _vp, _vp, _vp, _i, _l, _l, _l, _l, _vp, _f, _f, _vp, _l, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
     "plm_linear_scan": [_vp, _vp, _vp, _vp, _i, _l, _l, _l, _l, _i, _vp, _vp, _vp, _f, _f, _vp, _l, _vp, _l, _vp, _vp,
                         _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp],
@@ -258,16 +259,23 @@ def _dev(t: torch.Tensor, name: str) -> None:
 
 
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()              # (the entry points' argument types make a pointer of it)
 
 
 _bound_stream = None
+# the current stream's handle without a torch.cuda.Stream around it (some five microseconds a launch: a layer of ten launches
+# outside a scope took 255 us of host time, HOST_NOW with this and pointers as plain numbers)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def _current_stream():
+    if _raw_stream is not None:
+        return _raw_stream(torch.cuda.current_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _stream():
-    if _bound_stream is not None:
-        return _bound_stream
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _bound_stream if _bound_stream is not None else _current_stream()
 
 
 class stream_scope:
@@ -278,7 +286,7 @@ class stream_scope:
     def __enter__(self):
         global _bound_stream
         self.outer = _bound_stream
-        _bound_stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _bound_stream = _current_stream()
         return self
 
     def __exit__(self, *exc):
@@ -356,7 +364,8 @@ def set_bounds(library: str, extra_flags=(), *, n_pages: int = 0, n_seqs: int = 
 
 # What the status word says: what the checked build met (csrc/common.cuh), or whose wait ran out.
 _OUT_OF_BOUNDS = {16: "page number", 17: "sequence index", 18: "position", 19: "row index"}
-_WAITS = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting", 5: "a decode step's pages", 40: "the walk over chunks",
+_WAITS = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting", 5: "a decode step's pages", 40: "the walk over chunks", 44: "the chunks' TMA producer", 45: "the chunks' MMA issuer",
+          46: "the chunks' split", 47: "the chunks' sums",
           41: "the experts' streamed weights", 42: "the experts' streamed products", 43: "the experts' streamed rows",
           51: "the experts' TMA producer", 52: "the experts' MMA issuer, results unread", 53: "the experts' MMA issuer",
           54: "the experts' epilogue", 60: "the float32 product's TMA producer", 61: "the float32 product's MMA issuer",
