@@ -47,6 +47,7 @@ LIBRARIES: Dict[str, List[str]] = {
     "routed_stream": ["routed_stream.cu"],
     "routed_tc": ["routed_tc.cu"],
     "decay_chunk": ["decay_chunk.cu"],
+    "decay_tc": ["decay_tc.cu"],
     "delta_chunk": ["delta_chunk.cu"],
     "scan_chunk": ["scan_chunk.cu"],
 }

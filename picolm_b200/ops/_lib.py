@@ -25,6 +25,8 @@ _SIGNATURES = {
     "plm_squash": [_vp, _l, _f, _f, _vp],
     "plm_decay_step": [_vp, _vp, _vp, _i, _l, _l, _l, _vp, _vp, _l, _vp, _l, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _f, _vp],
     "plm_rotate_rows": [_vp, _vp, _vp, _i, _l, _l, _l, _vp, _vp, _vp, _i, _f, _vp, _vp, _i, _i, _i, _i, _vp],
+    "plm_decay_tc_floats": [_i, _i, _i, _i, _i, _i, _i],
+    "plm_decay_tc_scan": [_vp, _vp, _vp, _l, _l, _l, _vp, _vp, _l, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp, _vp, _i, _f, _vp, _vp, _vp],
     "plm_decay_chunk_plan": [_i, _i, _i, _i, _i, _i, _vp],
     "plm_decay_chunk_scan": [_vp, _vp, _vp, _l, _l, _l, _vp, _vp, _l, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _i, _i, _vp, _vp,
                              _vp, _i, _f, _vp],
@@ -365,7 +367,7 @@ def set_bounds(library: str, extra_flags=(), *, n_pages: int = 0, n_seqs: int = 
 # What the status word says: what the checked build met (csrc/common.cuh), or whose wait ran out.
 _OUT_OF_BOUNDS = {16: "page number", 17: "sequence index", 18: "position", 19: "row index"}
 _WAITS = {1: "TMA producer", 2: "MMA issuer", 3: "epilogue", 4: "the CTAs' meeting", 5: "a decode step's pages", 40: "the walk over chunks", 44: "the chunks' TMA producer", 45: "the chunks' MMA issuer",
-          46: "the chunks' split", 47: "the chunks' sums",
+          46: "the chunks' split", 47: "the chunks' sums", 48: "a retention chunk's products",
           41: "the experts' streamed weights", 42: "the experts' streamed products", 43: "the experts' streamed rows",
           51: "the experts' TMA producer", 52: "the experts' MMA issuer, results unread", 53: "the experts' MMA issuer",
           54: "the experts' epilogue", 60: "the float32 product's TMA producer", 61: "the float32 product's MMA issuer",

@@ -277,6 +277,12 @@ def decay_chunk_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key
             and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, k, v)))
 
 
+# tokens of a step's longest sequence, and of its sequences on average, from which a constant decay's recurrence over rotated
+# rows runs 128 tokens at a time on tcgen05: below, a chunk is mostly empty (16 heads of 128 x 256, us 64 at a time / 128: one
+# sequence of 65 tokens 17 / 20, of 129 26 / 22, of 256 35 / 22, of 2,048 107 / 66; three of 100, 40, 30 21 / 26)
+DECAY_TC_FROM = 129
+
+
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, powers: torch.Tensor,
                state: torch.Tensor, step, heads: int, key_dim: int, value_dim: int,
                activation: Optional[str] = None, rotation=None, k_scale: Optional[float] = None) -> torch.Tensor:
@@ -307,6 +313,16 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if state.dtype != torch.float32 or state.shape[1] < H * N * P:
         raise KernelError("decay_scan: the state must be float32 with heads * key_dim * value_dim values a row")
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
+    floats = _decay_tc_floats(T, step.n_seqs, step.max_new, H, N, P, turn)
+    if floats:
+        ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
+        _check(_fn("decay_tc", "plm_decay_tc_scan")(
+            _p(q), _p(k), _p(v), ldq, ldk, ldv, _p(powers), _p(state), lds, _p(y), H * P, _p(step.seq_start), _p(step.seq_slot), T,
+            step.n_seqs, int(step.max_new), H, N, P, *_turn_args(turn, step, False), _p(ws), _p(status_word(v.device)), _stream()),
+            f"decay_tc_scan T={T} H={H} N={N} P={P}", kernels=3,
+            nbytes=T * (2 * H * N + H * P) * v.element_size() + T * H * P * 4 + 2 * step.n_seqs * H * N * P * 4,
+            flops=2 * T * H * (128 // 2 * (N + P) + 2 * N * P))
+        return y
     seg_len, n_segs = _decay_chunk_plan(step.n_seqs, H, N, P, step.max_new, T)
     seg_state = torch.empty((step.n_seqs, n_segs, H * N * P), dtype=torch.float32, device=v.device) if n_segs > 1 else None
     _check(_fn("decay_chunk", "plm_decay_chunk_scan")(
@@ -318,6 +334,13 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
         nbytes=T * (2 * H * N + H * P) * v.element_size() + T * H * P * 4 + 2 * step.n_seqs * H * N * P * 4,
         flops=2 * T * H * (DECAY_CHUNK // 2 * (N + P) + 2 * N * P))
     return y
+
+
+def _decay_tc_floats(n_tokens: int, n_seqs: int, max_new: int, H: int, N: int, P: int, turn) -> int:
+    """Floats of workspace that a step takes on tcgen05, 128 tokens at a time (csrc/decay_tc.cu); 0: it runs 64 at a time."""
+    if turn is None or max_new < DECAY_TC_FROM or n_tokens < DECAY_TC_FROM * n_seqs:
+        return 0
+    return _fn("decay_tc", "plm_decay_tc_floats")(n_tokens, n_seqs, int(max_new), H, N, P, turn.half)
 
 
 class _Turn:

@@ -138,3 +138,72 @@ def test_chunk_products_keep_what_is_not_finite_where_it_belongs():
     assert not torch.isfinite(got[100:, 5]).any() and torch.isnan(got[150:, 200]).all()
     keep = [c for c in range(H * P) if c not in (5, 200)]
     assert torch.equal(got[:, keep], clean[:, keep])
+
+
+def _retention(N, P, lens, H=3, positions=0, odd=None):
+    """ops.decay_scan over rotated rows, its inputs, and the same in float64 with everything that the kernels are handed."""
+    from picolm_b200 import ops
+    torch.manual_seed(N + P + sum(lens))
+    T = sum(lens)
+    start = [sum(lens[:b]) for b in range(len(lens))]
+    step = _step(lens)
+    step.tok_pos = _i32([positions + p for n in lens for p in range(n)])
+    step.max_position = positions + max(lens) - 1
+    rows = torch.randn(T, 2 * H * N + H * P).to(torch.bfloat16).to(DEV)
+    q, k, v = rows[:, :H * N], rows[:, H * N:2 * H * N], rows[:, 2 * H * N:]
+    if odd:
+        for t, c, x in odd:
+            v[t, c] = x
+    decay = torch.tensor([1.0 - 2.0 ** (-3.0 - 2 * h) for h in range(H)], dtype=torch.float64)
+    half = N // 2
+    angle = torch.arange(positions + max(lens), dtype=torch.float64)[:, None] * 10000.0 ** (-torch.arange(half, dtype=torch.float64) / half)
+    rotation = types.SimpleNamespace(cos=angle.cos().float().to(DEV), sin=angle.sin().float().to(DEV), rotary_dim=N, pairing="half")
+    state = torch.randn(len(lens), H * N * P, device=DEV)
+    before = state.clone()
+    y = ops.decay_scan(q, k, v, decay.float().to(DEV), ops.decay_powers(decay).to(DEV), state, step, H, N, P, rotation=rotation, k_scale=N ** -0.5)
+    want, states = [], []
+    for b, n in enumerate(lens):
+        c, s = (f[positions:positions + n].double()[:, None] for f in (rotation.cos, rotation.sin))
+        turn = lambda x: (lambda u, w: torch.cat([u * c - w * s, w * c + u * s], -1))(*x[start[b]:start[b] + n].double().view(n, H, N).split(half, -1))
+        qq, kk, vv = turn(q), turn(k) * N ** -0.5, v[start[b]:start[b] + n].double().view(n, H, P)
+        S, out = before[b].double().view(H, N, P), []
+        for i in range(n):
+            S = S * decay.to(DEV)[:, None, None] + kk[i][:, :, None] * vv[i][:, None]
+            out.append(torch.bmm(qq[i][:, None], S)[:, 0].reshape(-1))
+        want.append(torch.stack(out))
+        states.append(S.reshape(-1))
+    ops.check_status(DEV)
+    return y, torch.cat(want), state, torch.stack(states)
+
+
+@pytest.mark.parametrize("N,P", [(64, 128), (128, 128), (128, 256), (64, 384)])
+@pytest.mark.parametrize("lens", [[129], [128, 150, 200], [513, 70, 3], [400, 257]])
+def test_retention_128_tokens_at_a_time(N, P, lens):
+    """Chunks that end early, sequences in the midst of others, several value tiles, a state that is carried on, positions that do
+    not begin at 0."""
+    y, want, state, states = _retention(N, P, lens, positions=17)
+    # operands in two bf16 terms: 2^-17 of each at most, two or three a product
+    assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
+    for t in range(0, want.shape[0], 37):
+        assert (y[t].double() - want[t]).norm() <= 6 * 2.0 ** -17 * want[t].norm()
+
+
+def test_many_retention_chunks_share_their_weights_between_value_tiles():
+    y, want, state, states = _retention(128, 256, [1200, 1100], H=9)
+    assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
+
+
+@pytest.mark.parametrize("H", [2, 40])
+def test_retention_keeps_what_is_not_finite_where_it_belongs(H):
+    """(2 heads: a CTA a value tile; 40: a CTA all of them)"""
+    N, P, lens = 64, 256, [300, 200]
+    clean, _, _, _ = _retention(N, P, lens, H=H)
+    odd = [(40, 5, math.inf), (170, 140, math.nan), (299, 3, -math.inf), (300, 200, math.inf)]
+    y, _, state, _ = _retention(N, P, lens, H=H, odd=odd)
+    for t, c, _ in odd:
+        end = 300 if t < 300 else 500
+        assert not torch.isfinite(y[t:end, c]).any()
+        assert torch.equal(y[:t, c], clean[:t, c]) and torch.equal(y[end:, c], clean[end:, c])
+        assert not torch.isfinite(state.view(2, H, N, P)[t // 300, c // P, :, c % P]).all()
+    rest = [c for c in range(H * P) if c not in (5, 140, 3, 200)]
+    assert torch.equal(y[:, rest], clean[:, rest])
