@@ -648,16 +648,15 @@ __global__ void moe_combine_kernel(const float* y, long ldy, const int* where,
 
 // The same sums in the same order with nothing in shared memory: a warp takes TT tokens and EE rows of w, four consecutive k a
 // lane and step, so that a load serves EE or TT products; the lanes' shares meet in a tree that hands every lane one or
-// more of the TT x EE sums.  Large tiles where there are warps for all SMs (bound by the conversions and the second-level cache:
-// each tile reads its rows of h and w once), one token and row a warp below (bound by the loads' latency: sixteen steps are in
-// flight).  2,048 tokens x 32 x 2,048: 26.8 -> 14.2 us; 8 tokens x 16 x 4,096 without warm caches: 19.3 us in
-// tiles of 2 x 2, now 9.7.
+// more of the TT x EE sums.  Bound by the second-level cache where there are many pairs of a token and a row (a tile reads its rows of
+// h and w once) and by the loads' latency where there are few, so the tile grows with the pairs (router_tiles).
 constexpr int RT_WARPS = 4;
+// (Without a number of blocks the compiler keeps to few registers, and so to few loads in flight: 24 us for 11.)
 template <typename Th, typename Tw, int TT, int EE, int AHEAD>
-__global__ void __launch_bounds__(RT_WARPS * 32)
+__global__ void __launch_bounds__(RT_WARPS * 32, TT * EE == 32 && sizeof(Th) + sizeof(Tw) == 4 ? 4 : 1)
 router_tile_kernel(const Th* h, const Tw* w, float* __restrict__ out, int T, int E, int K) {
     constexpr int ACC = TT * EE;
-    static_assert(ACC == 32 || ACC == 1, "the tree below");
+    static_assert(32 % ACC == 0, "the tree below");
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, e_tiles = (E + EE - 1) / EE;
@@ -717,17 +716,27 @@ router_tile_kernel(const Th* h, const Tw* w, float* __restrict__ out, int T, int
         }
     }
     const int t = t0 + at / EE, e = e0 + at % EE;
-    if ((ACC == 32 || lane == 0) && t < T && e < E) out[(size_t)t * E + e] = acc[0];
+    if (lane % (32 / ACC) == 0 && t < T && e < E) out[(size_t)t * E + e] = acc[0];
 }
 
+template <typename Th, typename Tw, int TT, int EE, int AHEAD>
+int router_tile(const void* h, const void* w, float* out, int T, int E, int K, cudaStream_t stream) {
+    const long tiles = (long)((T + TT - 1) / TT) * ((E + EE - 1) / EE);
+    return plm_status_of(launch_pdl(router_tile_kernel<Th, Tw, TT, EE, AHEAD>, dim3((unsigned)((tiles + RT_WARPS - 1) / RT_WARPS)), dim3(RT_WARPS * 32), 0,
+                                    stream, (const Th*)h, (const Tw*)w, out, T, E, K));
+}
+// us in tiles of 1 x 1 / 2 x 2 / 4 x 4 / 8 x 4, inputs not in the first-level cache: bf16, 8 x 16 x 4,096 2.1 / 3.2 / 5.9 / 9.5, 64 x 32 x 2,048
+// 2.6 / 2.5 / 3.6 / 5.5, 128 x 64 x 7,168 13 / 11 / 18 / 23, 512 x 32 x 2,048 8.9 / 5.6 / 7.2 / 8.9, 256 x 128 x 2,048 16 / 9.5 / 8.0 / 10.2,
+// 2,048 x 32 x 2,048 31 / 18 / 15.0 / 23, 4,096 x 128 x 2,048 - / 125 / 91 / 101; float32, 64 x 32 x 2,048 2.8 / 2.8 / 4.3 / 5.5, 512 x 32 x 2,048
+// 14 / 8.2 / 8.4 / 10.4, 256 x 128 x 2,048 24 / 12 / 8.0 / 10.5, 512 x 128 x 7,168 139 / 69 / 43 / 55, 2,048 x 256 x 2,048 - / 172 / 95 / 85.
 template <typename Th, typename Tw>
 int router_tiles(const void* h, const void* w, float* out, int T, int E, int K, cudaStream_t stream) {
-    const long large = (long)((T + 7) / 8) * ((E + 3) / 4), small = (long)T * E;
-    if (large >= 4 * PLM_SM_COUNT)                  // a warp for every scheduler
-        return plm_status_of(launch_pdl(router_tile_kernel<Th, Tw, 8, 4, 2>, dim3((unsigned)((large + RT_WARPS - 1) / RT_WARPS)), dim3(RT_WARPS * 32), 0,
-                                        stream, (const Th*)h, (const Tw*)w, out, T, E, K));
-    return plm_status_of(launch_pdl(router_tile_kernel<Th, Tw, 1, 1, 16>, dim3((unsigned)((small + RT_WARPS - 1) / RT_WARPS)), dim3(RT_WARPS * 32), 0,
-                                    stream, (const Th*)h, (const Tw*)w, out, T, E, K));
+    constexpr bool SHORT = sizeof(Th) + sizeof(Tw) == 4;                 // both in 16 bits
+    const long pairs = (long)T * E;
+    if (pairs <= 2048) return router_tile<Th, Tw, 1, 1, 16>(h, w, out, T, E, K, stream);
+    if (pairs <= 24576) return router_tile<Th, Tw, 2, 2, 8>(h, w, out, T, E, K, stream);
+    if (pairs > (SHORT ? 131072 : 262144)) return router_tile<Th, Tw, 8, 4, 2>(h, w, out, T, E, K, stream);
+    return router_tile<Th, Tw, 4, 4, SHORT ? 4 : 2>(h, w, out, T, E, K, stream);
 }
 
 }  // namespace

@@ -207,3 +207,19 @@ def test_retention_keeps_what_is_not_finite_where_it_belongs(H):
         assert not torch.isfinite(state.view(2, H, N, P)[t // 300, c // P, :, c % P]).all()
     rest = [c for c in range(H * P) if c not in (5, 140, 3, 200)]
     assert torch.equal(y[:, rest], clean[:, rest])
+
+
+@pytest.mark.parametrize("types_", [(torch.bfloat16, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("T,E,K", [(64, 32, 132), (2049, 1, 2052), (683, 3, 2052), (1024, 24, 260), (1025, 24, 260), (2731, 48, 388), (10923, 12, 128), (10923, 24, 132), (10925, 25, 4)])
+def test_router_logits_have_the_same_bits_in_every_tile(T, E, K, types_):
+    """Pairs on both sides of each line between tiles, tokens and rows that fill no tile, K with and without whole groups of steps."""
+    from picolm_b200 import ops
+    torch.manual_seed(T + E + K)
+    h, w = torch.randn(T, K).to(types_[0]).to(DEV), torch.randn(E, K).to(types_[1]).to(DEV)
+    odd = torch.empty(T * K + 1, dtype=types_[0], device=DEV)[1:].view(T, K).copy_(h)      # rows on no boundary: the general form
+    got = ops.router_logits(h, w)
+    assert torch.equal(got, ops.router_logits(odd, w))
+    ref = h.double() @ w.double().t()
+    # a lane's K / 32 terms one after the other, then five additions: each rounds a sum of at most `size`
+    size = h.double().abs() @ w.double().abs().t()
+    assert ((got.double() - ref).abs() <= (K / 32 + 9) * 2.0 ** -24 * size).all()
