@@ -417,8 +417,13 @@ struct PageMaps {               // the TMA form: the caches as [pages * G * 64 r
     CUtensorMap k, v;
 };
 
+// CTAs an SM that the kernel's registers leave room for, as many as its tiles in shared memory allow.  Left unsaid, the compiler kept to
+// fewer registers than that (80 for 118 at head size 64) and so to less in flight.  us a call before / now, 32 heads over 8 and without
+// a rotation: head size 64, 64 sequences to 4,096 66.3 / 63.7, one of 4,096 8.8 / 8.2, 256 of 700 41.7 / 40.5; 128, 8 of 2,048 12.9 / 12.4,
+// 64 to 4,096 113.4 / 112.7; 96, 32 of 2,000 41.6 / 40.4; 256, 16 heads over 4, 32 of 2,000 37.9 / 36.5.  At head size 32 nothing changes.
+template <bool ROPE> constexpr int dc_ctas() { return HD <= 32 ? (ROPE ? 6 : 8) : HD <= 64 ? 4 : HD <= 128 ? 2 : 1; }
 template <bool CLUSTER, bool ROPE, bool TMA, bool EXTRA>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, dc_ctas<ROPE>())
 attn_decode_kernel(const bf16* q, const bf16* kc, const bf16* vc,
                    bf16* __restrict__ out, float* __restrict__ ws_o, float* __restrict__ ws_ml,
                    const int* tok_pos, const int* tok_seq, const int* block_table,
