@@ -223,3 +223,25 @@ def test_router_logits_have_the_same_bits_in_every_tile(T, E, K, types_):
     # a lane's K / 32 terms one after the other, then five additions: each rounds a sum of at most `size`
     size = h.double().abs() @ w.double().abs().t()
     assert ((got.double() - ref).abs() <= (K / 32 + 9) * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("scores", ["sigmoid", "softmax", "logits"])
+@pytest.mark.parametrize("E,top", [(5, 5), (33, 1), (64, 32), (70, 33), (130, 70)])
+def test_choices_among_equal_scores(E, top, scores):
+    """Many ties and scores of both zeros' signs and of minus infinity: the lowest expert first, weights in the choices' order."""
+    from picolm_b200 import ops
+    T = 9
+    torch.manual_seed(E + top)
+    z = torch.randint(-6, 7, (T, E)).float() / 4
+    if scores == "logits":
+        z[z == 0] = -0.0
+        z[1, ::2] = 0.0
+        z[2, 1:E - top + 1 if top < E else 1] = -math.inf
+    ids, weights, _ = ops.route_topk(z.to(DEV), E, top, scores=scores)
+    order = torch.sort(z.double(), dim=1, descending=True, stable=True).indices[:, :top]
+    assert torch.equal(ids.cpu().long(), order)
+    chosen = z.double().gather(1, order)
+    s = torch.sigmoid(chosen) if scores == "sigmoid" else torch.softmax(z.double(), 1).gather(1, order) if scores == "softmax" else torch.softmax(chosen, 1)
+    want = s / s.sum(1, keepdim=True)
+    # an exponential within 2 units, a sum of E or `top` terms, three more roundings
+    assert ((weights.cpu().double() - want).abs() <= (E + top + 16) * 2.0 ** -24 * want).all()
