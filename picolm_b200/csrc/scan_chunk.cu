@@ -817,6 +817,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
     // D fp32, A and B bf16, B with N contiguous
     constexpr uint32_t IDESC = plm_tc::instr_desc_bf16(NB) | (1u << 16);
     static_assert(R % 2 == 0 && STEPS % 2 == 0, "a splitting warp must not take a phase for the one after the next");
+    static_assert(!OUT || STEPS >= 4, "a mark would stand where the unit before the last has not cleared its own");
     extern __shared__ unsigned char tc_raw[];
     __shared__ uint64_t bars[2 * R + 4];
     __shared__ uint32_t tmem_at;
@@ -946,6 +947,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                 ok = ok && plm_tc::mbar_wait(raw_full(b), (now / R) & 1, a.status, 46);
                 const float* raw_p = reinterpret_cast<const float*>(smem + b * T::RAW) + member * 32 + lane;
                 const float* raw_n = reinterpret_cast<const float*>(smem + b * T::RAW + T::RAW_P);
+                int from = NOWHERE;
                 uint32_t w[2][3][8];                             // (before the MMAs that read the buffers last are waited for)
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
@@ -963,9 +965,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                             for (int i = 0; i < 16; ++i)
                                 if (!(fabsf(v[i]) < INFINITY)) {
                                     v[i] = 0.f;
-                                    const int from = s < NP / TC_STEP ? 0 : (s - NP / TC_STEP) * TC_STEP + half * 16 + i;
-                                    atomicMin(&reached_from[turn][0][member * 32 + lane], from);
-                                    atomicMin(&reached_from[turn][1][member * 32 + lane], from);
+                                    from = min(from, s < NP / TC_STEP ? 0 : (s - NP / TC_STEP) * TC_STEP + half * 16 + i);
                                 }
                     }
 #pragma unroll
@@ -974,6 +974,12 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                         for (int i = 0; i < 8; ++i) w[half][t][i] = plm_split::next_terms(v[2 * i], v[2 * i + 1]);
                 }
                 if (now >= 2) ok = ok && plm_tc::mbar_wait(mma_done(group), ((now - 2) >> 1) & 1, a.status, 46);
+                // (a mark's place is that of the unit before the last, whose marks must be read and cleared: behind this wait the
+                // sums of step now - 4 are read, which is of the last unit where a unit has four steps)
+                if (OUT && from != NOWHERE) {
+                    atomicMin(&reached_from[turn][0][member * 32 + lane], from);
+                    atomicMin(&reached_from[turn][1][member * 32 + lane], from);
+                }
                 __syncwarp();
                 plm_tc::tc_fence_after();
 #pragma unroll

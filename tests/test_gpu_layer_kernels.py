@@ -140,6 +140,36 @@ def test_chunk_products_keep_what_is_not_finite_where_it_belongs():
     assert torch.equal(got[:, keep], clean[:, keep])
 
 
+@pytest.mark.parametrize("N", [40, 64, 128])
+def test_units_of_one_cta_keep_their_own_marks(N):
+    """More than three units a CTA, and values that are not finite in units that one CTA takes one after the other, in a state and
+    in the values: each reaches its own column's later results, whichever unit comes before or behind it."""
+    from picolm_b200 import ops
+    torch.manual_seed(N)
+    H, P, lens = 8, 128, [64 * 37, 64 * 37 - 5]                  # 592 units: 148 CTAs take four each
+    T, step = sum(lens), _step(lens)
+    q, k, v, raw = (torch.randn(T, H * c, device=DEV) * 0.1 for c in (N, N, P, N))
+    bias, state = torch.zeros(H * N, device=DEV), torch.randn(2, H * N * P, device=DEV)
+    run = lambda x, s: ops.linear_scan(q, k, x, raw, ops.DECAY_SIGMOID, bias, None, None, 1.0, 1.0 / 16.0, s, step, H, N, P)
+    clean = run(v, state.clone())
+    bad, old = v.clone(), state.clone()
+    # a column of every head: from the state on, from a token of every third chunk on (the column is of no number from the first
+    # on, so each chunk has one of its own)
+    marks = [(t, (c % H) * P + 3 * c + 1) for c, t in enumerate(range(7, T, 64 * 3)) if t < T]
+    for i, (t, c) in enumerate(marks):
+        bad[t, c] = (math.inf, -math.inf, math.nan)[i % 3]
+    old.view(2, H, N, P)[1, 2, 5, 127] = math.nan
+    ends = lambda t: lens[0] if t < lens[0] else T
+    for _ in range(3):
+        got = run(bad, old.clone())
+        rest = torch.ones(T, H * P, dtype=torch.bool, device=DEV)
+        for t, c in marks + [(lens[0], 2 * P + 127)]:
+            assert not torch.isfinite(got[t:ends(t), c]).any(), (t, c)
+            rest[t:ends(t), c] = False
+        assert torch.equal(got[rest], clean[rest])
+    ops.check_status(DEV)
+
+
 def _retention(N, P, lens, H=3, positions=0, odd=None):
     """ops.decay_scan over rotated rows, its inputs, and the same in float64 with everything that the kernels are handed."""
     from picolm_b200 import ops
