@@ -1,7 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T in float32 on the tensor cores, with the error of float32 sums.
 //
-// Every float is the sum of three bfloat16 terms, exactly: h = bf16(x), m = bf16(x - h), l = x - h - m (24 bits of mantissa in
-// three times 8, each remainder exact in fp32).  A product of two terms has 16 bits and is exact in the tensor cores, so six
+// Every float (times 2^24, see TERM_SCALE) is the sum of three bfloat16 terms, exactly: h = bf16(x), m = bf16(x - h), l = x - h - m
+// (24 bits of mantissa in three times 8, each remainder exact in fp32; a known way to split, as in S. Markidis et al., "NVIDIA
+// Tensor Core Programmability, Performance & Precision", 2018).  A product of two terms has 16 bits and is exact in the tensor cores, so six
 // products (hh, hm, mh, hl, lh, mm) leave out less than 2^-25 of a term: what remains is the rounding of the accumulator.
 // Each PIECE terms of K are accumulated from zero, the small products first, and the piece's sum is added to a double.
 //
@@ -10,7 +11,8 @@
 // on how many rows stand beside it, though tiles have 16 to 128 rows of A and the segments of a tile may be dealt out to the
 // CTAs of a cluster.
 //
-// What is not finite: an infinity's remainder is no number, so a result that is not finite (also after an overflow) is
+// What is not finite: an infinity's remainder is no number, so a result that is not finite (also after an overflow, which
+// operands from 2^104 and sums from 2^80 on meet) is
 // taken again from the rows themselves, by fused multiply-adds as gemm_simt.cu does.
 //
 // The error against 64 bits (2-norm, normal numbers; 1 to 1,300 rows, K of 100 to 14,336): 1.26 x 2^-24 of the result, the CUDA
@@ -212,6 +214,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (int i = 0; i < 4; ++i)
                         *reinterpret_cast<float4*>(x + 4 * i) = *reinterpret_cast<const float4*>(raw + (member * 32 + lane) * 128 + ((4 * h + i) ^ (lane % 8)) * 16);
 #pragma unroll
+                    for (int i = 0; i < 16; ++i) x[i] *= TERM_SCALE;
+#pragma unroll
                     for (int t = 0; t < 3; ++t)
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[h][t][i] = next_terms(x[2 * i], x[2 * i + 1]);
@@ -230,6 +234,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     float x[8];
                     *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(raw + block * 1024 + ((2 * q) ^ a_row) * 16);
                     *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(raw + block * 1024 + ((2 * q + 1) ^ a_row) * 16);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) x[i] *= TERM_SCALE;
 #pragma unroll
                     for (int t = 0; t < 3; ++t) {
                         uint4 v;
@@ -365,7 +371,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             for (int j = 0; j < (CS > 1 ? 1 : 4); ++j) {
                 double wide = CS > 1 ? total[CS > 1 ? c : 0] : sum_of(c + j);
                 if (CS == 1 && n_segments > 1) wide = __hiloint2double((int)r[2 * j + 1], (int)r[2 * j]) + wide;
-                const float v = (float)wide;
+                const float v = (float)wide * SUM_SCALE;
                 if (n < g.N && c + j < count) {
                     finite = finite && fabsf(v) <= 3.402823466e38f;
                     to[(c + j) * ld] = v;

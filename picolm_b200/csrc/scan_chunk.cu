@@ -969,6 +969,8 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                                 }
                     }
 #pragma unroll
+                    for (int i = 0; i < 16; ++i) v[i] *= plm_split::TERM_SCALE;
+#pragma unroll
                     for (int t = 0; t < 3; ++t)
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[half][t][i] = plm_split::next_terms(v[2 * i], v[2 * i + 1]);
@@ -992,6 +994,8 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     float v[8];
                     *reinterpret_cast<float4*>(v) = ld4(raw_n + k * NB + c8 * 8);
                     *reinterpret_cast<float4*>(v + 4) = ld4(raw_n + k * NB + c8 * 8 + 4);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] *= plm_split::TERM_SCALE;
                     unsigned char* to = n_to + c8 / 8 * T::BLOCK + k * 128 + ((c8 % 8) ^ (k & 7)) * 16;
 #pragma unroll
                     for (int t = 0; t < 3; ++t) {
@@ -1072,7 +1076,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     if (!OUT && j >= rows) sum[j] = 0.f;         // (padding stays zero, whatever U holds)
                     if (!OUT || j < rows) {
                         finite = finite && fabsf(sum[j]) < INFINITY;
-                        to[j * ld] = sum[j];
+                        to[j * ld] = sum[j] * plm_split::SUM_SCALE;
                     }
                 }
                 if (!finite || from != NOWHERE)

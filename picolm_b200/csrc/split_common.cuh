@@ -40,6 +40,12 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b_desc, 
         ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(more) : "memory");
 }
 
+// What a float is multiplied by before it is split, and what a sum of products of two such is multiplied by.  bfloat16 has no bits
+// below 2^-133, so the third term of a float below 2^-109 would be cut off, and more of it the smaller it is; 2^24 times as
+// large all 24 bits of every float stand at 2^-125 and above, subnormal ones included.  What that sends beyond the largest
+// float (operands from 2^104 on, sums from 2^80 on) becomes no number and is taken again with the other results of that kind.
+constexpr float TERM_SCALE = 0x1p24f, SUM_SCALE = 0x1p-48f;
+
 // two floats as pairs of bf16 terms; a and b become the remainders
 __device__ __forceinline__ uint32_t next_terms(float& a, float& b) {
     const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);

@@ -79,6 +79,26 @@ def test_float32_tc_values_that_are_not_finite(form):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("small,large", [(1e-36, 1e30), (1e-39, 1e30), (2e-44, 1e37), (1e-33, 1e-6), (1e-20, 1e-21), (1e-3, 1e26), (1e-5, 1e33)])
+def test_float32_tc_of_the_smallest_and_largest_operands(small, large):
+    """Operands next to and below the smallest normal number, whose last bits bfloat16 has no place for, and large ones: as exact
+    as any others.  Rows of ordinary numbers beside them stay as they are."""
+    from picolm_b200 import ops
+    torch.manual_seed(8)
+    M, N, K = 40, 140, 300
+    a, w = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV)
+    plain = ops.gemm_f32_tc(a, w)
+    a[::2] *= small
+    w[::2] *= large
+    got, ref, mag = ops.gemm_f32_tc(a, w), a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # (16 fused multiply-adds one after the other where the sums are taken again; a result may be subnormal)
+    assert ((got.double() - ref).abs() <= 16 * 2.0 ** -24 * mag + 2.0 ** -149).all()
+    assert (got.double() - ref)[::2, ::2].norm() <= 2 * 2.0 ** -24 * ref[::2, ::2].norm() + 2.0 ** -149 * (M * N) ** 0.5
+    assert torch.equal(got[1::2, 1::2], plain[1::2, 1::2])
+    assert int(ops.status_word(DEV).item()) == 0
+
+
+@pytest.mark.gpu
 def test_linear_of_float32_rows_off_their_boundaries_takes_the_cuda_cores():
     from picolm_b200 import ops
     torch.manual_seed(6)

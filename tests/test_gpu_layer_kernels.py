@@ -170,6 +170,25 @@ def test_units_of_one_cta_keep_their_own_marks(N):
     ops.check_status(DEV)
 
 
+@pytest.mark.parametrize("small,large", [(1e-36, 1e30), (1e-41, 1e34), (1e-12, 1e33)])
+def test_chunk_products_of_the_smallest_and_largest_values(small, large):
+    """Values whose last bits bfloat16 has no place for against large queries."""
+    from picolm_b200 import ops
+    torch.manual_seed(4)
+    H, N, P, T = 3, 64, 128, 190
+    step = _step([T])
+    q, k, v, raw = (torch.randn(T, H * c, device=DEV) for c in (N, N, P, N))
+    q, k, v, bias = q * large, k * N ** -0.5, v * small, torch.zeros(H * N, device=DEV)
+    state = torch.zeros(1, H * N * P, device=DEV)
+    got = ops.linear_scan(q, k, v, raw, ops.DECAY_SIGMOID, bias, None, None, 1.0, 1.0 / 16.0, state, step, H, N, P)
+    view = lambda x, c: x.double().view(T, H, c)
+    want, S = _scan(view(q, N), view(k, N), view(v, P), view(torch.nn.functional.logsigmoid(raw.double()) / 16.0, N))
+    # (as for ordinary numbers; a value of the state may be subnormal)
+    assert (state.double() - S.reshape(-1)).abs().max() <= 2e-6 * S.abs().max() + 4 * 2.0 ** -149
+    if small > 1e-38:
+        assert (got.double() - want.reshape(T, -1)).norm() <= 2e-6 * want.norm()
+
+
 def _retention(N, P, lens, H=3, positions=0, odd=None):
     """ops.decay_scan over rotated rows, its inputs, and the same in float64 with everything that the kernels are handed."""
     from picolm_b200 import ops
