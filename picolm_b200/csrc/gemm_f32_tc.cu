@@ -152,21 +152,22 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     auto stages_of = [&](int round) { return CS > 1 ? max(0, min(SEGMENT_STAGES, n_stages_all - first_of(round))) : n_stages_all; };
     bool ok = true;
     int done = 0;                                              // stages of the rounds before
+    // (a warp whose wait runs out arrives nowhere any more, so that those behind it give up as well, and each meets its cluster's
+    // barriers all the same)
     if (warp >= LOADER) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REST_REGS));
+        int asked = 0;                                         // stages that the loader has asked for
         for (int round = 0; round < n_rounds; ++round) {
             const int first = first_of(round), n_stages = stages_of(round);
             if (warp == LOADER && lane == 0) {
-                for (int s = 0; s < n_stages && ok; ++s) {
-                    const int at = done + s, b = at % R;
+                for (int s = 0; s < n_stages && ok; ++s, ++asked) {
+                    const int at = asked, b = at % R;
                     if (at >= R) ok = mbar_wait(raw_empty(b), ((at - R) / R) & 1, g.status, 60);
                     if (!ok) break;
-                    mbar_expect_tx(raw_full(b), T::RAW);
+                    mbar_expect_tx(raw_full(b), T::RAW + PLM_STALL_BYTES);
                     tma_load_2d(smem_u32(smem + b * T::RAW), &map_w, raw_full(b), (first + s) * STAGE, n0);
                     tma_load_2d(smem_u32(smem + b * T::RAW + ROWS * STAGE * 4), &map_a, raw_full(b), (first + s) * STAGE, m0);
                 }
-                if (!ok)                                       // a wait ran out: no copy may be under way when the CTA ends
-                    for (int b = 0; b < R; ++b) mbar_wait(raw_full(b), 0, g.status, 60);
             } else if (warp == ISSUER || warp == ISSUER + 1) {
                 // two warps, so that one's waits pass while the other's MMAs run; the smallest products first
                 const int b = warp - ISSUER;
@@ -195,6 +196,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 cluster_sync_all();
             }
         }
+        if (warp == LOADER && lane == 0)                       // no copy may be under way when the CTA ends, whoever gave up
+            for (int i = max(0, asked - R); i < asked; ++i) mbar_wait(raw_full(i % R), (i / R) & 1, nullptr, 0);
+        __syncwarp();
     } else if (warp >= FOLDERS) {
         // split: of W a lane a row, of A eight terms of a row at a time
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SPLIT_REGS));
@@ -202,9 +206,10 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const uint32_t w_to = tmem + ((uint32_t)(member * 32) << 16) + T::TERMS_W;
         for (int round = 0; round < n_rounds; ++round) {
             const int n_stages = stages_of(round);
-            for (int s = (group + GROUPS - done % GROUPS) % GROUPS; s < n_stages; s += GROUPS) {
+            for (int s = (group + GROUPS - done % GROUPS) % GROUPS; s < n_stages && ok; s += GROUPS) {
                 const int at = done + s, b = at % R;
-                ok = ok && mbar_wait(raw_full(b), (at / R) & 1, g.status, 62);
+                ok = mbar_wait_warp(raw_full(b), (at / R) & 1, g.status, 62);
+                if (!ok) break;
                 const unsigned char* raw = smem + b * T::RAW;
                 uint32_t w[2][3][8];                           // (before the MMAs that read the buffers last are waited for)
 #pragma unroll
@@ -220,8 +225,8 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[h][t][i] = next_terms(x[2 * i], x[2 * i + 1]);
                 }
-                if (at >= 2) ok = ok && mbar_wait(mma_done(at & 1), ((at - 2) >> 1) & 1, g.status, 62);
-                __syncwarp();
+                if (at >= 2) ok = mbar_wait_warp(mma_done(at & 1), ((at - 2) >> 1) & 1, g.status, 62);
+                if (!ok) break;
                 tc_fence_after();
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
@@ -282,10 +287,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         __syncwarp();
         for (int round = 0; round < n_rounds; ++round) {
             const int n_stages = stages_of(round);
-            for (int s = 0; s < n_stages; ++s) {
+            for (int s = 0; s < n_stages && ok; ++s) {
                 const int at = done + s, b = at & 1;
-                ok = ok && mbar_wait(mma_done(b), (at >> 1) & 1, g.status, 63);
-                __syncwarp();
+                ok = mbar_wait_warp(mma_done(b), (at >> 1) & 1, g.status, 63);
+                if (PLM_GIVES_UP(warp, at)) {
+                    atomicCAS(g.status, 0, 63);
+                    ok = false;
+                }
+                if (!ok) break;
                 tc_fence_after();
                 auto take = [&](auto& r, int c) {
                     constexpr int n = sizeof(r) / 4;
@@ -356,7 +365,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         const int n = n0 + warp % 4 * 32 + lane;
         const uint32_t sums = lanes + T::SUMS + 2 * half;
         constexpr int STEP = CS > 1 ? CS : 1;                  // from one of this thread's columns to the next
-        const int first = m0 + half + (CS > 1 ? rank : 0), count = min(COLS / STEP, (g.M - first + STEP - 1) / STEP);
+        const int first = m0 + half + (CS > 1 ? rank : 0), count = ok ? min(COLS / STEP, (g.M - first + STEP - 1) / STEP) : 0;
         float* to = g.C + (size_t)first * g.ldc + n;
         const size_t ld = (size_t)STEP * g.ldc;
         bool finite = true;

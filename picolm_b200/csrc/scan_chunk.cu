@@ -893,7 +893,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                                               : x.w + Lay::KE + (long)s * TC_STEP * NP;
                     const uint32_t to = plm_tc::smem_u32(smem + b * T::RAW);
                     if (plm_tc::elect_one()) {
-                        plm_tc::mbar_expect_tx(raw_full(b), T::RAW);
+                        plm_tc::mbar_expect_tx(raw_full(b), T::RAW + PLM_STALL_BYTES);
                         asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                                      ::"r"(to), "l"((uint64_t)(first ? &map_s : &map_u)), "r"(raw_full(b)), "r"(x.p0),
                                        "r"((OUT && !first ? j : s) * TC_STEP), "r"(x.block) : "memory");
@@ -902,10 +902,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     }
                     __syncwarp();
                 }
-                if (!ok) {                                       // a wait ran out: no copy may be under way when the CTA ends
-                    for (int i = max(0, at - R); i < at; ++i) plm_tc::mbar_wait(raw_full(i % R), (i / R) & 1, nullptr, 0);
-                    break;
-                }
+                if (!ok) break;
             } else if (warp == TC_ISSUER || warp == TC_ISSUER + 1) {         // every other step each, the smallest products first
                 const int b = warp - TC_ISSUER;
                 const uint32_t p = tmem + T::TERMS_P + b * 48, d = tmem + b * NB;
@@ -932,6 +929,8 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                 if (!ok) break;
             }
         }
+        if (warp == TC_LOADER)                                   // no copy may be under way when the CTA ends, whoever gave up
+            for (int i = max(0, at - R); i < at; ++i) plm_tc::mbar_wait(raw_full(i % R), (i / R) & 1, nullptr, 0);
         __syncwarp();
     } else if (warp >= TC_FOLDERS) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
@@ -944,7 +943,8 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
             if (!some) continue;
             for (int s = group; s < STEPS; s += 2) {             // (a unit has an even number of steps)
                 const int now = at + s, b = now % R;
-                ok = ok && plm_tc::mbar_wait(raw_full(b), (now / R) & 1, a.status, 46);
+                ok = plm_tc::mbar_wait_warp(raw_full(b), (now / R) & 1, a.status, 46);
+                if (!ok) break;                                  // (a warp whose wait runs out arrives nowhere any more)
                 const float* raw_p = reinterpret_cast<const float*>(smem + b * T::RAW) + member * 32 + lane;
                 const float* raw_n = reinterpret_cast<const float*>(smem + b * T::RAW + T::RAW_P);
                 int from = NOWHERE;
@@ -975,7 +975,8 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
 #pragma unroll
                         for (int i = 0; i < 8; ++i) w[half][t][i] = plm_split::next_terms(v[2 * i], v[2 * i + 1]);
                 }
-                if (now >= 2) ok = ok && plm_tc::mbar_wait(mma_done(group), ((now - 2) >> 1) & 1, a.status, 46);
+                if (now >= 2) ok = plm_tc::mbar_wait_warp(mma_done(group), ((now - 2) >> 1) & 1, a.status, 46);
+                if (!ok) break;
                 // (a mark's place is that of the unit before the last, whose marks must be read and cleared: behind this wait the
                 // sums of step now - 4 are read, which is of the last unit where a unit has four steps)
                 if (OUT && from != NOWHERE) {
@@ -1016,7 +1017,6 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     plm_split::mbar_arrive(raw_empty(b));
                 }
             }
-            ok = __all_sync(0xffffffffu, ok);
             at += STEPS;
             turn ^= 1;
         }
@@ -1039,8 +1039,12 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
 #pragma unroll 1
             for (int s = 0; s < STEPS; ++s, ++at) {
                 const int b = at & 1;
-                ok = ok && plm_tc::mbar_wait(mma_done(b), (at >> 1) & 1, a.status, 47);
-                __syncwarp();
+                ok = plm_tc::mbar_wait_warp(mma_done(b), (at >> 1) & 1, a.status, 47);
+                if (PLM_GIVES_UP(warp, at)) {
+                    atomicCAS(a.status, 0, 47);
+                    ok = false;
+                }
+                if (!ok) break;
                 plm_tc::tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < COLS; c += 32) {
@@ -1056,6 +1060,7 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                     for (int j = 0; j < 32; ++j) sum[c + j] += __uint_as_float(r[j]);
                 }
             }
+            if (!ok) break;
             // (the stores first and what is not finite behind them: a look at each sum on its way out took 7,000 cycles a unit, more
             // than its six steps)
             const int p = x.p0 + warp % 4 * 32 + lane;
@@ -1085,7 +1090,6 @@ chunk_product_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_con
                         if (c0 + j >= from || !(fabsf(to[j * ld]) < INFINITY)) to[j * ld] = sum_again<NP, OUT>(x.w, PP, p, c0 + j);
             }
             __syncwarp();
-            ok = __all_sync(0xffffffffu, ok);
         }
         plm_tc::tc_fence_before();
     }

@@ -6,6 +6,19 @@
 namespace plm_split {
 using namespace plm_tc;
 
+// A test build only (-DPLM_TEST_GIVE_UP, never the library that serves): while the switch is 1, the loader announces 64 bytes
+// more for every stage than it loads, so that every wait runs out; while it is 2, one of the warps that add sums up acts as if
+// its wait for the CTA's sixth stage had run out.  The kernel must record it, let what it has in flight land, free its tensor
+// memory and return.
+#ifdef PLM_TEST_GIVE_UP
+__device__ int give_up_switch = 0;
+#define PLM_STALL_BYTES (plm_split::give_up_switch == 1 ? 64u : 0u)
+#define PLM_GIVES_UP(warp, stage) (plm_split::give_up_switch == 2 && (warp) == 3 && (stage) == 5)
+#else
+#define PLM_STALL_BYTES 0u
+#define PLM_GIVES_UP(warp, stage) false
+#endif
+
 template <int NC> __device__ __forceinline__ void tmem_load(uint32_t addr, uint32_t (&r)[NC]) {
     static_assert(NC == 8 || NC == 16 || NC == 32, "columns");
     if constexpr (NC == 32) tc_ld32(addr, r);
@@ -56,3 +69,9 @@ __device__ __forceinline__ uint32_t next_terms(float& a, float& b) {
 }
 
 }  // namespace plm_split
+
+#ifdef PLM_TEST_GIVE_UP
+extern "C" int plm_test_give_up(int how, cudaStream_t stream) {
+    return plm_status_of(cudaMemcpyToSymbolAsync(plm_split::give_up_switch, &how, sizeof(int), 0, cudaMemcpyHostToDevice, stream));
+}
+#endif

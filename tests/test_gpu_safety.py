@@ -96,6 +96,73 @@ def test_the_experts_product_gives_up_as_one(epilogue, how):
     assert torch.allclose(out[used].double(), z, atol=2e-3 if epilogue == 0 else 2e-2, rtol=1e-4 if epilogue == 0 else 1.2e-2)
 
 
+@pytest.mark.parametrize("form", [16 + 8000, 32 + 2000, 64 + 1000, 96 + 1000])
+@pytest.mark.parametrize("how", [1, 2])
+def test_the_float32_product_gives_up(form, how):
+    """The same for the float32 product on the tensor cores, alone and in clusters, whose ring has been round more than once
+    when one of the warps that add sums up gives up (2)."""
+    from picolm_b200 import ops
+    from picolm_b200.csrc.build import load_library
+    from picolm_b200.ops import _lib
+    lib = load_library("gemm_f32_tc@give_up", ["-DPLM_WAIT_LIMIT=20000", "-DPLM_TEST_GIVE_UP"])
+    lib.plm_gemm_f32_tc.argtypes = _lib._SIGNATURES["plm_gemm_f32_tc"]
+    lib.plm_test_give_up.argtypes = [ctypes.c_int, ctypes.c_void_p]
+    stream = torch.cuda.current_stream().cuda_stream
+    M, N, K = 90, 300, 9000
+    torch.manual_seed(6)
+    a, w, out = torch.randn(M, K, device=DEV), torch.randn(N, K, device=DEV), torch.zeros(M, N, device=DEV)
+    status = ops.status_word(DEV)
+    ops.check_status(DEV)
+
+    def product():
+        return lib.plm_gemm_f32_tc(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, K, K, N, form, status.data_ptr(), stream)
+
+    assert lib.plm_test_give_up(how, stream) == 0
+    assert product() == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) in ((60, 61, 62, 63) if how == 1 else (63,))
+    with pytest.raises(ops.KernelError, match="gave up waiting"):
+        ops.check_status(DEV)
+    assert lib.plm_test_give_up(0, stream) == 0
+    assert product() == 0
+    torch.cuda.synchronize()
+    ops.check_status(DEV)
+    assert torch.equal(out, ops.gemm_f32_tc(a, w))
+
+
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("how", [1, 2])
+def test_the_chunk_products_give_up(N, how, monkeypatch):
+    """The same for the chunk products of a recurrence, with several units a CTA."""
+    import types
+    from picolm_b200 import ops
+    from picolm_b200.csrc.build import load_library
+    from picolm_b200.ops import _lib
+    H, P, T = 8, 128, 64 * 40
+    torch.manual_seed(7)
+    q, k, v, raw = (torch.randn(T, H * c, device=DEV) * 0.1 for c in (N, N, P, N))
+    bias = torch.zeros(H * N, device=DEV)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    step = types.SimpleNamespace(n_seqs=1, n_tokens=T, max_new=T, is_decode=False, seq_start=i32([0, T]), seq_slot=i32([0]), tok_seq=i32([0] * T))
+    run = lambda: ops.linear_scan(q, k, v, raw, ops.DECAY_SIGMOID, bias, None, None, 1.0, 1.0 / 16.0, torch.zeros(1, H * N * P, device=DEV), step, H, N, P)
+    ops.check_status(DEV)
+    want = run()
+    flags = ["-DPLM_WAIT_LIMIT=20000", "-DPLM_TEST_GIVE_UP"]
+    lib = load_library("scan_chunk@give_up", flags)
+    lib.plm_test_give_up.argtypes = [ctypes.c_int, ctypes.c_void_p]
+    stream = torch.cuda.current_stream().cuda_stream
+    monkeypatch.setitem(_lib.VARIANT_OF, "scan_chunk", ("scan_chunk@give_up", flags))
+    assert lib.plm_test_give_up(how, stream) == 0
+    run()
+    torch.cuda.synchronize()
+    assert int(ops.status_word(DEV).item()) in ((44, 45, 46, 47) if how == 1 else (47,))
+    with pytest.raises(ops.KernelError, match="gave up waiting"):
+        ops.check_status(DEV)
+    assert lib.plm_test_give_up(0, stream) == 0
+    assert torch.equal(run(), want)
+    ops.check_status(DEV)
+
+
 CHECKED_SCRIPT = r'''
 import os, sys, json
 sys.path.insert(0, sys.argv[1]); sys.path.insert(0, os.path.join(sys.argv[1], "tests"))
