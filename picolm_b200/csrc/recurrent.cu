@@ -117,17 +117,9 @@ __global__ void causal_conv_vec8_kernel(const bf16* u, long ldu, const float* w,
     *reinterpret_cast<uint4*>(out + (long)t * C + c) = *reinterpret_cast<const uint4*>(o);
 }
 
-// x sigmoid(x) where the result is rounded to bfloat16: the special-function unit's 2^x and reciprocal, whose errors (below
-// 2^-20) are far below that rounding.  The exact exponential and division were most of the kernel's instructions.
-__device__ __forceinline__ float silu_for_bf16(float x) {
-    float e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
-    return __fdividef(x, 1.f + e);
-}
-
 // The same for four taps, four tokens a thread: their seven rows of inputs are asked for at once and each is read once, where a
 // token a thread waited for its own chain of a sequence's number, its first token and four rows (2,048 tokens x 2,048 channels:
-// 14.5 -> 11.3 us without warm caches).  A sum has the order of the kernel above.
+// 14.5 -> 13.4 us without warm caches).  The same sums and activation as the kernel above, bit for bit.
 constexpr int CONV_TOKENS = 4;
 __global__ void __launch_bounds__(128)
 causal_conv_four_kernel(const bf16* u, long ldu, const float* w, const float* bias, const float* state, long state_stride,
@@ -179,7 +171,7 @@ causal_conv_four_kernel(const bf16* u, long ldu, const float* w, const float* bi
         }
         __nv_bfloat162 o[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) o[e] = __floats2bfloat162_rn(silu_for_bf16(acc[2 * e]), silu_for_bf16(acc[2 * e + 1]));
+        for (int e = 0; e < 4; ++e) o[e] = __floats2bfloat162_rn(silu_f(acc[2 * e]), silu_f(acc[2 * e + 1]));
         *reinterpret_cast<uint4*>(out + (long)(t0 + j) * C + c) = *reinterpret_cast<const uint4*>(o);
     }
 }

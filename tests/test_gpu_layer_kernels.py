@@ -45,12 +45,28 @@ def test_convolution_of_four_taps(lens, C):
     state = torch.randn(len(lens), 3 * C, device=DEV)
     back = [torch.cat([state[b].view(3, C).double(), u[s:s + n].double()]) for b, (s, n) in enumerate(zip([sum(lens[:b]) for b in range(len(lens))], lens))]
     raw = torch.cat([sum(x[j:j + n] * w[j].double() for j in range(4)) for x, n in zip(back, lens)])
+    before = state.clone()
     got = ops.causal_conv(u, w, None, state, step)
     want = torch.nn.functional.silu(raw)
-    # sums of four terms in fp32, the activation within 2^-20, one rounding to bfloat16
+    # sums of four terms in fp32 (the activation's slope is at most 1.1), the activation within 2^-20, one rounding to bfloat16
     mag = torch.cat([sum((x[j:j + n] * w[j].double()).abs() for j in range(4)) for x, n in zip(back, lens)])
-    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -19 * (mag + 1)).all()
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1.1 * 2.0 ** -22 * mag + 2.0 ** -130).all()
     assert torch.equal(state.double().view(len(lens), 3, C), torch.stack([x[-3:] for x in back]))
+    # a fifth tap of zero takes the kernel for any number of taps
+    w5, state5 = torch.cat([torch.zeros(1, C, device=DEV), w]), torch.cat([torch.zeros(len(lens), C, device=DEV), before], 1)
+    assert torch.equal(got, ops.causal_conv(u, w5, None, state5, step))
+
+
+def test_activations_of_the_convolution_far_from_zero():
+    """Inputs down to -88: a result is as exact as one rounding to bfloat16 lets it be, also where it is tiny."""
+    from picolm_b200 import ops
+    C, T = 64, 177
+    x = torch.linspace(-88, 88, T, dtype=torch.float64).to(torch.bfloat16)
+    w = torch.zeros(4, C, device=DEV)
+    w[3] = 1.0
+    got = ops.causal_conv(x[:, None].expand(T, C).contiguous().to(DEV), w, None, torch.zeros(1, 3 * C, device=DEV), _step([T]))
+    want = torch.nn.functional.silu(x.double()).to(DEV)[:, None]
+    assert ((got.double() - want).abs() <= (2.0 ** -8 + 2.0 ** -20) * want.abs()).all()
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
