@@ -1,26 +1,32 @@
-// C[M,N] = A[M,K] * W[N,K]^T in float32 on the tensor cores, with the error of float32 sums.
+// C[M,N] = A[M,K] * W[N,K]^T in float32 on the tensor cores.  Sums of terms of both signs are as exact as float32 ones on the CUDA
+// cores (gemm_simt.cu), sums of terms of one sign less so, see below.
 //
 // Every float (times 2^24, see TERM_SCALE) is the sum of three bfloat16 terms, exactly: h = bf16(x), m = bf16(x - h), l = x - h - m
 // (24 bits of mantissa in three times 8, each remainder exact in fp32; a known way to split, as in S. Markidis et al., "NVIDIA
 // Tensor Core Programmability, Performance & Precision", 2018).  A product of two terms has 16 bits and is exact in the tensor cores, so six
 // products (hh, hm, mh, hl, lh, mm) leave out less than 2^-25 of a term: what remains is the rounding of the accumulator.
-// Each PIECE terms of K are accumulated from zero, the small products first, and the piece's sum is added to a double.
+// Each STAGE of 32 terms of K is accumulated from zero, the small products first: a piece.  SETTLE pieces are added up in fp32, and
+// their sum joins the two floats (head and rest) that hold the sum so far.
 //
-// The order of a result's sums is fixed by K alone: pieces of PIECE terms in ascending order make a segment of SEGMENT
-// terms, the segments' doubles are added in ascending order, and the sum is rounded once.  So a row's result does not depend
-// on how many rows stand beside it, though tiles have 16 to 128 rows of A and the segments of a tile may be dealt out to the
+// The order of a result's sums is fixed by K alone: pieces of 32 terms in ascending order make a segment of SEGMENT
+// terms, the segments' sums are added as doubles in ascending order, and the sum is rounded once.  So a row's result does not depend
+// on how many rows stand beside it, though tiles have 16 to 96 rows of A and the segments of a tile may be dealt out to the
 // CTAs of a cluster.
 //
 // What is not finite: an infinity's remainder is no number, so a result that is not finite (also after an overflow, which
 // operands from 2^104 and sums from 2^80 on meet) is
 // taken again from the rows themselves, by fused multiply-adds as gemm_simt.cu does.
 //
-// The error against 64 bits (2-norm, normal numbers; 1 to 1,300 rows, K of 100 to 14,336): 1.26 x 2^-24 of the result, the CUDA
-// cores' 1.31.  Pieces of 64 terms in one accumulator: 5.3 (each MMA truncates its sum, so what counts is how many see a
-// whole-sized one); pieces of 32 added to the sum without SETTLE: 1.05, but a double's addition is slow here (2,000 cycles a
-// stage for 128 x 128 results).
-// 462 rows x 16,384 x 2,048: 893 -> 232 us (134 TFLOP/s of float32 products); x 2,048 x 8,192: 662 -> 135; 24 rows x 3,072 x
-// 2,048: 42.7 -> 19.5; 8 rows x 2,048 x 8,192: 71 -> 33.
+// The error against 64 bits, in 2^-24 of the result (2-norm; K of 128 to 14,336), here and on the CUDA cores: rows of normal numbers
+// times normal weights 1.18 to 1.22 and 1.31, rows silu(x) y of a gated feed-forward 1.26 to 1.28 and 1.28 to 1.31, both of a wide range
+// (x^5, signed) 1.40 to 1.43 and 1.23 to 1.42.  An MMA cuts its addends off a few bits below the largest and truncates its
+// sum, so terms of one sign come out low by 0.86: positive normal or uniform numbers 0.97 to 1.10 and 0.46 to 0.59; positive ones
+// over several decades (e^(2x)), where one term of 16 outweighs the others, 2.5 to 5.5 and 0.6 to 1.5.  A model's weights have both signs.
+// The longer the sums in fp32, the larger the error: pieces of 64 terms in one accumulator 5.3; of normal numbers and of silu(x) y SETTLE = 1
+// 1.11 and 1.18, 2 1.17 and 1.24, 4 1.27 and 1.33, at 328, 250 and 226 us for 462 x 16,384 x 2,048 and 236 with 3.  A double's addition
+// a piece: 1.05, but slow here (2,000 cycles a stage for 128 x 128 results).
+// The CUDA cores against this: 462 rows x 16,384 x 2,048 893 and 236 us (131 TFLOP/s of float32 products); x 2,048 x 8,192 662 and 137;
+// 24 rows x 3,072 x 2,048 42.7 and 17.3; 8 rows x 2,048 x 8,192 71 and 33.
 // Bound by the MMAs (106 cycles each at 96 columns, 79 at 64, 58 at 16) and the hand-overs between the warps.  Everything done by
 // the same eight warps, with W's terms in shared memory too: 490 us for 462 x 2,048 x 8,192; splitting and adding apart 275;
 // W's terms in tensor memory 237; two issuing warps behind elect.sync 190; four splitting warps a stage in turns 171.
@@ -36,7 +42,7 @@ namespace {
 constexpr int FOLDERS = 8, GROUPS = 2, LOADER = FOLDERS + 4 * GROUPS, ISSUER = LOADER + 1, THREADS = 32 * (LOADER + 4);
 constexpr int LAUNCH_REGS = 96, FOLD_REGS = 144, SPLIT_REGS = 80, REST_REGS = 32;
 static_assert(32 * (FOLDERS * FOLD_REGS + 4 * GROUPS * SPLIT_REGS + 4 * REST_REGS) <= THREADS * LAUNCH_REGS && THREADS * LAUNCH_REGS <= 65536, "registers");
-constexpr int SETTLE = 4;                                      // pieces that are summed in fp32 before their sum joins the head
+constexpr int SETTLE = 3;                                      // pieces that are summed in fp32 before their sum joins the head
 constexpr int STAGE = 32, SEGMENT = 1024, SEGMENT_STAGES = SEGMENT / STAGE;    // a stage is a piece of 32 terms of K
 constexpr int ROWS = 128;                                      // rows of W a tile (the MMA's M)
 

@@ -40,12 +40,37 @@ def test_float32_tc_forms(M, N, K):
     assert torch.equal(ops.gemm_f32_tc(wide[:, 4:4 + K], w), out)
     ref, mag = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
     # a piece of 32 terms: 12 truncations (a bit of 2^-23 each) of sums of at most the terms' magnitudes, two of them of whole
-    # ones, the others 2^-8 and less; left-out products below 2^-25; three roundings of four pieces; one to the result
+    # ones, the others 2^-8 and less; left-out products below 2^-25; the roundings of three pieces' sum; one to the result
     assert ((out.double() - ref).abs() <= (2 * 2.0 ** -23 + 2.0 ** -25 + 4 * 2.0 ** -24 + 2.0 ** -26) * mag).all()
     old = ops.gemm_simt(a, w, torch.float32)
     if M * N >= 10000:                                       # the error is no larger than the CUDA cores' (1.31e-7 / 2 against 1.26)
         assert (out.double() - ref).norm() <= 1.02 * (old.double() - ref).norm()
     assert int(ops.status_word(DEV).item()) == 0
+
+
+# what rows hold: the products of a gated feed-forward, whose sums must be as exact as on the CUDA cores (the norms of 61,440 errors
+# lie within 2 %), and terms of one sign, which come out low
+@pytest.mark.gpu
+@pytest.mark.parametrize("what", ["gated", "one sign", "one sign, several decades"])
+@pytest.mark.parametrize("K", [128, 2048, 8192])
+def test_float32_tc_error_by_what_rows_hold(what, K):
+    from picolm_b200 import ops
+    torch.manual_seed(K)
+    x, y, w = torch.randn(96, K, device=DEV), torch.randn(96, K, device=DEV), torch.randn(640, K, device=DEV)
+    a = torch.nn.functional.silu(x) * y if what == "gated" else x.abs()
+    if what != "gated":
+        w = w.abs()
+    if what == "one sign, several decades":
+        a, w = (2 * a).exp(), (2 * w).exp()
+    got, ref = ops.gemm_f32_tc(a, w), a.double() @ w.double().T
+    if what == "gated":
+        old = ops.gemm_simt(a, w, torch.float32)
+        assert (got.double() - ref).norm() <= 1.02 * (old.double() - ref).norm()
+        return
+    # a whole-sized MMA (two a piece, one of them of half the sum) truncates its result (2^-23) and cuts its 17 addends off two
+    # bits below that, all of the largest one's size at most; then the bounds of sums of both signs
+    cut = 17 * 2.0 ** -25 if what == "one sign, several decades" else 17 / 4 * 2.0 ** -25     # (the largest of 16: a quarter of them at most)
+    assert (got.double() - ref).norm() <= (1.5 * (2.0 ** -23 + cut) + 4 * 2.0 ** -24) * ref.norm()
 
 
 @pytest.mark.gpu
