@@ -336,6 +336,10 @@ int f32_form(int M, int N) {
 // out[t, n] for K of 8, 16 or 32 (a bottleneck's way back up): a thread keeps four columns' weights in registers and takes
 // NARROW_ROWS rows, whose values it reads from shared memory.  Bound by the rows written.  The same chain of sums as
 // gemm_simt_kernel (2,048 rows x 1,024 x 16: 7.8 -> 6.0 us without warm caches).
+// With few results a thread's rows one behind the other take longer than that kernel's blocks side by side, so they go there.  us here /
+// there, warm caches: 1 x 2,048 x 16 1.89 / 2.20, 4 x 2,048 x 32 3.09 / 3.50, 8 x 2,048 x 32 3.58 / 3.42, 64 x 2,048 x 16 3.25 / 2.74, 512 x
+// 1,024 x 16 3.32 / 2.88, 256 x 4,096 x 16 3.32 / 3.94, 1,024 x 1,024 x 32 4.48 / 5.64, 4,096 x 256 x 16 4.27 / 3.70 (half of a block idles); 8
+// terms: 16 x 1,024 2.55 / 2.48, 64 x 1,024 2.57 / 2.71, 2,048 x 1,024 3.18 / 5.94.
 constexpr int NARROW_ROWS = 16;
 template <int K>
 __global__ void __launch_bounds__(128)
@@ -380,6 +384,10 @@ gemm_narrow_kernel(const bf16* A, const bf16* W, bf16* __restrict__ C, int M, in
     }
 }
 
+bool narrow_pays(int M, int N, int K) {
+    return M <= 4 || (N >= 512 && (long)M * N >= (K == 8 ? 1l << 16 : 1l << 20));
+}
+
 template <int K>
 int launch_narrow(const void* A, const void* W, void* C, int M, int N, long lda, long ldw, long ldc, cudaStream_t stream) {
     gemm_narrow_kernel<K><<<dim3((N + 511) / 512, (M + NARROW_ROWS - 1) / NARROW_ROWS), 128, 0, stream>>>((const bf16*)A, (const bf16*)W, (bf16*)C, M, N, lda, ldw, ldc);
@@ -415,7 +423,7 @@ extern "C" int plm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dt
     if (a_dtype == PLM_F32 && w_dtype == PLM_F32 && c_dtype == PLM_F32)
         return launch<float, float, float>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     if (a_dtype == PLM_BF16 && w_dtype == PLM_BF16 && c_dtype == PLM_BF16 && (K == 8 || K == 16 || K == 32) && N % 4 == 0 && ldw % 8 == 0 &&
-        ldc % 4 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)C % 8 == 0 && (M + NARROW_ROWS - 1) / NARROW_ROWS <= 65535)
+        ldc % 4 == 0 && (uintptr_t)W % 16 == 0 && (uintptr_t)C % 8 == 0 && (M + NARROW_ROWS - 1) / NARROW_ROWS <= 65535 && narrow_pays(M, N, K))
         return K == 8 ? launch_narrow<8>(A, W, C, M, N, lda, ldw, ldc, stream) : K == 16 ? launch_narrow<16>(A, W, C, M, N, lda, ldw, ldc, stream)
                                                                               : launch_narrow<32>(A, W, C, M, N, lda, ldw, ldc, stream);
     if (a_dtype == PLM_BF16 && w_dtype == PLM_BF16 && c_dtype == PLM_BF16)

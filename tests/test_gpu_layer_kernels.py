@@ -21,7 +21,7 @@ def _step(lens):
 
 
 @pytest.mark.parametrize("K", [8, 16, 32])
-@pytest.mark.parametrize("M,N", [(1, 4), (17, 512), (50, 516), (33, 1028)])
+@pytest.mark.parametrize("M,N", [(1, 4), (3, 1028), (17, 512), (50, 516), (33, 1028), (130, 516), (1025, 1028), (2050, 516)])
 def test_products_with_few_terms_give_the_bits_of_the_general_one(M, N, K):
     from picolm_b200 import ops
     torch.manual_seed(M + N + K)
