@@ -5,9 +5,9 @@
 // row with the input (picolm/tensor.c:1394-1418), element types widened to fp32
 // inside the dot product (picolm/quant.c:133-153, picolm/quant.c:679).
 //
-// It is the product of the float32 path where rows do not start on 16-byte boundaries (the others run on the
-// tensor cores, gemm_f32_tc.cu), of few-column pieces that a part asks for here, and the any-size product of the
-// bfloat16 path when a shape does not fit the tensor-core kernel.  Each output element is accumulated over k in
+// It is the product of the float32 path where the weights are small (up to 131,072 of them) or rows do not start on
+// 16-byte boundaries (the others run on the tensor cores, gemm_f32_tc.cu), of few-column pieces that a part asks for here,
+// and the any-size product of the bfloat16 path when a shape does not fit the tensor-core kernel.  Each output element is accumulated over k in
 // ascending order by one thread, so a row's result never depends on which other
 // rows are in the batch.  With all three types float32 the sum of each piece of BK terms is folded into a
 // double: the error of a long dot product then stays that of a short one (a recurrence that keeps a state for

@@ -49,6 +49,17 @@ def gemm_f32_tc_supported(a: torch.Tensor, w: torch.Tensor, out_dtype: torch.dty
             and w.is_contiguous() and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
 
 
+def f32_tc_pays(N: int, K: int) -> bool:
+    """Whether a float32 product of N columns and K terms a sum runs on the tensor cores rather than on the CUDA cores.  By N and K
+    alone: a row's result must not depend on how many rows stand beside it.  A tile of the tensor cores' kernel takes 3.3 us and some
+    0.4 a piece of 32 terms however little there is to do.  Tensor cores / CUDA cores, us, for 1, 128, 512 and 2,048 rows: 128 x
+    128 4.6 / 2.3, 4.8 / 2.4, 5.0 / 3.1, 5.1 / 6.1; 512 x 256 6.1 / 3.4, 6.5 / 4.7, 6.6 / 10.5, 9.3 / 21; 128 x 1,024 14.7 / 9.4, 15.1 / 9.7,
+    15.5 / 14.8, 15.7 / 36; 1,024 x 256 6.1 / 3.4, 6.6 / 6.4, 7.5 / 17, 17 / 35; 512 x 512 9.0 / 5.4, 9.6 / 8.1, 9.7 / 19, 13 / 40; 256 x 2,048 15.5 /
+    17.6, 16.0 / 24, 16.2 / 39, 23 / 123.  So up to 131,072 weights and 1,024 terms the CUDA cores are faster up to some
+    hundreds of rows, above that the tensor cores for most numbers of rows."""
+    return K > 1024 or N * K > 1 << 17
+
+
 def gemm_f32_tc(a: torch.Tensor, w: torch.Tensor, form: int = 0) -> torch.Tensor:
     """out[M, N] = a[M, K] @ w[N, K]^T, all float32, on the tensor cores with every float in three bfloat16 terms and the error
     of float32 sums (csrc/gemm_f32_tc.cu).  `form`: rows of `a` a tile + 1000 * CTAs a tile, 0 for the one that fits; every
@@ -430,7 +441,8 @@ def linear(a, w: torch.Tensor, out_dtype: torch.dtype, defer: bool = False):
     """a [M, K] times w [N, K]^T -> [M, N].  The kernel is chosen by element
     types and shape, never by the model: the tensor cores for bfloat16 operands
     that TMA can address (the cluster kernel for up to 64 rows, the wide kernel
-    beyond) and for float32 ones with rows on 16-byte boundaries, the CUDA cores for everything else.
+    beyond) and for float32 ones with rows on 16-byte boundaries and more than a small matrix of weights (`f32_tc_pays`), the
+    CUDA cores for everything else.
 
     `a` may be `ScaledRows`.  With `defer` (a float32 delta for the residual stream) the product may
     come back as a `PendingLinear` for the next norm to run; whoever cannot use that calls `compute()`."""
@@ -453,6 +465,6 @@ def linear(a, w: torch.Tensor, out_dtype: torch.dtype, defer: bool = False):
         if a.shape[0] <= 64:
             return gemm_tc_skinny(a, w, out_dtype)
         return gemm_tc_wide(a, w, out_dtype, pair=pair_pays(a.shape[0], w.shape[0], a.shape[1], 0))
-    if gemm_f32_tc_supported(a, w, out_dtype):
+    if gemm_f32_tc_supported(a, w, out_dtype) and f32_tc_pays(*w.shape):
         return gemm_f32_tc(a, w)
     return gemm_simt(a, w, out_dtype)

@@ -127,9 +127,22 @@ def test_float32_tc_of_the_smallest_and_largest_operands(small, large):
 def test_linear_of_float32_rows_off_their_boundaries_takes_the_cuda_cores():
     from picolm_b200 import ops
     torch.manual_seed(6)
-    wide, w = torch.randn(20, 68, device=DEV), torch.randn(96, 64, device=DEV)
+    wide, w = torch.randn(20, 68, device=DEV), torch.randn(2100, 64, device=DEV)
     odd = wide[:, 1:65]
     assert torch.equal(ops.linear(odd, w, torch.float32), ops.gemm_simt(odd, w, torch.float32))
     assert torch.equal(ops.linear(odd.contiguous(), w, torch.float32), ops.gemm_f32_tc(odd.contiguous(), w))
     with pytest.raises(ops.KernelError):
         ops.gemm_f32_tc(odd, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N,K,tensor_cores", [(64, 64, False), (2048, 64, False), (2052, 64, True), (128, 1024, False), (64, 1028, True)])
+def test_linear_of_small_float32_weights_takes_the_cuda_cores(N, K, tensor_cores):
+    """By the weights' sizes alone, so that a row's bits are the same beside any number of others."""
+    from picolm_b200 import ops
+    torch.manual_seed(7)
+    a, w = torch.randn(600, K, device=DEV), torch.randn(N, K, device=DEV)
+    out = ops.linear(a, w, torch.float32)
+    assert torch.equal(out, ops.gemm_f32_tc(a, w) if tensor_cores else ops.gemm_simt(a, w, torch.float32))
+    for rows in (1, 7, 33, 300):
+        assert torch.equal(ops.linear(a[:rows], w, torch.float32), out[:rows])
