@@ -10,11 +10,11 @@
 // fp32.
 //
 // Why beside decay_chunk.cu: `mma.sync` runs at an eighth of tcgen05's rate here (some 16 cycles an m16n8k16 and scheduler), and
-// that kernel spends its time on it.  16 heads of 128 x 256, us there / here: one sequence of 2,048 tokens 107 / 66, of 256 35 / 22, of 129
-// 26 / 22; 8 heads of 64 x 128, 300 and 100 tokens 29 / 18; below 129 tokens a sequence a chunk is mostly empty (three sequences of
-// 100, 40, 30: 21 / 26) and the step runs there.  Of the 66 the outputs are 41 (a CTA's phases follow one another: loads and
-// rotation, products, results), the chunks' sums 19, the states 10.  Errors against 64 bits are the same (8.9e-6 of 2,048 tokens'
-// outputs, 1.0e-5 of the state, from the 16 bits of what is kept in two terms).
+// that kernel spends its time on it.  16 heads of 128 x 256, us there / here: one sequence of 2,048 tokens 107 / 65, of 256 35 / 24, of 129
+// 25 / 22; 8 heads of 64 x 128, 300 tokens and eight of 16 30 / 20.  Many short sequences leave the chunks half empty and run there
+// (which step runs where: ops/recurrent.py, decay_in_128).  Of the 65 the outputs are 41 (a CTA's phases follow one another: loads and
+// rotation, products, results), the chunks' sums 19, the states 10.  Errors against 64 bits, there / here (the 16 bits of what is kept in
+// two terms): 5.9e-6 / 5.1e-6 of 2,048 tokens' outputs, 4.1e-6 / 2.5e-6 of the state.
 //
 // What is not finite in a token's v goes in as zero and makes the outputs of its column no numbers from that token on, so that
 // the zero weights of earlier tokens make none of it; in the state it stays as it is.
@@ -35,7 +35,7 @@ struct DecayArgs {
     float* y;
     long ldy;
     const int *seq_start, *seq_slot;
-    int n_seqs, H, N, P, chunks;                       // chunks of the longest sequence
+    int n_seqs, H, N, P;
     const float *cos_t, *sin_t;
     const int* tok_pos;
     int half;
@@ -48,17 +48,38 @@ struct DecayArgs {
     __device__ long slot(int s0, int b, int c) const { return s0 / C + b + c; }
 };
 
+// A block's chunk, head and value tiles.  Blocks stand for the chunks' places and not for every sequence's chunks up to the longest
+// one's, so at most one place a sequence is empty: a block finds its chunk's sequence by a warp's search over the places where
+// sequences begin.  (A block for every sequence and chunk of the longest: 2,000 tokens beside 63 of 1, 16 heads of 128 x 256, 547 us for 334;
+// 700 beside 20 of 60 with a captured step's bounds 241 for 140.)
 struct Where { int b, h, c, p0, t0, n; };
 __device__ __forceinline__ Where where_of(const DecayArgs& a) {
     Where w;
     unsigned u = blockIdx.x;
     const unsigned parts = (unsigned)((a.tiles + a.per - 1) / a.per);
     w.p0 = (int)(u % parts) * a.per * PT, u /= parts;
-    w.h = (int)(u % (unsigned)a.H), w.c = (int)(u / (unsigned)a.H);
-    w.b = blockIdx.y;
-    const int s0 = a.seq_start[w.b], s1 = a.seq_start[w.b + 1];
+    w.h = (int)(u % (unsigned)a.H);
+    const int place = (int)(u / (unsigned)a.H), lane = threadIdx.x & 31;
+    int s0, s1;
+    if (a.n_seqs < 32) {                               // all of them in one load
+        const int start = a.seq_start[min(lane, a.n_seqs)];
+        const bool begun = lane < a.n_seqs && (int)a.slot(start, lane, 0) <= place;
+        w.b = max(__popc(__ballot_sync(0xffffffffu, begun)) - 1, 0);             // (places ascend)
+        s0 = __shfl_sync(0xffffffffu, start, w.b), s1 = __shfl_sync(0xffffffffu, start, w.b + 1);
+    } else {
+        int hi = a.n_seqs;                             // the sequence is one from w.b on and before this
+        w.b = 0;
+        while (hi - w.b > 1) {
+            const int step = (hi - w.b + 31) / 32, b = w.b + lane * step;
+            const bool begun = b < hi && (int)a.slot(a.seq_start[b], b, 0) <= place;
+            w.b += max(__popc(__ballot_sync(0xffffffffu, begun)) - 1, 0) * step;
+            hi = min(hi, w.b + step);
+        }
+        s0 = a.seq_start[w.b], s1 = a.seq_start[w.b + 1];
+    }
+    w.c = place - (int)a.slot(s0, w.b, 0);
     w.t0 = s0 + w.c * C;
-    w.n = min(C, s1 - w.t0);
+    w.n = w.c < 0 ? 0 : min(C, s1 - w.t0);
     return w;
 }
 // d^e for e of 0 .. 128 from the table of 65
@@ -506,12 +527,12 @@ __global__ void __launch_bounds__(OUT_ALL, 1) decay_out_kernel(const DecayArgs a
 }
 
 template <int NP>
-int launch(const DecayArgs& a, cudaStream_t stream) {
+int launch(const DecayArgs& a, long places, cudaStream_t stream) {
     static std::atomic<unsigned long long> add_devices{0}, out_devices{0};
     static_assert(out_smem<NP>() <= 232448 - 1536, "shared memory");
     cudaError_t e = plm_allow_smem(decay_add_kernel<NP>, add_smem<NP>(), add_devices);
     if (e == cudaSuccess) e = plm_allow_smem(decay_out_kernel<NP>, out_smem<NP>(), out_devices);
-    const dim3 units((unsigned)((long)a.chunks * a.H * ((a.tiles + a.per - 1) / a.per)), (unsigned)a.n_seqs);
+    const dim3 units((unsigned)(places * a.H * ((a.tiles + a.per - 1) / a.per)));
     if (e == cudaSuccess) e = launch_pdl(decay_add_kernel<NP>, units, dim3(ADD_NT), add_smem<NP>(), stream, a);
     const long quads = (long)a.H * a.N * a.P / 4;
     if (e == cudaSuccess) e = launch_pdl(decay_states_kernel, dim3((unsigned)((quads + STATES_NT - 1) / STATES_NT), (unsigned)a.n_seqs), dim3(STATES_NT), 0, stream, a);
@@ -525,7 +546,7 @@ int launch(const DecayArgs& a, cudaStream_t stream) {
 // runs in decay_chunk.cu.
 extern "C" long plm_decay_tc_floats(int n_tokens, int n_seqs, int max_new, int H, int N, int P, int half) {
     if (n_seqs <= 0 || n_seqs > 65535 || max_new <= 0 || H <= 0 || (N != 64 && N != 128) || P <= 0 || P % PT || half % 8) return 0;
-    const long floats = 2 * ((long)n_tokens / C + n_seqs) * H * N * P, units = ((long)max_new + C - 1) / C * H * (P / PT);
+    const long floats = 2 * ((long)n_tokens / C + n_seqs) * H * N * P, units = ((long)n_tokens / C + n_seqs) * H * (P / PT);
     return floats <= (1l << 28) && units <= 0x7fffffffl ? floats : 0;
 }
 
@@ -542,8 +563,9 @@ extern "C" int plm_decay_tc_scan(const void* q, const void* k, const void* v, lo
         ldq % 8 || ldk % 8 || ldv % 8 || state_stride % 4 || ldy % 4)
         return PLM_ERR_ALIGN;
     DecayArgs a = {(const bf16*)q, (const bf16*)k, (const bf16*)v, ldq, ldk, ldv, powers, state, state_stride, y, ldy, seq_start, seq_slot,
-                         n_seqs, H, N, P, (max_new + C - 1) / C, cos_t, sin_t, tok_pos, half, k_scale, ws, (bf16*)(ws + ((long)n_tokens / C + n_seqs) * H * N * P), status, P / PT, 1};
+                         n_seqs, H, N, P, cos_t, sin_t, tok_pos, half, k_scale, ws, (bf16*)(ws + ((long)n_tokens / C + n_seqs) * H * N * P), status, P / PT, 1};
     // a CTA takes all value tiles of its (chunk, head) where that leaves a CTA for most SMs
-    a.per = ((long)n_tokens / C + n_seqs) * H >= PLM_SM_COUNT ? a.tiles : 1;
-    return N == 64 ? launch<64>(a, stream) : launch<128>(a, stream);
+    const long places = (long)n_tokens / C + n_seqs;
+    a.per = places * H >= PLM_SM_COUNT ? a.tiles : 1;
+    return N == 64 ? launch<64>(a, places, stream) : launch<128>(a, places, stream);
 }

@@ -18,7 +18,7 @@ from .gemm import (PLAIN_ACTIVATIONS, PendingLinear, ScaledRows, gemm_f32_tc, ge
                    residual_norm_supported)
 from .recurrent import (IN_CHUNKS, ONE_PASS, SCAN_CHUNK_KEYS, StepShape, delta_scan_in_chunks, linear_scan_route, step_shape,  # noqa: F401
                         DECAY_CONST, DECAY_SIGMOID, DECAY_STEP, GATE_AFTER_NORM, GATE_BEFORE_NORM, GATE_NONE, causal_conv,  # noqa: F401
-                        decay_chunk_supported, decay_powers, decay_scan, delta_head_chunk_sizes, delta_prep, delta_scan, diag_scan, gated_norm, head_linear, linear_scan, rglru_gates,
+                        decay_chunk_supported, decay_in_128, decay_in_128_supported, decay_powers, decay_scan, delta_head_chunk_sizes, delta_prep, delta_scan, diag_scan, gated_norm, head_linear, linear_scan, rglru_gates,
                         store_rows_paged, latent_store)
 from .routed import (TC_EXPERTS, SortedPairs, moe_align, moe_combine, moe_down, moe_down_tc, moe_gate_up, moe_gate_up_tc,  # noqa: F401
                      moe_gather, moe_max_tiles, moe_tc_supported, moe_up, moe_up_tc, route_topk, router_logits)

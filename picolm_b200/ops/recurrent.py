@@ -277,10 +277,28 @@ def decay_chunk_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key
             and all(t.data_ptr() % 16 == 0 and t.stride(0) % 8 == 0 for t in (q, k, v)))
 
 
-# tokens of a step's longest sequence, and of its sequences on average, from which a constant decay's recurrence over rotated
-# rows runs 128 tokens at a time on tcgen05: below, a chunk is mostly empty (16 heads of 128 x 256, us 64 at a time / 128: one
-# sequence of 65 tokens 17 / 20, of 129 26 / 22, of 256 35 / 22, of 2,048 107 / 66; three of 100, 40, 30 21 / 26)
-DECAY_TC_FROM = 129
+def decay_in_128_supported(key_dim: int, value_dim: int) -> bool:
+    """Whether a constant decay's recurrence over rotated bfloat16 rows can run 128 tokens at a time (csrc/decay_tc.cu)."""
+    return key_dim in (64, 128) and value_dim % 128 == 0
+
+
+def decay_in_128(shape: StepShape, heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether a constant decay's recurrence over rotated rows runs a step of this shape 128 tokens at a time on tcgen05 rather than 64
+    at a time.  Where the latter cuts sequences into segments (two passes) it always does; else by an estimate of both in microseconds,
+    fitted to what was measured (1 to 64 sequences of 1 to 3,000 tokens, eager and with a captured step's bounds): there a sequence's
+    chunks are a chain and all states pass the same memory, here there are some 15 us of launches, then the chunks, side by
+    side.  64 at a time / 128, 16 heads of 128 x 256: one sequence of 100 tokens 20 / 20, of 129 25 / 22, of 200 34 / 22, of 2,048 107 / 65 (in
+    segments); two of 129 26 / 27, of 200 34 / 27; four of 129 26 / 42, of 256 39 / 43, of 400 60 / 67; 8 of 256 76 / 77, 16 of 100 78 / 88; 2,048
+    beside three of 1 210 / 82, 2,000 beside 63 486 / 334, 700 beside 20 of 60 100 / 128.  8 heads of 64 x 128: one of 129 16 / 18, of 200 21 / 17,
+    four of 170 18 / 18, of 256 23 / 19, 16 of 100 13 / 24."""
+    longest, tokens, seqs, chunks = shape
+    if longest <= DECAY_CHUNK:
+        return False
+    if _decay_chunk_plan(seqs, heads, key_dim, value_dim, longest, tokens)[1] > 1:
+        return True
+    work, of_128 = heads * key_dim * value_dim / (16 * 128 * 256), chunks / 2 + seqs / 4
+    in_64 = max((8.2 if key_dim > 64 else 5.2) * ((longest + 63) // 64), 2.1 * work * chunks)
+    return 14.5 + of_128 * (3.0 * work + 0.11) + seqs * work < in_64
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, powers: torch.Tensor,
@@ -293,8 +311,9 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     token's position and `k_scale` multiplies k, on the way in, in float32 and without a rounding behind (either of
     them given: no activation).
     `state` float32 [slots, >= heads * key_dim * value_dim] is carried on.  Steps with prompts in bfloat16 run 64 tokens
-    at a time on the tensor cores where the sizes allow it, steps of single tokens stream the state through once,
-    everything else goes token by token (`linear_scan`)."""
+    at a time on the tensor cores where the sizes allow it, rotated or scaled ones 128 at a time on tcgen05 where that is faster
+    (`decay_in_128`: it depends on all sequences of the step, and with it the order of the sums); steps of single tokens stream the
+    state through once, everything else goes token by token (`linear_scan`)."""
     H, N, P = heads, key_dim, value_dim
     T = v.shape[0]
     if q.shape != (T, H * N) or k.shape != (T, H * N) or v.shape != (T, H * P) or activation not in (None, "silu"):
@@ -313,7 +332,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     if state.dtype != torch.float32 or state.shape[1] < H * N * P:
         raise KernelError("decay_scan: the state must be float32 with heads * key_dim * value_dim values a row")
     y = torch.empty((T, H * P), dtype=torch.float32, device=v.device)
-    floats = _decay_tc_floats(T, step.n_seqs, step.max_new, H, N, P, turn)
+    floats = _decay_tc_floats(step, H, N, P, turn)
     if floats:
         ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
         _check(_fn("decay_tc", "plm_decay_tc_scan")(
@@ -336,11 +355,11 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.T
     return y
 
 
-def _decay_tc_floats(n_tokens: int, n_seqs: int, max_new: int, H: int, N: int, P: int, turn) -> int:
-    """Floats of workspace that a step takes on tcgen05, 128 tokens at a time (csrc/decay_tc.cu); 0: it runs 64 at a time."""
-    if turn is None or max_new < DECAY_TC_FROM or n_tokens < DECAY_TC_FROM * n_seqs:
+def _decay_tc_floats(step, H: int, N: int, P: int, turn) -> int:
+    """Floats of workspace that a step takes 128 tokens at a time; 0: it runs 64 at a time."""
+    if turn is None or not decay_in_128_supported(N, P) or not decay_in_128(step_shape(step), H, N, P):
         return 0
-    return _fn("decay_tc", "plm_decay_tc_floats")(n_tokens, n_seqs, int(max_new), H, N, P, turn.half)
+    return _fn("decay_tc", "plm_decay_tc_floats")(step.n_tokens, step.n_seqs, int(step.max_new), H, N, P, turn.half)
 
 
 class _Turn:

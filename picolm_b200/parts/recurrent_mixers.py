@@ -257,6 +257,13 @@ class Retention(_StateMixer):
         if self.position is not None:
             self.position.prepare(max_seq_tokens)
 
+    @property
+    def chooses_by_shape(self) -> bool:
+        return self.runtime.dtype == torch.bfloat16 and ops.decay_in_128_supported(self.N, self.P)
+
+    def step_route(self, shape):
+        return ops.decay_in_128(shape, self.H, self.N, self.P)
+
     def forward(self, h, step, cache):
         dt = self.runtime.dtype
         HN, HP = self.H * self.N, self.H * self.P

@@ -2,6 +2,7 @@
 plain computations."""
 import math
 import types
+from unittest import mock
 
 import pytest
 import torch
@@ -208,6 +209,7 @@ def test_chunk_products_of_the_smallest_and_largest_values(small, large):
 def _retention(N, P, lens, H=3, positions=0, odd=None):
     """ops.decay_scan over rotated rows, its inputs, and the same in float64 with everything that the kernels are handed."""
     from picolm_b200 import ops
+    from picolm_b200.ops import recurrent
     torch.manual_seed(N + P + sum(lens))
     T = sum(lens)
     start = [sum(lens[:b]) for b in range(len(lens))]
@@ -225,7 +227,8 @@ def _retention(N, P, lens, H=3, positions=0, odd=None):
     rotation = types.SimpleNamespace(cos=angle.cos().float().to(DEV), sin=angle.sin().float().to(DEV), rotary_dim=N, pairing="half")
     state = torch.randn(len(lens), H * N * P, device=DEV)
     before = state.clone()
-    y = ops.decay_scan(q, k, v, decay.float().to(DEV), ops.decay_powers(decay).to(DEV), state, step, H, N, P, rotation=rotation, k_scale=N ** -0.5)
+    with mock.patch.object(recurrent, "decay_in_128", lambda *a: True):                # (whatever the rule would choose)
+        y = ops.decay_scan(q, k, v, decay.float().to(DEV), ops.decay_powers(decay).to(DEV), state, step, H, N, P, rotation=rotation, k_scale=N ** -0.5)
     want, states = [], []
     for b, n in enumerate(lens):
         c, s = (f[positions:positions + n].double()[:, None] for f in (rotation.cos, rotation.sin))
@@ -235,7 +238,7 @@ def _retention(N, P, lens, H=3, positions=0, odd=None):
         for i in range(n):
             S = S * decay.to(DEV)[:, None, None] + kk[i][:, :, None] * vv[i][:, None]
             out.append(torch.bmm(qq[i][:, None], S)[:, 0].reshape(-1))
-        want.append(torch.stack(out))
+        want += [torch.stack(out)] if out else []
         states.append(S.reshape(-1))
     ops.check_status(DEV)
     return y, torch.cat(want), state, torch.stack(states)
@@ -251,6 +254,13 @@ def test_retention_128_tokens_at_a_time(N, P, lens):
     assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
     for t in range(0, want.shape[0], 37):
         assert (y[t].double() - want[t]).norm() <= 6 * 2.0 ** -17 * want[t].norm()
+
+
+@pytest.mark.parametrize("lens", [[0, 140, 0, 0, 1, 300, 0], [(7 * i) % 40 for i in range(70)], [300] + [i % 3 for i in range(1100)] + [129]])
+def test_retention_chunks_find_their_sequences(lens):
+    """Sequences of no tokens, more sequences than a warp has lanes, more than a warp's square."""
+    y, want, state, states = _retention(64, 128, lens, H=1)
+    assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
 
 
 def test_many_retention_chunks_share_their_weights_between_value_tiles():
