@@ -15,7 +15,7 @@ def _marks_behind_the_wait():
     with open(SOURCE) as f:
         text = f.read()
     text = text[text.index("chunk_product_kernel("):]
-    return text.index("mbar_wait(mma_done(group)") < text.index("atomicMin(&reached_from")
+    return text.index("(mma_done(group)") < text.index("atomicMin(&reached_from")
 
 
 def _before(event, behind, ring, steps):
