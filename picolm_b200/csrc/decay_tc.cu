@@ -542,12 +542,13 @@ int launch(const DecayArgs& a, long places, cudaStream_t stream) {
 
 }  // namespace
 
-// Whether a step runs here, and the floats of workspace it takes (2 * (tokens / 128 + sequences) * H * N * P, at most 1 GiB); 0: it
-// runs in decay_chunk.cu.
+// Whether a step runs here, and the floats of workspace it takes (2 * (tokens / 128 + sequences) * H * N * P); 0: it
+// runs in decay_chunk.cu.  At most 512 MB, as scan_chunk.cu takes (16 heads of 128 x 256: 16,000 tokens): a state for every chunk is
+// more than that kernel's one for every segment.
 extern "C" long plm_decay_tc_floats(int n_tokens, int n_seqs, int max_new, int H, int N, int P, int half) {
     if (n_seqs <= 0 || n_seqs > 65535 || max_new <= 0 || H <= 0 || (N != 64 && N != 128) || P <= 0 || P % PT || half % 8) return 0;
     const long floats = 2 * ((long)n_tokens / C + n_seqs) * H * N * P, units = ((long)n_tokens / C + n_seqs) * H * (P / PT);
-    return floats <= (1l << 28) && units <= 0x7fffffffl ? floats : 0;
+    return floats <= (1l << 27) && units <= 0x7fffffffl ? floats : 0;
 }
 
 // q, k [T, H * N], v [T, H * P] bf16 with row strides (rows on 16-byte boundaries); powers [H][65] fp32; state [slots][>= H * N * P]

@@ -24,6 +24,14 @@ def test_a_captured_step_goes_by_its_shape_and_not_by_its_bounds(lens, tokens, s
     assert floats == (2 * (tokens // 128 + seqs) * 16 * 128 * 256 if expected else 0)
 
 
+@pytest.mark.parametrize("tokens,expected", [(127 * 128 + 127, True), (128 * 128, False), (40000, False)])
+def test_no_more_workspace_than_half_a_gigabyte(tokens, expected):
+    """Beyond that a step runs 64 tokens at a time, whose workspace is a state a segment."""
+    step = types.SimpleNamespace(n_tokens=tokens, n_seqs=1, max_new=tokens)
+    floats = recurrent._decay_tc_floats(step, 16, 128, 256, types.SimpleNamespace(half=64))
+    assert (floats > 0) == expected and floats * 4 <= 512 << 20
+
+
 def test_a_part_says_how_it_runs_a_shape():
     def part(dtype, dim, vdim):
         params = dict(hidden_size=64, heads=16, dim=dim, vdim=vdim, decay=[0.9] * 16, eps=1e-5, position=None)
