@@ -1238,24 +1238,16 @@ extern "C" int plm_delta_channel_scan(const float* qn, const float* kn, const fl
                             : by_size<bf16, true>(a, n_tokens, n_seqs, max_new, ws_floats, stream);
 }
 
-// The device word where this thread's launches of plm_sigmoid_chunk_scan leave a wait that ran out (a launch takes it along as an
-// argument).
-static thread_local int* g_sigmoid_status = nullptr;
-extern "C" int plm_sigmoid_chunk_status(int* status) {
-    g_sigmoid_status = status;
-    return PLM_OK;
-}
-
 // Linear attention with the decays sigmoid(raw + bias)^power: q, k, v, raw of `dtype`.
 extern "C" int plm_sigmoid_chunk_scan(const void* q, const void* k, const void* v, const void* raw, int dtype, long ldq, long ldk, long ldv,
                                       long ldr, const float* bias, float q_scale, float power, float* state, long state_stride, float* y,
                                       float* ws, long ws_floats, const int* seq_start, const int* seq_slot, int n_tokens, int n_seqs,
-                                      int max_new, int H, int N, int P, int heads_per_group, cudaStream_t stream) {
+                                      int max_new, int H, int N, int P, int heads_per_group, int* status, cudaStream_t stream) {
     if (!bias) return PLM_ERR_SHAPE;
     if (n_seqs <= 0 || max_new <= 0) return PLM_OK;
     const Args a = {q, k, v, raw, ldq, ldk, ldv, ldr, nullptr, bias, power, q_scale, ws, state, state_stride, y, seq_start, seq_slot,
                     H, N, P, heads_per_group, 0,
-                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, g_sigmoid_status, 0, 0, 0};
+                    P % 4 == 0 && ldv % 4 == 0 && (uintptr_t)v % (dtype == PLM_F32 ? 16 : 8) == 0, status, 0, 0, 0};
     const int e = check(a, n_seqs, max_new, dtype);
     if (e != PLM_OK) return e;
     return dtype == PLM_F32 ? by_size<float, false>(a, n_tokens, n_seqs, max_new, ws_floats, stream)

@@ -94,8 +94,7 @@ _SIGNATURES = {
     "plm_delta_scan": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _l, _vp, _l, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp],
     "plm_scan_chunk_floats": [_i, _i],
     "plm_delta_channel_scan": [_vp, _vp, _vp, _vp, _vp, _i, _l, _vp, _l, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
-    "plm_sigmoid_chunk_status": [_vp],
-    "plm_sigmoid_chunk_scan": [_vp, _vp, _vp, _vp, _i, _l, _l, _l, _l, _vp, _f, _f, _vp, _l, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
+    "plm_sigmoid_chunk_scan": [_vp, _vp, _vp, _vp, _i, _l, _l, _l, _l, _vp, _f, _f, _vp, _l, _vp, _vp, _l, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp, _vp],
     "plm_linear_scan": [_vp, _vp, _vp, _vp, _i, _l, _l, _l, _l, _i, _vp, _vp, _vp, _f, _f, _vp, _l, _vp, _l, _vp, _vp,
                         _i, _i, _i, _i, _i, _i, _i, _vp, _vp, _i, _vp],
     "plm_sigmoid_decay": [_vp, _i, _l, _vp, _f, _vp, _i, _i, _vp],

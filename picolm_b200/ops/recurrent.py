@@ -139,10 +139,10 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, raw: Optional
     if route == IN_CHUNKS and step.n_seqs <= SCAN_CHUNK_SEQS:
         floats, stretches = scan_chunk_plan(T, step.n_seqs, int(step.max_new), H, N, P)
         ws = torch.empty((floats,), dtype=torch.float32, device=v.device)
-        _fn("scan_chunk", "plm_sigmoid_chunk_status")(_p(status_word(v.device)))
         _check(_fn("scan_chunk", "plm_sigmoid_chunk_scan")(
             _p(q), _p(k), _p(v), _p(raw), _dt(v, "v"), ldq, ldk, ldv, ldr, _p(p0), float(q_scale), float(power), _p(state), lds, _p(y),
-            _p(ws), floats, _p(step.seq_start), _p(step.seq_slot), T, step.n_seqs, int(step.max_new), H, N, P, heads_per_group, _stream()),
+            _p(ws), floats, _p(step.seq_start), _p(step.seq_slot), T, step.n_seqs, int(step.max_new), H, N, P, heads_per_group,
+            _p(status_word(v.device)), _stream()),
             f"sigmoid_chunk_scan T={T} H={H} N={N} P={P}", kernels=4 * stretches,
             nbytes=T * ((2 * G * N + H * N + H * P) * v.element_size() + H * P * 4) + 2 * step.n_seqs * H * N * P * 4,
             flops=2 * T * H * (2 * N * P + 64 // 2 * (N + P)))

@@ -20,7 +20,7 @@ def test_a_decay_from_logits_wants_its_bias(max_new):
     row = H * N
     assert _entry("scan_chunk", "plm_sigmoid_chunk_scan")(
         some, some, some, some, bf16, row, row, H * P, row, None, 1.0, 0.5, some, H * N * P, some, some, 1 << 20, some, some, T, 1, max_new, H, N, P, 1,
-        None) == -2
+        None, None) == -2
     assert _entry("recurrent", "plm_sigmoid_decay")(some, bf16, row, None, 0.5, some, T, row, None) == -2
     mode = 2                                                 # the decay from logits
     assert _entry("recurrent", "plm_linear_scan")(
