@@ -1,4 +1,4 @@
-// Recurrences with a decay per key channel, for prompts, 64 tokens at a time in fp32 on the CUDA cores:
+// Recurrences with a decay per key channel, for prompts, 64 tokens at a time in fp32:
 //   linear attention   S <- diag(d_t) S + k_t v_t^T,                                   o_t = S^T q_t
 //   the delta rule     S <- diag(d_t) S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T,  o_t = S^T q_t
 // With S the state before a chunk, L_t the running sum of the decays' logarithms inside it (per head and key channel) and C
@@ -13,11 +13,14 @@
 // What limits these is the chain from chunk to chunk, so only what needs the state stands in it.  All chunks side by side:
 // the scaled keys and queries, M, A and both triangular systems (`chunk_prep`).  In a sequence's order: for the delta rule
 // U and the state (`chunk_walk`, eight columns of the state a block), for linear attention a multiply and an add per value
-// of the state (`chunk_chain`, behind every chunk's own sum of k u^T, `chunk_outer`).  Then the outputs, all chunks side by
-// side (`chunk_out`).
-// 2,048 tokens, 8 heads of 128 x 128: the delta rule 518 us (32 tokens at a time, everything but the scaled keys and queries in
-// the chain) -> 145, linear attention 144 us (token by token in segments) -> 93; errors against 64 bits 4.9e-7 -> 2.0e-7 and
-// 2.0e-6 -> 2.7e-7 (outputs), 6.2e-7 -> 2.1e-7 and 2.4e-6 -> 1.6e-7 (state).
+// of the state (`chunk_chain`, behind every chunk's own sum of k u^T).  Then the outputs, all chunks side by side.  Those sums and
+// the outputs are products on the tensor cores where the state has more than 64 columns (`chunk_product`), else FFMA tiles
+// (`chunk_outer`, `chunk_out`); the rest runs on the CUDA cores.
+// 2,048 tokens, 8 heads of 128 x 128, warm caches: the delta rule 518 us (32 tokens at a time, everything but the scaled keys and queries in
+// the chain) -> SCAN_DELTA, linear attention 144 us (token by token in segments) -> SCAN_GLA.  Errors against 64 bits in 2^-24, all products FFMA / on
+// the tensor cores (512 tokens, 4 heads of 128 x 128, normal numbers; rows behind SiLU): linear attention's outputs 3.9 / 2.3 (2.8 / 1.4),
+// state 2.5 / 1.5 (1.7 / 1.2), the delta rule's outputs 3.4 / 3.2 (2.6 / 2.4); where all values are positive and spread over several
+// decades the tensor cores' are larger (3.3 / 4.2 and 1.8 / 3.0; see gemm_f32_tc.cu).
 #include "split_common.cuh"
 #include <type_traits>
 
@@ -558,16 +561,15 @@ chunk_walk_kernel(const Args a) {
     }
 }
 
-// A tile of 64 rows x PT columns of sums over rows of two row-major operands, A^T B, 16 rows of each at a time through a ring
-// of three stages: `rows(step, a, b)` says where a step's rows start (a: 64 floats a row, b: PT or as many as are left).
-// 128 threads, 8 x PT / 16 results each.
+// A tile of 64 rows x 64 columns of sums over rows of two row-major operands, A^T B, 16 rows of each at a time through a ring
+// of three stages: `rows(step, a, b)` says where a step's rows start (a: 64 floats a row, b: 64 or as many as there are).
+// 128 threads, 8 x 4 results each.
 constexpr int TK = 16, TSTAGES = 3;
-template <int PT> struct Tile {
-    float a[TSTAGES][TK][64], b[TSTAGES][TK][PT];
+struct Tile {
+    float a[TSTAGES][TK][64], b[TSTAGES][TK][64];
 };
-template <int PT, typename Rows>
-__device__ __forceinline__ void tile_sums(Tile<PT>& tile, uint64_t (&acc)[4][PT / 16], int n_steps, int b_cols, Rows rows) {
-    constexpr int TN = PT / 16;
+template <typename Rows>
+__device__ __forceinline__ void tile_sums(Tile& tile, uint64_t (&acc)[4][4], int n_steps, int b_cols, Rows rows) {
     const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
     auto fetch = [&](int i) {
         const float *pa, *pb;
@@ -581,9 +583,9 @@ __device__ __forceinline__ void tile_sums(Tile<PT>& tile, uint64_t (&acc)[4][PT 
             cp16(da + idx * 4, pa + (idx / 16) * lda + idx % 16 * 4);
         }
 #pragma unroll
-        for (int x = 0; x < TK * PT / 4 / 128; ++x) {
-            const int idx = tid + 128 * x, col = idx % (PT / 4) * 4;
-            if (col < b_cols) cp16(db + idx * 4, pb + (idx / (PT / 4)) * ldb + col);
+        for (int x = 0; x < TK * 16 / 128; ++x) {
+            const int idx = tid + 128 * x, col = idx % 16 * 4;
+            if (col < b_cols) cp16(db + idx * 4, pb + (idx / 16) * ldb + col);
             else *reinterpret_cast<float4*>(db + idx * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
@@ -600,69 +602,63 @@ __device__ __forceinline__ void tile_sums(Tile<PT>& tile, uint64_t (&acc)[4][PT 
         const int st = i % TSTAGES;
 #pragma unroll
         for (int k = 0; k < TK; ++k) {
-            uint64_t a2[4], b2[TN];
+            uint64_t a2[4], b2[4];
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
                 const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&tile.a[st][k][x * 32 + ty * 4]);
                 a2[2 * x] = v.x;
                 a2[2 * x + 1] = v.y;
             }
-#pragma unroll
-            for (int x = 0; x < TN / 4; ++x) {
-                const float4 v = ld4(&tile.b[st][k][x * 64 + tx * 4]);
-                b2[4 * x] = pair_of(v.x, v.x);
-                b2[4 * x + 1] = pair_of(v.y, v.y);
-                b2[4 * x + 2] = pair_of(v.z, v.z);
-                b2[4 * x + 3] = pair_of(v.w, v.w);
-            }
+            const float4 v = ld4(&tile.b[st][k][tx * 4]);
+            b2[0] = pair_of(v.x, v.x);
+            b2[1] = pair_of(v.y, v.y);
+            b2[2] = pair_of(v.z, v.z);
+            b2[3] = pair_of(v.w, v.w);
 #pragma unroll
             for (int x = 0; x < 4; ++x)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) acc[x][j] = fma2(a2[x], b2[j], acc[x][j]);
+                for (int j = 0; j < 4; ++j) acc[x][j] = fma2(a2[x], b2[j], acc[x][j]);
         }
     }
 }
-// the four columns x * 64 + tx * 4 .. of row r (0..7) of a thread's results
-template <int TN> __device__ __forceinline__ float4 four(const uint64_t (&acc)[4][TN], int r, int x) {
+// the four columns tx * 4 .. of row r (0..7) of a thread's results
+__device__ __forceinline__ float4 four(const uint64_t (&acc)[4][4], int r) {
     float v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float lo, hi;
-        halves(acc[r / 2][4 * x + j], lo, hi);
+        halves(acc[r / 2][j], lo, hi);
         v[j] = r & 1 ? hi : lo;
     }
     return make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // Linear attention: what a chunk adds to the state, sum_s (k_s e^(L_C - L_s)) v_s^T, into the state's place in the workspace.
-// grid (chunk x channels by 64 x columns by PT, head, sequence)
-template <int NP, int PT>
+// States of up to 64 columns; grid (chunk x channels by 64, head, sequence)
+template <int NP>
 __global__ void __launch_bounds__(128)
 chunk_outer_kernel(const Args a) {
     using Lay = Layout<NP>;
     constexpr int MT = NP / 64;
-    __shared__ __align__(16) Tile<PT> tile;
+    __shared__ __align__(16) Tile tile;
     pdl_launch_dependents();
     pdl_wait();
-    const int PP = pad4(a.P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, n0 = blockIdx.x / ptiles % MT * 64, c = a.c0 + blockIdx.x / ptiles / MT, h = blockIdx.y, b = a.b0 + blockIdx.z;
+    const int PP = pad4(a.P), n0 = blockIdx.x % MT * 64, c = a.c0 + blockIdx.x / MT, h = blockIdx.y, b = a.b0 + blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
     float* w = a.ws + (a.slot(s0, b, c) * a.H + h) * Lay::floats(PP);
-    uint64_t acc[4][PT / 16] = {};
-    tile_sums<PT>(tile, acc, (nt + TK - 1) / TK, PP - p0, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
+    uint64_t acc[4][4] = {};
+    tile_sums(tile, acc, (nt + TK - 1) / TK, PP, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
         pa = w + Lay::KE + (long)i * TK * NP + n0, lda = NP;
-        pb = w + Lay::U + (long)i * TK * PP + p0, ldb = PP;
+        pb = w + Lay::U + (long)i * TK * PP, ldb = PP;
     });
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
-#pragma unroll
-        for (int x = 0; x < PT / 64; ++x) {
-            const int n = n0 + r / 4 * 32 + ty * 4 + r % 4, p = p0 + x * 64 + tx * 4;
-            if (p < PP)                                  // (padding stays zero, whatever U holds)
-                *reinterpret_cast<float4*>(w + Lay::s(PP) + (long)n * PP + p) = n < a.N ? four(acc, r, x) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+    for (int r = 0; r < 8; ++r) {
+        const int n = n0 + r / 4 * 32 + ty * 4 + r % 4, p = tx * 4;
+        if (p < PP)                                      // (padding stays zero, whatever U holds)
+            *reinterpret_cast<float4*>(w + Lay::s(PP) + (long)n * PP + p) = n < a.N ? four(acc, r) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 }
 
 // Linear attention: the state at every chunk's start, a thread four columns of one channel; grid (NP * PP / 4 by 256, head, sequence)
@@ -710,28 +706,27 @@ chunk_chain_kernel(const Args a) {
     }
 }
 
-// O = Q S + M U of one chunk; grid (chunk x columns by PT, head, sequence).  M is multiplied whole, zeros above its diagonal
+// O = Q S + M U of one chunk, for states of up to 64 columns; grid (chunk, head, sequence).  M is multiplied whole, zeros above its diagonal
 // included; where a later token's row of U holds an infinity or no number, those products are no zeros, and a thread with a sum
 // that comes out so takes its sums once more without them.  (Leaving them out of the tiles' steps, by steps and a select in the step on the
 // diagonal, took 2 to 3 % of a mixer's time.)
-template <int NP, int PT>
+template <int NP>
 __global__ void __launch_bounds__(128)
 chunk_out_kernel(const Args a) {
     using Lay = Layout<NP>;
-    __shared__ __align__(16) Tile<PT> tile;
+    __shared__ __align__(16) Tile tile;
     pdl_launch_dependents();
     pdl_wait();
-    const int P = a.P, PP = pad4(P), ptiles = (PP + PT - 1) / PT;
-    const int p0 = blockIdx.x % ptiles * PT, c = a.c0 + blockIdx.x / ptiles, h = blockIdx.y, b = a.b0 + blockIdx.z;
+    const int P = a.P, PP = pad4(P), c = a.c0 + blockIdx.x, h = blockIdx.y, b = a.b0 + blockIdx.z;
     const int s0 = a.seq_start[b], t0 = s0 + c * C, nt = min(C, a.seq_start[b + 1] - t0);
     if (nt <= 0) return;
     const float* w = a.ws + (a.slot(s0, b, c) * a.H + h) * Lay::floats(PP);
-    uint64_t acc[4][PT / 16] = {};
-    tile_sums<PT>(tile, acc, NP / TK + (nt + TK - 1) / TK, PP - p0, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
+    uint64_t acc[4][4] = {};
+    tile_sums(tile, acc, NP / TK + (nt + TK - 1) / TK, PP, [&](int i, const float*& pa, long& lda, const float*& pb, long& ldb) {
         const int j = i - NP / TK;
         lda = C, ldb = PP;
         pa = w + (j < 0 ? Lay::QT + (long)i * TK * C : Lay::MT + (long)j * TK * C);
-        pb = w + (j < 0 ? Lay::s(PP) + (long)i * TK * PP : Lay::U + (long)j * TK * PP) + p0;
+        pb = w + (j < 0 ? Lay::s(PP) + (long)i * TK * PP : Lay::U + (long)j * TK * PP);
     });
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     bool finite = true;
@@ -740,25 +735,22 @@ chunk_out_kernel(const Args a) {
         const int t = r / 4 * 32 + ty * 4 + r % 4;
         if (t >= nt) continue;
         float* y = a.y + (long)(t0 + t) * a.H * P + (long)h * P;
-#pragma unroll
-        for (int x = 0; x < PT / 64; ++x) {
-            const int p = p0 + x * 64 + tx * 4;
-            const float4 v = four(acc, r, x);
-            if (p < P) finite = finite && fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY;
-            if (P % 4 == 0) {
-                if (p < P) *reinterpret_cast<float4*>(y + p) = v;
-            } else {
-                if (p < P) y[p] = v.x;
-                if (p + 1 < P) y[p + 1] = v.y;
-                if (p + 2 < P) y[p + 2] = v.z;
-                if (p + 3 < P) y[p + 3] = v.w;
-            }
+        const int p = tx * 4;
+        const float4 v = four(acc, r);
+        if (p < P) finite = finite && fabsf(v.x) + fabsf(v.y) + fabsf(v.z) + fabsf(v.w) < INFINITY;
+        if (P % 4 == 0) {
+            if (p < P) *reinterpret_cast<float4*>(y + p) = v;
+        } else {
+            if (p < P) y[p] = v.x;
+            if (p + 1 < P) y[p + 1] = v.y;
+            if (p + 2 < P) y[p + 2] = v.z;
+            if (p + 3 < P) y[p + 3] = v.w;
         }
     }
     if (!finite)                         // (rare: the same sums in the same order, over the rows that a token sees)
 #pragma unroll 1
-        for (int i = 0; i < 8 * (PT / 16); ++i) {
-            const int t = i % 8 / 4 * 32 + ty * 4 + i % 4, p = p0 + i / 32 * 64 + tx * 4 + i / 8 % 4;
+        for (int i = 0; i < 8 * 4; ++i) {
+            const int t = i % 8 / 4 * 32 + ty * 4 + i % 4, p = tx * 4 + i / 8;
             if (t >= nt || p >= P) continue;
             float sum = 0.f;
 #pragma unroll 1
@@ -1163,7 +1155,7 @@ int run_stretch(const Args& a, long ws_floats, int n_seqs, unsigned chunks, cuda
     static std::atomic<unsigned long long> devices{0};
     const cudaError_t prep_ok = plm_allow_smem(chunk_prep_kernel<T, NP, DELTA>, prep_smem<NP>(), devices);
     if (prep_ok != cudaSuccess) return (int)prep_ok;
-    constexpr int PT = 64;               // columns of an FFMA tile: a P of at most 64 is one
+    if (!TC && a.P > 64) return PLM_ERR_SHAPE;                 // (the FFMA tiles have 64 columns)
     cudaError_t e = launch_pdl(chunk_prep_kernel<T, NP, DELTA>, dim3(chunks, a.H, n_seqs), dim3(PREP_THREADS), prep_smem<NP>(), stream, a);
     if (e != cudaSuccess) return (int)e;
     if (DELTA) {
@@ -1173,13 +1165,13 @@ int run_stretch(const Args& a, long ws_floats, int n_seqs, unsigned chunks, cuda
             const int r = launch_product<NP, false>(a, ws_floats, n_seqs, chunks, stream);
             if (r != PLM_OK) return r;
         } else
-            e = launch_pdl(chunk_outer_kernel<NP, PT>, dim3(chunks * (NP / 64), a.H, n_seqs), dim3(128), 0, stream, a);
+            e = launch_pdl(chunk_outer_kernel<NP>, dim3(chunks * (NP / 64), a.H, n_seqs), dim3(128), 0, stream, a);
         if (e != cudaSuccess) return (int)e;
         e = launch_pdl(chunk_chain_kernel<NP>, dim3((NP * (pad4(a.P) / 4) + 255) / 256, a.H, n_seqs), dim3(256), 0, stream, a);
     }
     if (e != cudaSuccess) return (int)e;
     if constexpr (TC) return launch_product<NP, true>(a, ws_floats, n_seqs, chunks, stream);
-    else return plm_status_of(launch_pdl(chunk_out_kernel<NP, PT>, dim3(chunks, a.H, n_seqs), dim3(128), 0, stream, a));
+    else return plm_status_of(launch_pdl(chunk_out_kernel<NP>, dim3(chunks, a.H, n_seqs), dim3(128), 0, stream, a));
 }
 
 // The whole step at once where the workspace holds it.  Else so many chunks of so many sequences at a time as it holds: a state
