@@ -27,9 +27,11 @@
 // a piece: 1.05, but slow here (2,000 cycles a stage for 128 x 128 results).
 // The CUDA cores against this: 462 rows x 16,384 x 2,048 893 and 236 us (131 TFLOP/s of float32 products); x 2,048 x 8,192 662 and 137;
 // 24 rows x 3,072 x 2,048 42.7 and 17.3; 8 rows x 2,048 x 8,192 71 and 33.
-// Bound by the MMAs (106 cycles each at 96 columns, 79 at 64, 58 at 16) and the hand-overs between the warps.  Everything done by
+// Bound by the chain of hand-overs between the warps and by their instructions (issue slots 62 to 69 % taken, the tensor pipe busy for
+// 33 to 35 % of the time; an MMA takes 106 cycles at 96 columns, 79 at 64, 58 at 16, W's terms out of tensor memory among them).  Everything done by
 // the same eight warps, with W's terms in shared memory too: 490 us for 462 x 2,048 x 8,192; splitting and adding apart 275;
-// W's terms in tensor memory 237; two issuing warps behind elect.sync 190; four splitting warps a stage in turns 171.
+// W's terms in tensor memory 237; two issuing warps behind elect.sync 190; four splitting warps a stage in turns 171
+// (all of these with SETTLE = 4).
 #include "split_common.cuh"
 
 using namespace plm_tc;

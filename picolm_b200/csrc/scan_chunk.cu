@@ -17,7 +17,7 @@
 // the outputs are products on the tensor cores where the state has more than 64 columns (`chunk_product`), else FFMA tiles
 // (`chunk_outer`, `chunk_out`); the rest runs on the CUDA cores.
 // 2,048 tokens, 8 heads of 128 x 128, warm caches: the delta rule 518 us (32 tokens at a time, everything but the scaled keys and queries in
-// the chain) -> SCAN_DELTA, linear attention 144 us (token by token in segments) -> SCAN_GLA.  Errors against 64 bits in 2^-24, all products FFMA / on
+// the chain) -> 120, linear attention 144 us (token by token in segments) -> 65.  Errors against 64 bits in 2^-24, all products FFMA / on
 // the tensor cores (512 tokens, 4 heads of 128 x 128, normal numbers; rows behind SiLU): linear attention's outputs 3.9 / 2.3 (2.8 / 1.4),
 // state 2.5 / 1.5 (1.7 / 1.2), the delta rule's outputs 3.4 / 3.2 (2.6 / 2.4); where all values are positive and spread over several
 // decades the tensor cores' are larger (3.3 / 4.2 and 1.8 / 3.0; see gemm_f32_tc.cu).
@@ -770,9 +770,9 @@ chunk_out_kernel(const Args a) {
 // copies (their rows lie row by row in the workspace) and both are transposed on the way: a lane of the splitting warps reads one
 // column's 32 rows for tensor memory, and the other operand stays as it lies, rows of 128 bytes with the 128-byte swizzle that
 // the MMA reads with its N contiguous.
-// Bound by the MMAs (12 a step of 64 columns, 60 to 80 cycles each) and by the hand-overs, some 1,000 cycles a step.  2,361 tokens in two
-// sequences, 8 heads of 128 x 256, warm caches: outputs 47 us as FFMA tiles of 64 x 128 -> 30, what the chunks add 30 -> 20.5; 2,048
-// tokens, 8 heads of 128 x 128: outputs 23.4 -> 13.9.
+// Bound by the hand-overs between the warps, some 1,000 cycles a step (the tensor pipe is busy for 12 to 15 % of the time).  2,361 tokens in two
+// sequences, 8 heads of 128 x 256, warm caches: outputs 47 us as FFMA tiles of 64 x 128 -> 31, what the chunks add 30 -> 21; 2,048
+// tokens, 8 heads of 128 x 128: outputs 23.4 -> 14.5.
 constexpr int TC_FOLDERS = 8, TC_LOADER = 16, TC_ISSUER = 17, TC_THREADS = 640, TC_RING = 4, TC_ROWS = 128, TC_STEP = 32;
 
 template <int NB> struct TcTile {                                // NB columns of a unit: 64 or 128

@@ -206,7 +206,7 @@ def test_chunk_products_of_the_smallest_and_largest_values(small, large):
         assert (got.double() - want.reshape(T, -1)).norm() <= 2e-6 * want.norm()
 
 
-def _retention(N, P, lens, H=3, positions=0, odd=None):
+def _retention(N, P, lens, H=3, positions=0, odd=None, rotary_dim=None):
     """ops.decay_scan over rotated rows, its inputs, and the same in float64 with everything that the kernels are handed."""
     from picolm_b200 import ops
     from picolm_b200.ops import recurrent
@@ -222,17 +222,17 @@ def _retention(N, P, lens, H=3, positions=0, odd=None):
         for t, c, x in odd:
             v[t, c] = x
     decay = torch.tensor([1.0 - 2.0 ** (-3.0 - 2 * h) for h in range(H)], dtype=torch.float64)
-    half = N // 2
+    half = (N if rotary_dim is None else rotary_dim) // 2
     angle = torch.arange(positions + max(lens), dtype=torch.float64)[:, None] * 10000.0 ** (-torch.arange(half, dtype=torch.float64) / half)
-    rotation = types.SimpleNamespace(cos=angle.cos().float().to(DEV), sin=angle.sin().float().to(DEV), rotary_dim=N, pairing="half")
+    rotation = types.SimpleNamespace(cos=angle.cos().float().to(DEV), sin=angle.sin().float().to(DEV), rotary_dim=2 * half, pairing="half") if half else None
     state = torch.randn(len(lens), H * N * P, device=DEV)
     before = state.clone()
     with mock.patch.object(recurrent, "decay_in_128", lambda *a: True):                # (whatever the rule would choose)
         y = ops.decay_scan(q, k, v, decay.float().to(DEV), ops.decay_powers(decay).to(DEV), state, step, H, N, P, rotation=rotation, k_scale=N ** -0.5)
     want, states = [], []
     for b, n in enumerate(lens):
-        c, s = (f[positions:positions + n].double()[:, None] for f in (rotation.cos, rotation.sin))
-        turn = lambda x: (lambda u, w: torch.cat([u * c - w * s, w * c + u * s], -1))(*x[start[b]:start[b] + n].double().view(n, H, N).split(half, -1))
+        c, s = (f[positions:positions + n].to(DEV).float().double()[:, None] for f in (angle.cos(), angle.sin()))
+        turn = lambda x: (lambda u, w, r: torch.cat([u * c - w * s, w * c + u * s, r], -1))(*x[start[b]:start[b] + n].double().view(n, H, N).split([half, half, N - 2 * half], -1))
         qq, kk, vv = turn(q), turn(k) * N ** -0.5, v[start[b]:start[b] + n].double().view(n, H, P)
         S, out = before[b].double().view(H, N, P), []
         for i in range(n):
@@ -254,6 +254,12 @@ def test_retention_128_tokens_at_a_time(N, P, lens):
     assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
     for t in range(0, want.shape[0], 37):
         assert (y[t].double() - want[t]).norm() <= 6 * 2.0 ** -17 * want[t].norm()
+
+
+@pytest.mark.parametrize("N,rotary_dim", [(64, 0), (64, 16), (128, 32), (128, 112)])
+def test_retention_with_part_of_a_head_rotated(N, rotary_dim):
+    y, want, state, states = _retention(N, 128, [200, 131], positions=5, rotary_dim=rotary_dim)
+    assert (y.double() - want).norm() <= 3 * 2.0 ** -17 * want.norm() and (state.double() - states).norm() <= 3 * 2.0 ** -17 * states.norm()
 
 
 @pytest.mark.parametrize("lens", [[0, 140, 0, 0, 1, 300, 0], [(7 * i) % 40 for i in range(70)], [300] + [i % 3 for i in range(1100)] + [129]])
